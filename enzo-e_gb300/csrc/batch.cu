@@ -78,6 +78,12 @@ struct mhdvlct_batch {
   int tile_full[2] = {0, 0};  // 1: every tile of the stage is tile_tx x tile_ty
   int block_m = 0;            // every block's extent along all axes, if equal; else 0
   int* d_queue = nullptr;     // 2 counters
+  // FP64: the split stages' jobs and groups, and the workspace they share
+  // (null when it could not be had: the fused kernels run instead)
+  SplitJob* d_jobs[2] = {nullptr, nullptr};
+  std::vector<SplitGroup> sp_groups[2];
+  void* d_ws = nullptr;
+  size_t ws_elems = 0;
   int* d_nbr = nullptr;
   // mesh refresh from a face list (replaces the 27-neighbour same-level
   // refresh when set): pointer tables of both face-buffer parities, the
@@ -100,6 +106,9 @@ struct mhdvlct_batch {
   std::vector<int> hg_first;        // first block of each group (+ end)
   StageTile* d_gtiles = nullptr;
   std::vector<int> hg_tile0, hg_ntile;
+  SplitJob* d_gjobs = nullptr;      // FP64: the split full-dt stage's jobs by group
+  std::vector<std::vector<SplitGroup>> hg_groups;
+  std::vector<int> hg_job0;
   int* d_gqueue = nullptr;
   cudaStream_t s_d2h = nullptr, s_h2d = nullptr;
   std::vector<cudaEvent_t> ev;      // 3 per group: stage done, out, in
@@ -338,6 +347,23 @@ int build_descriptors(mhdvlct_batch* b, cudaStream_t st) {
     if ((rc = upload((void**)&b->d_tiles[s], tiles[s].data(),
                      tiles[s].size() * sizeof(StageTile))))
       return rc;
+  // the split stages depend on the blocks' extents alone: planned once
+  std::vector<SplitJob> jobs[2];
+  if (sizeof(R) == 8 && !b->d_jobs[0]) {
+    std::vector<int> m;
+    for (const auto& o : b->off) m.insert(m.end(), o.m, o.m + 3);
+    b->ws_elems = 0;
+    for (int s = 0; s < 2; s++)
+      split_plan(m, {}, sp.S[s], s == 1, b->h->mhd != 0, b->h->de != 0, jobs[s], b->sp_groups[s],
+                 b->ws_elems);
+    if (bmalloc(b, &b->d_ws, std::max<size_t>(b->ws_elems, 1) * sizeof(R)) != cudaSuccess) {
+      cudaGetLastError();
+      b->d_ws = nullptr;
+    }
+    for (int s = 0; s < 2; s++)
+      if ((rc = upload((void**)&b->d_jobs[s], jobs[s].data(), jobs[s].size() * sizeof(SplitJob))))
+        return rc;
+  }
   cudaStreamSynchronize(st);
   drop_graphs(b);
   b->hg_n = 0;  // the host-run groups are rebuilt from the new tiles
@@ -375,13 +401,27 @@ StageInfo batch_stage_info(const mhdvlct_batch* b, int s, int* queue) {
   return info;
 }
 
+// A split stage's launch over `groups` of `jobs` (none: the fused kernel).
+SplitLaunch split_launch(const mhdvlct_batch* b, const SplitJob* jobs,
+                         const std::vector<SplitGroup>& groups) {
+  SplitLaunch l;
+  if (b->d_ws) {
+    l.jobs = jobs;
+    l.groups = groups.data();
+    l.ngroups = (int)groups.size();
+    l.ws = b->d_ws;
+  }
+  return l;
+}
+
 template <class R>
 cudaError_t launch_one_stage(mhdvlct_batch* b, int s, cudaStream_t st) {
   const StagePlan sp = stage_plan(b->h);
   const StageInfo info = batch_stage_info(b, s, b->d_queue + s);
   return launch_stage<R>(b->h->solver, sp.recon[s], b->h->de != 0,
                          (const StageBlock<R>*)b->d_sblocks[b->parity][s],
-                         b->d_tiles[s], b->ntiles[s], info, b->h->phys, b->grid, st);
+                         b->d_tiles[s], b->ntiles[s], info, b->h->phys, b->grid, st,
+                         split_launch(b, b->d_jobs[s], b->sp_groups[s]));
 }
 
 template <class R>
@@ -618,6 +658,9 @@ extern "C" int mhdvlct_batch_destroy(mhdvlct_batch* b) {
   bfree(b, b->d_fcplan);
   bfree(b, b->d_gtiles);
   bfree(b, b->d_gqueue);
+  bfree(b, b->d_gjobs);
+  for (int s = 0; s < 2; s++) bfree(b, b->d_jobs[s]);
+  bfree(b, b->d_ws);
   for (cudaEvent_t x : b->ev) cudaEventDestroy(x);
   if (b->s_d2h) cudaStreamDestroy(b->s_d2h);
   if (b->s_h2d) cudaStreamDestroy(b->s_h2d);
@@ -959,14 +1002,40 @@ int setup_host_groups(mhdvlct_batch* b, int ngroups) {
       if (group_of[t.block] == g) sorted.push_back(t);
     b->hg_ntile[g] = (int)sorted.size() - b->hg_tile0[g];
   }
+  // FP64: the full-dt stage's split jobs of each group
+  std::vector<SplitJob> jobs;
+  b->hg_groups.assign(ng, {});
+  b->hg_job0.assign(ng, 0);
+  if (b->d_ws) {
+    const StagePlan sp = stage_plan(b->h);
+    std::vector<int> m;
+    for (const auto& o : b->off) m.insert(m.end(), o.m, o.m + 3);
+    for (int g = 0; g < ng; g++) {
+      std::vector<int> ids;
+      for (int i = b->hg_first[g]; i < b->hg_first[g + 1]; i++) ids.push_back(i);
+      std::vector<SplitJob> part;
+      size_t ws = 0;
+      split_plan(m, ids, sp.S[1], true, b->h->mhd != 0, b->h->de != 0, part, b->hg_groups[g], ws,
+                 b->ws_elems);
+      b->hg_job0[g] = (int)jobs.size();
+      jobs.insert(jobs.end(), part.begin(), part.end());
+    }
+  }
   bfree(b, b->d_gtiles);
   bfree(b, b->d_gqueue);
+  bfree(b, b->d_gjobs);
   b->d_gtiles = nullptr;
   b->d_gqueue = nullptr;
+  b->d_gjobs = nullptr;
   if (bmalloc(b, (void**)&b->d_gtiles, std::max<size_t>(1, sorted.size()) * sizeof(StageTile)) !=
+          cudaSuccess ||
+      bmalloc(b, (void**)&b->d_gjobs, std::max<size_t>(1, jobs.size()) * sizeof(SplitJob)) !=
           cudaSuccess ||
       bmalloc(b, (void**)&b->d_gqueue, ng * sizeof(int)) != cudaSuccess)
     return bfail(b, MHD_ERR_NOMEM, "host-run tables");
+  if (!jobs.empty() && cudaMemcpy(b->d_gjobs, jobs.data(), jobs.size() * sizeof(SplitJob),
+                                  cudaMemcpyHostToDevice) != cudaSuccess)
+    return bfail(b, MHD_ERR_CUDA, "host-run jobs");
   cudaError_t e = cudaMemcpy(b->d_gtiles, sorted.data(), sorted.size() * sizeof(StageTile),
                              cudaMemcpyHostToDevice);
   if (e != cudaSuccess) return bfail(b, MHD_ERR_CUDA, cudaGetErrorString(e));
@@ -1059,7 +1128,8 @@ int run_host_t(mhdvlct_batch* b, char* host, int ncycles, cudaStream_t st) {
       e = launch_stage<R>(b->h->solver, sp.recon[1], b->h->de != 0,
                           (const StageBlock<R>*)b->d_sblocks[b->parity][1],
                           b->d_gtiles + b->hg_tile0[g], b->hg_ntile[g], info, b->h->phys,
-                          b->grid, st);
+                          b->grid, st,
+                          split_launch(b, b->d_gjobs + b->hg_job0[g], b->hg_groups[g]));
       if (e == cudaSuccess && !b->fc_on) e = cudaEventRecord(ev[g], st);
     }
     if (e == cudaSuccess && b->fc_on) {
@@ -1245,7 +1315,11 @@ int autotune_t(mhdvlct_batch* b, int reps, std::string& json, cudaStream_t st) {
         other_ty = std::max(other_ty, oc.tile_y[s]);
       }
       std::vector<TileChoice> cands;
+      // the split FP64 stages have no tiles: the choice in force is the only
+      // candidate
+      if (b->d_ws) cands.push_back(bestc);
       for (auto& sh : shapes) {
+        if (b->d_ws) break;
         if (stage_smem<R>(b->h->solver, sp.recon[s], b->h->de != 0,
                           std::max(sh.first, other_tx), std::max(sh.second, other_ty)) >
             smem_cap)

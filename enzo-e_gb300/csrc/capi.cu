@@ -87,6 +87,54 @@ void make_tiles(int block, const int m[3], int S, bool final, int tile_x,
         out.push_back({block, x.first, x.second, y.first, y.second, z.first, z.second});
 }
 
+void split_plan(const std::vector<int>& m, const std::vector<int>& ids, int S, bool final,
+                bool mhd, bool de, std::vector<SplitJob>& jobs, std::vector<SplitGroup>& groups,
+                size_t& ws_elems, size_t max_elems) {
+  // cells of a group: enough faces for tens of waves of the GPU's FP64 pipes
+  // (a group ends in a partly filled wave), 0.3 GB of workspace with CT
+  constexpr size_t kGroupCells = 1300000;
+  constexpr int kGroupJobs = 16384;  // below the grid's y limit
+  const size_t arrays = split_arrays(mhd, de);
+  const size_t limit = max_elems ? max_elems / arrays : kGroupCells;
+  struct Piece {
+    SplitJob j;
+    size_t cells;
+  };
+  std::vector<Piece> pieces;
+  const int nb = ids.empty() ? (int)(m.size() / 3) : (int)ids.size();
+  for (int k = 0; k < nb; k++) {
+    const int i = ids.empty() ? k : ids[k];
+    const int* e = &m[3 * (size_t)i];
+    const int lo = final ? S : S + 1;
+    if (e[0] <= 2 * lo || e[1] <= 2 * lo || e[2] <= 2 * lo) continue;
+    // a block too large for a group goes in slabs of planes
+    const size_t plane = (size_t)e[0] * e[1];
+    const int most = (int)std::max<long long>(1, (long long)(kGroupCells / plane) - 4);
+    const int len = e[2] - 2 * lo, parts = (len + most - 1) / most;
+    for (int p = 0, z = lo; p < parts; p++) {
+      const int n = len / parts + (p < len % parts ? 1 : 0);
+      pieces.push_back({SplitJob{i, z, z + n, 0}, plane * (size_t)(n + 4)});
+      z += n;
+    }
+  }
+  std::stable_sort(pieces.begin(), pieces.end(),
+                   [](const Piece& a, const Piece& b) { return a.cells > b.cells; });
+  jobs.clear();
+  groups.clear();
+  for (const Piece& p : pieces) {
+    if (groups.empty() || groups.back().total + p.cells > limit ||
+        groups.back().count >= kGroupJobs)
+      groups.push_back(SplitGroup{(int)jobs.size(), 0, 0, 0});
+    SplitGroup& g = groups.back();
+    jobs.push_back(p.j);
+    jobs.back().off = g.total * arrays;
+    g.count++;
+    g.cells = std::max(g.cells, p.cells);
+    g.total += p.cells;
+    ws_elems = std::max(ws_elems, g.total * arrays);
+  }
+}
+
 template <class R>
 FieldSet<R> fieldset_of(const MhdBlockView* b) {
   FieldSet<R> f;
@@ -584,6 +632,8 @@ template <class R> struct PlainScratch {
   AuxBlock<R>* d_aux;        // [1]
   int* d_nbr;                // [27]
   void* d_fc;                // FluxOut<R> for the boundary fluxes
+  SplitJob* d_jobs;          // the split stages' jobs, likewise
+  void* ws;                  // their workspace (null: the fused kernels)
   StageTile* d_tiles;        // stage 0 tiles then stage 1 tiles
   int ntiles[2];
   int tile[2];               // largest tile extent of each stage
@@ -622,16 +672,37 @@ int ensure_scratch(mhdvlct_handle* h, const int m[3], int dtype,
   take(27 * sizeof(int));
   take(sizeof(FluxOut<R>));
   take((size_t)(nt[0] + nt[1]) * sizeof(StageTile));
-  const bool same = h->scratch && h->cache_dtype == dtype && h->cache_m[0] == m[0] &&
-                    h->cache_m[1] == m[1] && h->cache_m[2] == m[2] &&
-                    h->cache_np == np && h->scratch_bytes >= off;
+  const bool geom = h->scratch && h->cache_dtype == dtype && h->cache_m[0] == m[0] &&
+                    h->cache_m[1] == m[1] && h->cache_m[2] == m[2] && h->cache_np == np;
+  if (!geom) {
+    h->sp_ws = 0;
+    for (int i = 0; i < 2; i++) {
+      h->sp_jobs[i].clear();
+      h->sp_groups[i].clear();
+      if (sizeof(R) == 8 && i < sp.nstages)
+        split_plan({m[0], m[1], m[2]}, {}, sp.S[i], i + 1 == sp.nstages, h->mhd != 0, h->de != 0,
+                   h->sp_jobs[i], h->sp_groups[i], h->sp_ws);
+    }
+  }
+  // the split stages' part comes last: without room for it (no such block has
+  // been seen before the state itself fills the GPU) the fused kernels run
+  const size_t fused_bytes = off;
+  take((h->sp_jobs[0].size() + h->sp_jobs[1].size()) * sizeof(SplitJob));
+  take(h->sp_ws * sizeof(R));
+  const bool same = geom && h->scratch_bytes >= (h->split ? off : fused_bytes);
   if (!same) {
     if (h->scratch) {
       cudaStreamSynchronize(st);
       cudaFree(h->scratch);
       h->scratch = nullptr;
     }
+    h->split = h->sp_ws > 0;
     cudaError_t e = cudaMalloc(&h->scratch, off);
+    if (e != cudaSuccess && h->split) {
+      cudaGetLastError();
+      h->split = false;
+      e = cudaMalloc(&h->scratch, off = fused_bytes);
+    }
     if (e != cudaSuccess) {
       h->scratch = nullptr;
       return fail(h, MHD_ERR_NOMEM, std::string("scratch allocation: ") + cudaGetErrorString(e));
@@ -660,10 +731,18 @@ int ensure_scratch(mhdvlct_handle* h, const int m[3], int dtype,
   S.ntiles[1] = (int)nt[1];
   S.tile[0] = dc.tile[0];
   S.tile[1] = dc.tile[1];
+  S.d_jobs = h->split ? (SplitJob*)(base + offs[i]) : nullptr;
+  S.ws = h->split ? (void*)(base + offs[i + 1]) : nullptr;
   if (!same) {
     cudaError_t e = launch_make_tiles(S.d_tiles, ts[0], st);
     if (e == cudaSuccess) e = launch_make_tiles(S.d_tiles + nt[0], ts[1], st);
     if (e != cudaSuccess) return cuda_fail(h, e, "tile set-up");
+    SplitJob* dj = S.d_jobs;
+    for (int k = 0; k < 2 && h->split; k++) {
+      e = put_bytes(dj, h->sp_jobs[k].data(), h->sp_jobs[k].size() * sizeof(SplitJob), st);
+      if (e != cudaSuccess) return cuda_fail(h, e, "job set-up");
+      dj += h->sp_jobs[k].size();
+    }
     // a single block refreshes from itself: every neighbour entry is 0
     e = cudaMemsetAsync(S.d_nbr, 0, 27 * sizeof(int), st);
     if (e != cudaSuccess) return cuda_fail(h, e, "neighbour set-up");
@@ -772,8 +851,15 @@ int block_step_on(mhdvlct_handle* h, const MhdBlockView* b, PlainScratch<R>& S,
       info.fc = S.d_fc;
       info.fc_g = b->ghost[0];
     }
+    SplitLaunch split;
+    if (S.ws) {
+      split.jobs = S.d_jobs + (i == 0 ? 0 : h->sp_jobs[0].size());
+      split.groups = h->sp_groups[i].data();
+      split.ngroups = (int)h->sp_groups[i].size();
+      split.ws = S.ws;
+    }
     e = launch_stage<R>(h->solver, sp.recon[i], h->de != 0, S.d_sblocks + i, tiles[i],
-                        S.ntiles[i], info, h->phys, 0, st);
+                        S.ntiles[i], info, h->phys, 0, st, split);
     if (e != cudaSuccess) return cuda_fail(h, e, "stage launch");
   }
   if (h->mhd) {

@@ -24,6 +24,12 @@ struct mhdvlct_handle {
   int cache_np = 0;            // passive-scalar scratch fields in the cache
   void* scratch = nullptr;     // one device allocation
   size_t scratch_bytes = 0;
+  // the split stages' jobs of that geometry (FP64): per stage, and the
+  // elements of workspace they share; split: the scratch holds them
+  std::vector<vlct::SplitJob> sp_jobs[2];
+  std::vector<vlct::SplitGroup> sp_groups[2];
+  size_t sp_ws = 0;
+  bool split = false;
   int tile = 0;                // tile extent used by the plain path
   int zchunk = 0;              // z-chunk length used by the plain path
   // mesh-refresh tables (pointer table, regions, chunks), reused across calls
@@ -54,6 +60,14 @@ StagePlan stage_plan(const mhdvlct_handle* h);
 // block, S: stale depth after reconstruction, final: last stage.
 void make_tiles(int block, const int m[3], int S, bool final, int tile_x,
                 int tile_y, int zchunk, std::vector<vlct::StageTile>& out);
+
+// The jobs of a split stage over blocks of ghosted extents m (3 per block),
+// blocks `ids` of them (all when empty), in groups whose workspace is bounded
+// (by max_elems too, when given); ws_elems is raised to the elements the
+// largest group needs.
+void split_plan(const std::vector<int>& m, const std::vector<int>& ids, int S, bool final,
+                bool mhd, bool de, std::vector<vlct::SplitJob>& jobs,
+                std::vector<vlct::SplitGroup>& groups, size_t& ws_elems, size_t max_elems = 0);
 
 // Device field pointers of a block view.
 template <class R>

@@ -7,6 +7,7 @@
 #include "vlct_aux.cuh"
 #include "vlct_launch.h"
 #include "vlct_passive.cuh"
+#include "vlct_split.cuh"
 #include "vlct_stage.cuh"
 
 namespace vlct {
@@ -67,10 +68,54 @@ StageKernelFn stage_fn(const StageInfo& info) {
   return f ? f : stage_kernel<VLCT_REAL, SOLVER, RECON, DE, EXTRA>;
 }
 
+// One stage as the kernels of vlct_split.cuh, group after group of jobs.
+template <class R, int SOLVER, int RECON, bool DE>
+cudaError_t stage_split(const StageBlock<R>* b, const SplitLaunch& sp, const StageInfo& info,
+                        const PhysParams& phys, cudaStream_t st) {
+  constexpr bool MHD = SOLVER != SOLVER_HLLC;
+  R* ws = static_cast<R*>(sp.ws);
+  static const int nsm = [] {
+    int dev = 0, n = 0;
+    cudaGetDevice(&dev);
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
+      n = 1;
+    return n;
+  }();
+  for (int k = 0; k < sp.ngroups; k++) {
+    const SplitGroup& G = sp.groups[k];
+    const SplitJob* jobs = sp.jobs + G.first;
+    const unsigned gx = (unsigned)((G.cells + 127) / 128);
+    const dim3 cells(gx, G.count);
+    // faces a thread takes: as many as leave 256 threads to every SM
+    int kmax = 1;
+    if (RECON != RECON_NN)
+      kmax = (int)std::max<size_t>(1, std::min<size_t>(12, 3 * G.total / ((size_t)nsm * 256)));
+    const int kmin = (kmax + 1) / 2;
+    const dim3 faces((gx + kmin - 1) / kmin, G.count, 3);
+    split_prim_kernel<R, MHD, DE><<<cells, 128, 0, st>>>(b, jobs, ws, info, phys);
+    split_flux_kernel<R, SOLVER, RECON, DE><<<faces, 128, 0, st>>>(b, jobs, ws, info, phys, kmax);
+    if constexpr (MHD) split_emf_kernel<R, DE><<<cells, 128, 0, st>>>(b, jobs, ws, info);
+    split_update_kernel<R, MHD, DE><<<cells, 128, 0, st>>>(b, jobs, ws, info, phys);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
 template <class R, int SOLVER, int RECON, bool DE>
 cudaError_t stage_one(const StageBlock<R>* b, const StageTile* t, int nt,
                       const StageInfo& info, const PhysParams& phys, int grid,
-                      cudaStream_t st) {
+                      cudaStream_t st, const SplitLaunch& split) {
+  if constexpr (std::is_same<R, double>::value) {
+    if (split.ngroups > 0) {
+      cudaError_t e = stage_split<R, SOLVER, RECON, DE>(b, split, info, phys, st);
+      if (e == cudaSuccess && info.npass > 0 && nt > 0) {
+        passive_kernel<R, RECON><<<nt, 256, 0, st>>>(b, t, info, phys);
+        e = cudaGetLastError();
+      }
+      return e;
+    }
+  }
   const bool all = info.gravity != 0 || info.npass > 0;
   const bool fc = info.fc != nullptr || info.block_fc != 0;
   const size_t smem = stage_smem_bytes<R, SOLVER, RECON, DE>(info.tx, info.ty);
@@ -113,12 +158,12 @@ cudaError_t stage_one(const StageBlock<R>* b, const StageTile* t, int nt,
 template <class R, int SOLVER, bool DE>
 cudaError_t stage_recon(int recon, const StageBlock<R>* b, const StageTile* t,
                         int nt, const StageInfo& info, const PhysParams& phys,
-                        int grid, cudaStream_t st) {
+                        int grid, cudaStream_t st, const SplitLaunch& split) {
   switch (recon) {
-    case RECON_NN: return stage_one<R, SOLVER, RECON_NN, DE>(b, t, nt, info, phys, grid, st);
-    case RECON_PLM: return stage_one<R, SOLVER, RECON_PLM, DE>(b, t, nt, info, phys, grid, st);
+    case RECON_NN: return stage_one<R, SOLVER, RECON_NN, DE>(b, t, nt, info, phys, grid, st, split);
+    case RECON_PLM: return stage_one<R, SOLVER, RECON_PLM, DE>(b, t, nt, info, phys, grid, st, split);
     case RECON_PLM_ATHENA:
-      return stage_one<R, SOLVER, RECON_PLM_ATHENA, DE>(b, t, nt, info, phys, grid, st);
+      return stage_one<R, SOLVER, RECON_PLM_ATHENA, DE>(b, t, nt, info, phys, grid, st, split);
   }
   return cudaErrorInvalidValue;
 }
@@ -126,9 +171,10 @@ cudaError_t stage_recon(int recon, const StageBlock<R>* b, const StageTile* t,
 template <class R, int SOLVER>
 cudaError_t stage_de(int recon, bool de, const StageBlock<R>* b,
                      const StageTile* t, int nt, const StageInfo& info,
-                     const PhysParams& phys, int grid, cudaStream_t st) {
-  return de ? stage_recon<R, SOLVER, true>(recon, b, t, nt, info, phys, grid, st)
-            : stage_recon<R, SOLVER, false>(recon, b, t, nt, info, phys, grid, st);
+                     const PhysParams& phys, int grid, cudaStream_t st,
+                     const SplitLaunch& split) {
+  return de ? stage_recon<R, SOLVER, true>(recon, b, t, nt, info, phys, grid, st, split)
+            : stage_recon<R, SOLVER, false>(recon, b, t, nt, info, phys, grid, st, split);
 }
 
 template <class R, int SOLVER, bool DE>
@@ -147,11 +193,11 @@ cudaError_t launch_stage<VLCT_REAL>(int solver, int recon, bool de,
                                     const StageTile* t, int nt,
                                     const StageInfo& info,
                                     const PhysParams& phys, int grid,
-                                    cudaStream_t st) {
+                                    cudaStream_t st, const SplitLaunch& split) {
   switch (solver) {
-    case SOLVER_HLLE: return stage_de<VLCT_REAL, SOLVER_HLLE>(recon, de, b, t, nt, info, phys, grid, st);
-    case SOLVER_HLLC: return stage_de<VLCT_REAL, SOLVER_HLLC>(recon, de, b, t, nt, info, phys, grid, st);
-    case SOLVER_HLLD: return stage_de<VLCT_REAL, SOLVER_HLLD>(recon, de, b, t, nt, info, phys, grid, st);
+    case SOLVER_HLLE: return stage_de<VLCT_REAL, SOLVER_HLLE>(recon, de, b, t, nt, info, phys, grid, st, split);
+    case SOLVER_HLLC: return stage_de<VLCT_REAL, SOLVER_HLLC>(recon, de, b, t, nt, info, phys, grid, st, split);
+    case SOLVER_HLLD: return stage_de<VLCT_REAL, SOLVER_HLLD>(recon, de, b, t, nt, info, phys, grid, st, split);
   }
   return cudaErrorInvalidValue;
 }

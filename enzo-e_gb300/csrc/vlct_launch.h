@@ -20,7 +20,8 @@ template <class R>
 cudaError_t launch_stage(int solver, int recon, bool de,
                          const StageBlock<R>* d_blocks, const StageTile* d_tiles,
                          int ntiles, const StageInfo& info,
-                         const PhysParams& phys, int grid, cudaStream_t st);
+                         const PhysParams& phys, int grid, cudaStream_t st,
+                         const SplitLaunch& split = SplitLaunch());
 
 template <class R>
 size_t stage_smem(int solver, int recon, bool de, int tx, int ty);

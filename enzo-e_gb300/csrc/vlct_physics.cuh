@@ -27,6 +27,31 @@ template <class R> __device__ __forceinline__ R smin(R a, R b) {
 template <class R> __device__ __forceinline__ R smax(R a, R b) {
   return (a < b) ? b : a;
 }
+// Sign tests.  For double they read the bit pattern on the integer pipe, as a
+// comparison would occupy the narrow FP64 pipe (false for NaN, zeros of either
+// sign alike, as the comparisons).
+template <class R> __device__ __forceinline__ bool gt0(R x) { return x > R(0); }
+template <class R> __device__ __forceinline__ bool lt0(R x) { return x < R(0); }
+template <class R> __device__ __forceinline__ bool ge0(R x) { return x >= R(0); }
+template <class R> __device__ __forceinline__ bool le0(R x) { return x <= R(0); }
+constexpr long long kInfBits = 0x7ff0000000000000LL;
+constexpr long long kAbsBits = 0x7fffffffffffffffLL;
+template <> __device__ __forceinline__ bool gt0<double>(double x) {
+  const long long i = __double_as_longlong(x);
+  return i > 0 && i <= kInfBits;
+}
+template <> __device__ __forceinline__ bool lt0<double>(double x) {
+  const long long i = __double_as_longlong(x), a = i & kAbsBits;
+  return i < 0 && a != 0 && a <= kInfBits;
+}
+template <> __device__ __forceinline__ bool ge0<double>(double x) {
+  const long long i = __double_as_longlong(x), a = i & kAbsBits;
+  return (i >= 0 || a == 0) && a <= kInfBits;
+}
+template <> __device__ __forceinline__ bool le0<double>(double x) {
+  const long long i = __double_as_longlong(x), a = i & kAbsBits;
+  return (i < 0 || a == 0) && a <= kInfBits;
+}
 // enzo_utils::min of three values (utils.hpp:82-89)
 template <class R> __device__ __forceinline__ R min3(R a, R b, R c) {
   if (a < b) return (c < a) ? c : a;
@@ -102,6 +127,40 @@ __device__ __forceinline__ R limiter_athena(R vm1, R v, R vp1) {
   return R(2.) * temp / (dv_l + dv_r);
 }
 
+// Half the limited slope of a cell: what PLM adds to and takes from the cell's
+// value at its two faces.
+template <class R, int RECON>
+__device__ __forceinline__ R half_slope(R vm1, R v, R vp1, R theta) {
+  return (RECON == RECON_PLM ? limiter_enzo_rk(vm1, v, vp1, theta)
+                             : limiter_athena(vm1, v, vp1)) * R(0.5);
+}
+// The theta limiter in FP64, with its sign tests, minimum and halving on the
+// integer pipe (the FP64 pipe, which bounds the FP64 stages, keeps five
+// operations of about twenty).  Magnitudes of finite doubles order like their
+// bit patterns, and halving one that stays normal is a step of its exponent;
+// anything else takes limiter_enzo_rk itself.  0.5 (sgn dl + sgn dr) times the
+// minimum is the minimum with the common sign, a zero of the sign of the one
+// that is not zero, or +0.
+template <>
+__device__ __forceinline__ double half_slope<double, RECON_PLM>(double vm1, double v,
+                                                                double vp1, double theta) {
+  const double dv_c = 0.5 * (vp1 - vm1);
+  const double dv_l = (v - vm1) * theta;
+  const double dv_r = (vp1 - v) * theta;
+  const long long il = __double_as_longlong(dv_l), ir = __double_as_longlong(dv_r);
+  const long long al = il & kAbsBits, ar = ir & kAbsBits,
+                  ac = __double_as_longlong(dv_c) & kAbsBits;
+  long long m = al < ar ? al : ar;
+  const long long most = al < ar ? ar : al;
+  m = ac < m ? ac : m;
+  if ((most < ac ? ac : most) >= kInfBits || (m != 0 && m < 0x0020000000000000LL))
+    return limiter_enzo_rk(vm1, v, vp1, theta) * 0.5;
+  const bool opposite = al != 0 && ar != 0 && (il ^ ir) < 0;
+  const long long sign = (al != 0 ? il : (ar != 0 ? ir : 0)) & ~kAbsBits;
+  if (m != 0) m -= 0x0010000000000000LL;
+  return opposite ? 0.0 : __longlong_as_double(m | sign);
+}
+
 // ------------------------------------------------------ Riemann solvers ----
 // Output of one face solve, in the face frame: 8 fluxes (flux[L_BI] == 0),
 // the passive internal-energy flux and the interface velocity v_i-bar.
@@ -111,7 +170,47 @@ template <class R> struct FaceFlux {
   R vbar;
 };
 
-// HLLD (riemann/EnzoRiemannHLLD.hpp:40-448)
+// HLLD (riemann/EnzoRiemannHLLD.hpp:40-448).  The flux is that of one side:
+// F_L or F_R, plus the jump terms of that side's star states, by the signs of
+// the five wave speeds.  So the speeds come first, and only the states that
+// the flux of this face is made of are formed: the side's own star state, and
+// the other side's only where the double-star state is needed.  Every value
+// that is formed is the reference's expression on the same operands, so the
+// result is the same bit for bit; on GB300, whose FP64 pipe bounds the FP64
+// stages, the operands' selection by integer moves is free.
+template <class R> struct HlldSide {
+  R d, u, vj, vk, by, bz, pt, e, sd, sdm_inv, sdm;  // left or right state
+  R st_d, st_inv;                                   // star density and 1 / it
+};
+template <class R> struct HlldStar {
+  R mx, my, mz, e, by, bz, vb;
+};
+template <class R>
+__device__ __forceinline__ HlldStar<R> hlld_star(const HlldSide<R>& W, R bxi, R bxsq, R spd2,
+                                                 R ptst, R thr) {
+  HlldStar<R> s;
+  s.mx = W.st_d * spd2;
+  const R den = W.d * W.sd * W.sdm - bxsq;
+  if (fabs(den) < thr) {
+    s.my = W.st_d * W.vj;
+    s.mz = W.st_d * W.vk;
+    s.by = W.by;
+    s.bz = W.bz;
+  } else {
+    R tmp = bxi * (W.sd - W.sdm) / den;
+    s.my = W.st_d * (W.vj - W.by * tmp);
+    s.mz = W.st_d * (W.vk - W.bz * tmp);
+    tmp = (W.d * (W.sd * W.sd) - bxsq) / den;
+    s.by = W.by * tmp;
+    s.bz = W.bz * tmp;
+  }
+  s.vb = (s.mx * bxi + (s.my * s.by + s.mz * s.bz)) * W.st_inv;
+  s.e = (W.sd * W.e - W.pt * W.u + ptst * spd2 +
+         bxi * (W.u * bxi + (W.vj * W.by + W.vk * W.bz) - s.vb)) *
+        W.sdm_inv;
+  return s;
+}
+
 template <class R>
 __device__ __forceinline__ void hlld(R g, const R* wli, const R* wri,
                                      FaceFlux<R>& out) {
@@ -122,197 +221,135 @@ __device__ __forceinline__ void hlld(R g, const R* wli, const R* wri,
   const R bxsq = bxi * bxi;
   const R pbl = R(0.5) * (bxsq + (wli[L_BJ] * wli[L_BJ] + wli[L_BK] * wli[L_BK]));
   const R pbr = R(0.5) * (bxsq + (wri[L_BJ] * wri[L_BJ] + wri[L_BK] * wri[L_BK]));
-  const R kel = R(0.5) * wli[L_RHO] *
-                (wli[L_VI] * wli[L_VI] +
-                 (wli[L_VJ] * wli[L_VJ] + wli[L_VK] * wli[L_VK]));
-  const R ker = R(0.5) * wri[L_RHO] *
-                (wri[L_VI] * wri[L_VI] +
-                 (wri[L_VJ] * wri[L_VJ] + wri[L_VK] * wri[L_VK]));
-  // conserved L/R states: d, mx, my, mz, e, by, bz
-  const R uld = wli[L_RHO], uld_mx = wli[L_VI] * uld, uld_my = wli[L_VJ] * uld,
-          uld_mz = wli[L_VK] * uld, ule = pressure_l * igm1 + kel + pbl,
-          ulby = wli[L_BJ], ulbz = wli[L_BK];
-  const R urd = wri[L_RHO], urd_mx = wri[L_VI] * urd, urd_my = wri[L_VJ] * urd,
-          urd_mz = wri[L_VK] * urd, ure = pressure_r * igm1 + ker + pbr,
-          urby = wri[L_BJ], urbz = wri[L_BK];
 
   const R cfl = cfast(g, wli[L_RHO], pressure_l, wli[L_BI], wli[L_BJ], wli[L_BK]);
   const R cfr = cfast(g, wri[L_RHO], pressure_r, wri[L_BI], wri[L_BJ], wri[L_BK]);
-  R spd0 = smin(wli[L_VI] - cfl, wri[L_VI] - cfr);
-  R spd4 = smax(wli[L_VI] + cfl, wri[L_VI] + cfr);
-
+  const R spd0 = smin(wli[L_VI] - cfl, wri[L_VI] - cfr);
+  const R spd4 = smax(wli[L_VI] + cfl, wri[L_VI] + cfr);
+  const R uld = wli[L_RHO], urd = wri[L_RHO];
   const R ptl = pressure_l + pbl;
   const R ptr = pressure_r + pbr;
-  const R fld = uld_mx;
-  const R flmx = uld_mx * wli[L_VI] + ptl - bxsq;
-  const R flmy = uld_my * wli[L_VI] - bxi * ulby;
-  const R flmz = uld_mz * wli[L_VI] - bxi * ulbz;
-  const R fle = wli[L_VI] * (ule + ptl - bxsq) -
-                bxi * (wli[L_VJ] * ulby + wli[L_VK] * ulbz);
-  const R flby = ulby * wli[L_VI] - bxi * wli[L_VJ];
-  const R flbz = ulbz * wli[L_VI] - bxi * wli[L_VK];
-  const R frd = urd_mx;
-  const R frmx = urd_mx * wri[L_VI] + ptr - bxsq;
-  const R frmy = urd_my * wri[L_VI] - bxi * urby;
-  const R frmz = urd_mz * wri[L_VI] - bxi * urbz;
-  const R fre = wri[L_VI] * (ure + ptr - bxsq) -
-                bxi * (wri[L_VJ] * urby + wri[L_VK] * urbz);
-  const R frby = urby * wri[L_VI] - bxi * wri[L_VJ];
-  const R frbz = urbz * wri[L_VI] - bxi * wri[L_VK];
-
   const R sdl = spd0 - wli[L_VI];
   const R sdr = spd4 - wri[L_VI];
-  const R spd2 = (sdr * urd_mx - sdl * uld_mx + (ptl - ptr)) /
+  const R sddl = uld * sdl, sddr = urd * sdr;
+  const R spd2 = (sdr * (wri[L_VI] * urd) - sdl * (wli[L_VI] * uld) + (ptl - ptr)) /
                  (sdr * urd - sdl * uld);
-  const R sdml = spd0 - spd2;
-  const R sdmr = spd4 - spd2;
-  const R sdml_inv = R(1.0) / sdml;
-  const R sdmr_inv = R(1.0) / sdmr;
-  R lst_d = uld * sdl * sdml_inv;
-  R rst_d = urd * sdr * sdmr_inv;
-  const R lst_d_inv = R(1.0) / lst_d;
-  const R rst_d_inv = R(1.0) / rst_d;
-  const R sqrtdl = sqrt(lst_d);
-  const R sqrtdr = sqrt(rst_d);
-  const R spd1 = spd2 - fabs(bxi) / sqrtdl;
-  const R spd3 = spd2 + fabs(bxi) / sqrtdr;
+  // the reference's order of the cases: F_L (spd0 >= 0), F_R (spd4 <= 0), then
+  // left star states for spd2 >= 0 and right ones otherwise
+  const bool sup_l = ge0(spd0), outer = sup_l || le0(spd4);
+  const bool left = sup_l || (!outer && ge0(spd2));
 
-  const R ptstl = ptl + uld * sdl * (spd2 - wli[L_VI]);
-  const R ptstr = ptr + urd * sdr * (spd2 - wri[L_VI]);
-  const R ptst = R(0.5) * (ptstr + ptstl);
-
-  R lst_mx = lst_d * spd2, lst_my, lst_mz, lst_by, lst_bz;
-  if (fabs(uld * sdl * sdml - bxsq) < SMALL * ptst) {
-    lst_my = lst_d * wli[L_VJ];
-    lst_mz = lst_d * wli[L_VK];
-    lst_by = ulby;
-    lst_bz = ulbz;
-  } else {
-    R tmp = bxi * (sdl - sdml) / (uld * sdl * sdml - bxsq);
-    lst_my = lst_d * (wli[L_VJ] - ulby * tmp);
-    lst_mz = lst_d * (wli[L_VK] - ulbz * tmp);
-    tmp = (uld * (sdl * sdl) - bxsq) / (uld * sdl * sdml - bxsq);
-    lst_by = ulby * tmp;
-    lst_bz = ulbz * tmp;
+  HlldSide<R> W;  // the side whose flux this is
+  W.d = left ? uld : urd;
+  W.u = left ? wli[L_VI] : wri[L_VI];
+  W.vj = left ? wli[L_VJ] : wri[L_VJ];
+  W.vk = left ? wli[L_VK] : wri[L_VK];
+  W.by = left ? wli[L_BJ] : wri[L_BJ];
+  W.bz = left ? wli[L_BK] : wri[L_BK];
+  W.pt = left ? ptl : ptr;
+  W.sd = left ? sdl : sdr;
+  const R mx = W.u * W.d, my = W.vj * W.d, mz = W.vk * W.d;
+  {
+    const R ke = R(0.5) * W.d * (W.u * W.u + (W.vj * W.vj + W.vk * W.vk));
+    W.e = (left ? pressure_l : pressure_r) * igm1 + ke + (left ? pbl : pbr);
   }
-  const R vbstl = (lst_mx * bxi + (lst_my * lst_by + lst_mz * lst_bz)) * lst_d_inv;
-  R lst_e = (sdl * ule - ptl * wli[L_VI] + ptst * spd2 +
-             bxi * (wli[L_VI] * bxi + (wli[L_VJ] * ulby + wli[L_VK] * ulbz) -
-                    vbstl)) *
-            sdml_inv;
+  R f[7];
+  f[0] = mx;
+  f[1] = mx * W.u + W.pt - bxsq;
+  f[2] = my * W.u - bxi * W.by;
+  f[3] = mz * W.u - bxi * W.bz;
+  f[4] = W.u * (W.e + W.pt - bxsq) - bxi * (W.vj * W.by + W.vk * W.bz);
+  f[5] = W.by * W.u - bxi * W.vj;
+  f[6] = W.bz * W.u - bxi * W.vk;
 
-  R rst_mx = rst_d * spd2, rst_my, rst_mz, rst_by, rst_bz;
-  if (fabs(urd * sdr * sdmr - bxsq) < SMALL * ptst) {
-    rst_my = rst_d * wri[L_VJ];
-    rst_mz = rst_d * wri[L_VK];
-    rst_by = urby;
-    rst_bz = urbz;
-  } else {
-    R tmp = bxi * (sdr - sdmr) / (urd * sdr * sdmr - bxsq);
-    rst_my = rst_d * (wri[L_VJ] - urby * tmp);
-    rst_mz = rst_d * (wri[L_VK] - urbz * tmp);
-    tmp = (urd * (sdr * sdr) - bxsq) / (urd * sdr * sdmr - bxsq);
-    rst_by = urby * tmp;
-    rst_bz = urbz * tmp;
+  if (!outer) {
+    const R ptstl = ptl + sddl * (spd2 - wli[L_VI]);
+    const R ptstr = ptr + sddr * (spd2 - wri[L_VI]);
+    const R ptst = R(0.5) * (ptstr + ptstl);
+    const R thr = SMALL * ptst;
+    const R spdo = left ? spd0 : spd4;  // the side's outermost speed
+    W.sdm = spdo - spd2;
+    W.sdm_inv = R(1.0) / W.sdm;
+    W.st_d = W.d * W.sd * W.sdm_inv;
+    W.st_inv = R(1.0) / W.st_d;
+    const R sq = sqrt(W.st_d);
+    const R va = fabs(bxi) / sq;
+    const R spdi = spd2 + (left ? -va : va);  // its Alfven speed (spd1 / spd3)
+    const bool two = left ? !ge0(spdi) : gt0(spdi);
+    const HlldStar<R> st = hlld_star(W, bxi, bxsq, spd2, ptst, thr);
+    f[0] = f[0] + spdo * (W.st_d - W.d);
+    f[1] = f[1] + spdo * (st.mx - mx);
+    f[2] = f[2] + spdo * (st.my - my);
+    f[3] = f[3] + spdo * (st.mz - mz);
+    f[4] = f[4] + spdo * (st.e - W.e);
+    f[5] = f[5] + spdo * (st.by - W.by);
+    f[6] = f[6] + spdo * (st.bz - W.bz);
+    if (two) {
+      R dy = st.my, dz = st.mz, de = st.e, dby = st.by, dbz = st.bz;
+      if (!(R(0.5) * bxsq < thr)) {
+        HlldSide<R> V;  // the other side
+        V.d = left ? urd : uld;
+        V.u = left ? wri[L_VI] : wli[L_VI];
+        V.vj = left ? wri[L_VJ] : wli[L_VJ];
+        V.vk = left ? wri[L_VK] : wli[L_VK];
+        V.by = left ? wri[L_BJ] : wli[L_BJ];
+        V.bz = left ? wri[L_BK] : wli[L_BK];
+        V.sd = left ? sdr : sdl;
+        V.sdm = (left ? spd4 : spd0) - spd2;
+        V.sdm_inv = R(1.0) / V.sdm;
+        V.st_d = V.d * V.sd * V.sdm_inv;
+        V.st_inv = R(1.0) / V.st_d;
+        V.pt = V.e = R(0);  // its energy is not needed
+        const R sqv = sqrt(V.st_d);
+        const HlldStar<R> sv = hlld_star(V, bxi, bxsq, spd2, ptst, thr);
+        // left and right values, in the reference's expressions
+        const R sqrtdl = left ? sq : sqv, sqrtdr = left ? sqv : sq;
+        const R invsumd = R(1.0) / (sqrtdl + sqrtdr);
+        const R bxsig = gt0(bxi) ? R(1.0) : R(-1.0);
+        const R vy = st.my * W.st_inv, vz = st.mz * W.st_inv;
+        const R oy = sv.my * V.st_inv, oz = sv.mz * V.st_inv;
+        const R lvy = left ? vy : oy, rvy = left ? oy : vy;
+        const R lvz = left ? vz : oz, rvz = left ? oz : vz;
+        const R lby = left ? st.by : sv.by, rby = left ? sv.by : st.by;
+        const R lbz = left ? st.bz : sv.bz, rbz = left ? sv.bz : st.bz;
+        const R lst_d = left ? W.st_d : V.st_d;
+        const R ty = invsumd * (sqrtdl * lvy + sqrtdr * rvy + bxsig * (rby - lby));
+        const R tz = invsumd * (sqrtdl * lvz + sqrtdr * rvz + bxsig * (rbz - lbz));
+        const R sqlr = bxsig * sqrtdl * sqrtdr;
+        dby = invsumd * (sqrtdl * rby + sqrtdr * lby + sqlr * (rvy - lvy));
+        dbz = invsumd * (sqrtdl * rbz + sqrtdr * lbz + sqlr * (rvz - lvz));
+        dy = W.st_d * ty;
+        dz = W.st_d * tz;
+        // v** . B**, from the left side's values for both sides
+        const R vb = spd2 * bxi + ((lst_d * ty) * dby + (lst_d * tz) * dbz) / lst_d;
+        const R t = sq * bxsig * (st.vb - vb);
+        de = st.e + (left ? -t : t);
+      }
+      f[0] = f[0] + spdi * (W.st_d - W.st_d);
+      f[1] = f[1] + spdi * (st.mx - st.mx);
+      f[2] = f[2] + spdi * (dy - st.my);
+      f[3] = f[3] + spdi * (dz - st.mz);
+      f[4] = f[4] + spdi * (de - st.e);
+      f[5] = f[5] + spdi * (dby - st.by);
+      f[6] = f[6] + spdi * (dbz - st.bz);
+    }
   }
-  const R vbstr = (rst_mx * bxi + (rst_my * rst_by + rst_mz * rst_bz)) * rst_d_inv;
-  R rst_e = (sdr * ure - ptr * wri[L_VI] + ptst * spd2 +
-             bxi * (wri[L_VI] * bxi + (wri[L_VJ] * urby + wri[L_VK] * urbz) -
-                    vbstr)) *
-            sdmr_inv;
-
-  R ldst_d, ldst_mx, ldst_my, ldst_mz, ldst_e, ldst_by, ldst_bz;
-  R rdst_d, rdst_mx, rdst_my, rdst_mz, rdst_e, rdst_by, rdst_bz;
-  if (R(0.5) * bxsq < SMALL * ptst) {
-    ldst_d = lst_d; ldst_mx = lst_mx; ldst_my = lst_my; ldst_mz = lst_mz;
-    ldst_e = lst_e; ldst_by = lst_by; ldst_bz = lst_bz;
-    rdst_d = rst_d; rdst_mx = rst_mx; rdst_my = rst_my; rdst_mz = rst_mz;
-    rdst_e = rst_e; rdst_by = rst_by; rdst_bz = rst_bz;
-  } else {
-    const R invsumd = R(1.0) / (sqrtdl + sqrtdr);
-    const R bxsig = (bxi > R(0.0) ? R(1.0) : R(-1.0));
-    ldst_d = lst_d;
-    rdst_d = rst_d;
-    ldst_mx = lst_mx;
-    rdst_mx = rst_mx;
-    R tmp = invsumd * (sqrtdl * (lst_my * lst_d_inv) +
-                       sqrtdr * (rst_my * rst_d_inv) + bxsig * (rst_by - lst_by));
-    ldst_my = ldst_d * tmp;
-    rdst_my = rdst_d * tmp;
-    tmp = invsumd * (sqrtdl * (lst_mz * lst_d_inv) +
-                     sqrtdr * (rst_mz * rst_d_inv) + bxsig * (rst_bz - lst_bz));
-    ldst_mz = ldst_d * tmp;
-    rdst_mz = rdst_d * tmp;
-    tmp = invsumd * (sqrtdl * rst_by + sqrtdr * lst_by +
-                     bxsig * sqrtdl * sqrtdr *
-                         ((rst_my * rst_d_inv) - (lst_my * lst_d_inv)));
-    ldst_by = rdst_by = tmp;
-    tmp = invsumd * (sqrtdl * rst_bz + sqrtdr * lst_bz +
-                     bxsig * sqrtdl * sqrtdr *
-                         ((rst_mz * rst_d_inv) - (lst_mz * lst_d_inv)));
-    ldst_bz = rdst_bz = tmp;
-    tmp = spd2 * bxi + (ldst_my * ldst_by + ldst_mz * ldst_bz) / ldst_d;
-    ldst_e = lst_e - sqrtdl * bxsig * (vbstl - tmp);
-    rdst_e = rst_e + sqrtdr * bxsig * (vbstr - tmp);
-  }
-
-  // jump terms S*(U* - U) (step 6, :308-339)
-  const R jl2_d = spd1 * (ldst_d - lst_d), jl2_mx = spd1 * (ldst_mx - lst_mx),
-          jl2_my = spd1 * (ldst_my - lst_my), jl2_mz = spd1 * (ldst_mz - lst_mz),
-          jl2_e = spd1 * (ldst_e - lst_e), jl2_by = spd1 * (ldst_by - lst_by),
-          jl2_bz = spd1 * (ldst_bz - lst_bz);
-  const R jl1_d = spd0 * (lst_d - uld), jl1_mx = spd0 * (lst_mx - uld_mx),
-          jl1_my = spd0 * (lst_my - uld_my), jl1_mz = spd0 * (lst_mz - uld_mz),
-          jl1_e = spd0 * (lst_e - ule), jl1_by = spd0 * (lst_by - ulby),
-          jl1_bz = spd0 * (lst_bz - ulbz);
-  const R jr2_d = spd3 * (rdst_d - rst_d), jr2_mx = spd3 * (rdst_mx - rst_mx),
-          jr2_my = spd3 * (rdst_my - rst_my), jr2_mz = spd3 * (rdst_mz - rst_mz),
-          jr2_e = spd3 * (rdst_e - rst_e), jr2_by = spd3 * (rdst_by - rst_by),
-          jr2_bz = spd3 * (rdst_bz - rst_bz);
-  const R jr1_d = spd4 * (rst_d - urd), jr1_mx = spd4 * (rst_mx - urd_mx),
-          jr1_my = spd4 * (rst_my - urd_my), jr1_mz = spd4 * (rst_mz - urd_mz),
-          jr1_e = spd4 * (rst_e - ure), jr1_by = spd4 * (rst_by - urby),
-          jr1_bz = spd4 * (rst_bz - urbz);
-
-  R* f = out.f;
-  if (spd0 >= R(0.0)) {
-    f[L_RHO] = fld; f[L_VI] = flmx; f[L_VJ] = flmy; f[L_VK] = flmz;
-    f[L_E] = fle; f[L_BJ] = flby; f[L_BK] = flbz;
-  } else if (spd4 <= R(0.0)) {
-    f[L_RHO] = frd; f[L_VI] = frmx; f[L_VJ] = frmy; f[L_VK] = frmz;
-    f[L_E] = fre; f[L_BJ] = frby; f[L_BK] = frbz;
-  } else if (spd1 >= R(0.0)) {
-    f[L_RHO] = fld + jl1_d; f[L_VI] = flmx + jl1_mx; f[L_VJ] = flmy + jl1_my;
-    f[L_VK] = flmz + jl1_mz; f[L_E] = fle + jl1_e; f[L_BJ] = flby + jl1_by;
-    f[L_BK] = flbz + jl1_bz;
-  } else if (spd2 >= R(0.0)) {
-    f[L_RHO] = fld + jl1_d + jl2_d; f[L_VI] = flmx + jl1_mx + jl2_mx;
-    f[L_VJ] = flmy + jl1_my + jl2_my; f[L_VK] = flmz + jl1_mz + jl2_mz;
-    f[L_E] = fle + jl1_e + jl2_e; f[L_BJ] = flby + jl1_by + jl2_by;
-    f[L_BK] = flbz + jl1_bz + jl2_bz;
-  } else if (spd3 > R(0.0)) {
-    f[L_RHO] = frd + jr1_d + jr2_d; f[L_VI] = frmx + jr1_mx + jr2_mx;
-    f[L_VJ] = frmy + jr1_my + jr2_my; f[L_VK] = frmz + jr1_mz + jr2_mz;
-    f[L_E] = fre + jr1_e + jr2_e; f[L_BJ] = frby + jr1_by + jr2_by;
-    f[L_BK] = frbz + jr1_bz + jr2_bz;
-  } else {
-    f[L_RHO] = frd + jr1_d; f[L_VI] = frmx + jr1_mx; f[L_VJ] = frmy + jr1_my;
-    f[L_VK] = frmz + jr1_mz; f[L_E] = fre + jr1_e; f[L_BJ] = frby + jr1_by;
-    f[L_BK] = frbz + jr1_bz;
-  }
-  f[L_BI] = R(0.0);
-  out.eflux = eint_flux(g, wli[L_RHO], pressure_l, wri[L_RHO], pressure_r,
-                        f[L_RHO]);
-  const R l_coef = (spd0 - wli[L_VI]) / (spd0 - spd2);
-  const R r_coef = (spd4 - wri[L_VI]) / (spd4 - spd2);
-  if (spd0 > R(0)) {
+  out.f[L_RHO] = f[0];
+  out.f[L_BI] = R(0.0);
+  out.f[L_BJ] = f[5];
+  out.f[L_BK] = f[6];
+  out.f[L_VI] = f[1];
+  out.f[L_VJ] = f[2];
+  out.f[L_VK] = f[3];
+  out.f[L_E] = f[4];
+  out.eflux = eint_flux(g, wli[L_RHO], pressure_l, wri[L_RHO], pressure_r, f[0]);
+  if (gt0(spd0)) {
     out.vbar = wli[L_VI];
-  } else if (spd4 < R(0)) {
+  } else if (lt0(spd4)) {
     out.vbar = wri[L_VI];
-  } else if (spd2 >= R(0)) {
-    out.vbar = spd2 * l_coef;
   } else {
-    out.vbar = spd2 * r_coef;
+    const bool l = ge0(spd2);
+    out.vbar = spd2 * ((l ? sdl : sdr) / ((l ? spd0 : spd4) - spd2));
   }
 }
 

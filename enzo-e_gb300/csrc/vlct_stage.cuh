@@ -35,6 +35,10 @@
 // for the passive scalars' advection (EXTRA_ALL; the scalars themselves are
 // advected by passive_kernel, vlct_passive.cuh); the default one compiles
 // all of these out.
+//
+// FP64 runs this kernel only where the split kernels' workspace cannot be had
+// (vlct_split.cuh: the no-allocation step, or a GPU that is full); FP32, whose
+// arithmetic is 64 times cheaper, always does.
 #pragma once
 #include <type_traits>
 
@@ -75,7 +79,7 @@ __device__ __forceinline__ void cp_async_wait_all() {
 // Upwind weight of CT from the sign of the density flux
 // (EnzoBfieldMethodCT.cpp:198-213).
 template <class R> __device__ __forceinline__ R upw(R fd) {
-  return (fd > R(0)) ? R(1.0) : ((fd < R(0)) ? R(0.0) : R(0.5));
+  return gt0(fd) ? R(1.0) : (lt0(fd) ? R(0.0) : R(0.5));
 }
 
 // compute_edge_<true> (EnzoBfieldMethodCT.cpp:384-457)

@@ -48,6 +48,33 @@ struct StageTile {
   int xa, xb, ya, yb, za, zb;
 };
 
+// One unit of work of the split stages (vlct_split.cuh): the output planes
+// [za, zb) of one block over its whole x-y extent, and where its workspace
+// arrays start (in elements).
+struct SplitJob {
+  int block;
+  int za, zb;
+  size_t off;
+};
+// Jobs [first, first + count) of a list that share the workspace in one
+// launch; cells: the most workspace cells of one of them, total: of all.
+struct SplitGroup {
+  int first, count;
+  size_t cells, total;
+};
+// Workspace arrays of a split stage: pressure, cell-centred E, the face fluxes
+// of three directions, edge EMFs.
+constexpr int split_arrays(bool mhd, bool de) {
+  return 1 + (mhd ? 6 : 0) + 3 * (de ? 9 : (mhd ? 7 : 5));
+}
+// A split stage's work as the host launches it (ngroups = 0: the fused kernel).
+struct SplitLaunch {
+  const SplitJob* jobs = nullptr;  // device
+  const SplitGroup* groups = nullptr;  // host
+  int ngroups = 0;
+  void* ws = nullptr;
+};
+
 struct PhysParams {
   double gamma;
   double density_floor;
