@@ -74,9 +74,6 @@ struct mhdvlct_batch {
   void* d_aux[2] = {nullptr, nullptr};
   StageTile* d_tiles[2] = {nullptr, nullptr};
   int ntiles[2] = {0, 0};
-  int tile_tx[2] = {0, 0}, tile_ty[2] = {0, 0};
-  int tile_full[2] = {0, 0};  // 1: every tile of the stage is tile_tx x tile_ty
-  int block_m = 0;            // every block's extent along all axes, if equal; else 0
   int* d_queue = nullptr;     // 2 counters
   // FP64: the split stages' jobs and groups, and the workspace they share
   // (null when it could not be had: the fused kernels run instead)
@@ -119,7 +116,6 @@ struct mhdvlct_batch {
   double* d_diag = nullptr;   // diagnostics: partial rows then the 8 totals
   int diag_rows = 0;
   int grid = 0;               // persistent grid size (0 = fill the GPU)
-  int threads[2] = {256, 256};  // CTA size of each stage's launches
   std::map<std::vector<int>, TileChoice> tune;  // per block-size class
   cudaGraphExec_t graph[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
   // stream-ordered batch (a serving request's): every device allocation and
@@ -169,57 +165,48 @@ void drop_graphs(mhdvlct_batch* b) {
       }
 }
 
-TileChoice choice_for(const mhdvlct_batch* b, int i) {
-  std::vector<int> key(b->dims.begin() + 3 * i, b->dims.begin() + 3 * i + 3);
-  auto it = b->tune.find(key);
+// The work decomposition of blocks of ghosted extents m: the one tuned or set
+// for their class, or the default.  The default is the tile that covers the
+// block with the least work, whole columns of it, when all blocks' columns
+// fill the GPU at least twice over (`columns`, per stage); a smaller batch (a
+// few large blocks, e.g. one serving request) takes the tile and z-chunk that
+// fill it best.
+TileChoice choice_for(const mhdvlct_batch* b, const std::vector<int>& cls, const long columns[2]) {
+  auto it = b->tune.find(cls);
+  if (it != b->tune.end()) return it->second;
   TileChoice c;
-  const bool tuned = it != b->tune.end();
-  if (tuned) c = it->second;
   const StagePlan sp = stage_plan(b->h);
-  for (int s = 0; s < 2; s++)
-    if (c.tile_x[s] <= 0 || c.tile_y[s] <= 0) {
-      default_tile_xy(b->dtype, b->h->solver, sp.recon[s], b->h->de, c.tile_x[s],
-                      c.tile_y[s]);
-    }
-  if (!tuned) {
-    // untuned default: when the batch has too few column tiles to fill the
-    // GPU (a few large blocks, e.g. one serving request), cut the columns
-    // into z-chunks so that a stage has about two waves of tiles
-    // SM count of the current device (thread-safe one-time initialisation)
-    static const int nsm = [] {
-      int dev = 0, n = 0;
-      cudaGetDevice(&dev);
-      if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-          n <= 0)
-        n = 1;
-      return n;
-    }();
-    const int target = 4 * nsm;
-    auto columns_of = [&](int tx, int ty) {
-      long columns = 0;
-      for (int k = 0; k < b->nblocks; k++) {
-        const int mx = b->dims[3 * k] + 2 * b->g, my = b->dims[3 * k + 1] + 2 * b->g;
-        columns += (long)((mx + tx - 1) / tx) * ((my + ty - 1) / ty);
-      }
-      return columns;
-    };
-    for (int s = 0; s < 2; s++) {
-      long columns = columns_of(c.tile_x[s], c.tile_y[s]);
-      if (columns < target && c.tile_x[s] != c.tile_y[s]) {
-        // a batch too small to fill the GPU with the large rectangular
-        // tiles: the smaller square tile (several CTAs per SM) instead
-        const int t = default_tile(b->dtype, b->h->solver, sp.recon[s], b->h->de);
-        c.tile_x[s] = c.tile_y[s] = t;
-        columns = columns_of(t, t);
-      }
-      const int mz = b->dims[3 * i + 2] + 2 * b->g;
-      if (columns < target && mz > 24) {
-        const long chunks = (target + columns - 1) / columns;
-        c.zchunk[s] = std::max(8, (int)((mz + chunks - 1) / chunks));
-      }
-    }
+  const int m[3] = {cls[0] + 2 * b->g, cls[1] + 2 * b->g, cls[2] + 2 * b->g};
+  for (int s = 0; s < 2; s++) {
+    const StageKind k = stage_kind(b->h, b->dtype, s);
+    if (columns[s] >= 2L * k.ctas() * sm_count()) continue;
+    const Decomp d = decompose(k, stage_window(m, sp.S[s], s == 1), b->nblocks);
+    c.tile_x[s] = d.tx;
+    c.tile_y[s] = d.ty;
+    c.zchunk[s] = d.zchunk;
   }
   return c;
+}
+
+std::vector<int> class_of(const mhdvlct_batch* b, int i) {
+  return std::vector<int>(b->dims.begin() + 3 * i, b->dims.begin() + 3 * i + 3);
+}
+
+// The decomposition of every block-size class of the batch.
+std::map<std::vector<int>, TileChoice> choices(const mhdvlct_batch* b) {
+  std::map<std::vector<int>, long> count;
+  for (int i = 0; i < b->nblocks; i++) count[class_of(b, i)]++;
+  const StagePlan sp = stage_plan(b->h);
+  long columns[2] = {0, 0};
+  for (const auto& k : count)
+    for (int s = 0; s < 2; s++) {
+      const int m[3] = {k.first[0] + 2 * b->g, k.first[1] + 2 * b->g, k.first[2] + 2 * b->g};
+      const Window w = stage_window(m, sp.S[s], s == 1);
+      columns[s] += k.second * tile_columns(stage_kind(b->h, b->dtype, s), w.len[0], w.len[1], 0, 0);
+    }
+  std::map<std::vector<int>, TileChoice> out;
+  for (const auto& k : count) out[k.first] = choice_for(b, k.first, columns);
+  return out;
 }
 
 // (Re)build the descriptor arrays and tile lists on the device.
@@ -231,8 +218,9 @@ int build_descriptors(mhdvlct_batch* b, cudaStream_t st) {
   std::vector<StageBlock<R>> sb[2][2];
   std::vector<AuxBlock<R>> aux[2];
   std::vector<StageTile> tiles[2];
-  int tx[2] = {1, 1}, ty[2] = {1, 1};
   std::vector<std::pair<double, StageTile>> order[2];
+  const std::map<std::vector<int>, TileChoice> choice = choices(b);
+  const StageKind kind[2] = {stage_kind(b->h, b->dtype, 0), stage_kind(b->h, b->dtype, 1)};
   for (int i = 0; i < b->nblocks; i++) {
     const auto& O = b->off[i];
     FieldSet<R> ext, tmp;
@@ -288,31 +276,16 @@ int build_descriptors(mhdvlct_batch* b, cudaStream_t st) {
       for (int d = 0; d < 3; d++) A.accel[d] = b->gravity ? b->ptr<R>(O.acc[d]) : nullptr;
       aux[p].push_back(A);
     }
-    const TileChoice c = choice_for(b, i);
+    const TileChoice& c = choice.at(class_of(b, i));
     for (int s = 0; s < 2; s++) {
       std::vector<StageTile> t;
-      make_tiles(i, O.m, sp.S[s], s == 1, c.tile_x[s], c.tile_y[s], c.zchunk[s], t);
+      make_tiles(kind[s], i, O.m, sp.S[s], s == 1, c.tile_x[s], c.tile_y[s], c.zchunk[s], t);
       for (auto& x : t) {
-        tx[s] = std::max(tx[s], x.xb - x.xa);
-        ty[s] = std::max(ty[s], x.yb - x.ya);
         const double cost = (double)(x.xb - x.xa + 2) * (x.yb - x.ya + 2) *
                             (x.zb - x.za + 2);
         order[s].push_back({cost, x});
       }
     }
-  }
-  // the launch shape: every tile at the largest extent; one cubic extent
-  // shared by every block
-  int block_m = b->off[0].m[0];
-  for (int i = 0; i < b->nblocks; i++)
-    for (int a = 0; a < 3; a++)
-      if (b->off[i].m[a] != block_m) block_m = 0;
-  b->block_m = block_m;
-  for (int s = 0; s < 2; s++) {
-    b->tile_full[s] = 1;
-    for (auto& o : order[s])
-      if (o.second.xb - o.second.xa != tx[s] || o.second.yb - o.second.ya != ty[s])
-        b->tile_full[s] = 0;
   }
   for (int s = 0; s < 2; s++) {
     std::stable_sort(order[s].begin(), order[s].end(),
@@ -321,8 +294,6 @@ int build_descriptors(mhdvlct_batch* b, cudaStream_t st) {
     for (auto& o : order[s]) tiles[s].push_back(o.second);
     b->ntiles[s] = (int)tiles[s].size();
     if (s == 1) b->h_tiles1 = tiles[s];
-    b->tile_tx[s] = tx[s];
-    b->tile_ty[s] = ty[s];
   }
   st = setup_stream(b, st);
   auto upload = [&](void** dst, const void* src, size_t bytes) -> int {
@@ -386,18 +357,13 @@ StageInfo batch_stage_info(const mhdvlct_batch* b, int s, int* queue) {
   info.S = sp.S[s];
   info.final_stage = s == 1;
   info.dt_factor = sp.dt_factor[s];
-  info.tx = b->tile_tx[s];
-  info.ty = b->tile_ty[s];
   info.queue = queue;
-  info.threads = b->threads[s];
   info.block_fc = (s == 1 && b->fc_on) ? 1 : 0;
   info.fc_g = b->g;
   // the gravity source enters the full-dt stage only
   // (EnzoMHDIntegratorStageCommands.cpp:279)
   info.gravity = s == 1 ? b->gravity : 0;
   info.npass = b->npass;
-  info.full_tiles = b->tile_full[s];
-  info.block_m = b->block_m;
   return info;
 }
 
@@ -950,21 +916,17 @@ extern "C" int mhdvlct_batch_set_stage_tile(mhdvlct_batch* b, int stage, int til
   const int tmax = b->dtype == MHD_DTYPE_F64 ? TileLimits<double>::TMAX
                                              : TileLimits<float>::TMAX;
   if (tile_x > tmax || tile_y > tmax) return bfail(b, MHD_ERR_INVALID, "tile too large");
-  const StagePlan sp = stage_plan(b->h);
-  const int tmax_threads = b->dtype == MHD_DTYPE_F64
-                               ? stage_max_threads<double>(sp.recon[stage])
-                               : stage_max_threads<float>(sp.recon[stage]);
-  if (threads != 0 && threads != 256 && !(threads == 512 && tmax_threads >= 512))
+  // the CTA's size is the kernel's own; the two an older form took still pass
+  if (threads != 0 && threads != 256 &&
+      !(threads == 512 && b->dtype == MHD_DTYPE_F32 && stage_plan(b->h).recon[stage] != RECON_NN))
     return bfail(b, MHD_ERR_INVALID, "threads must be 256 (or 512 where the stage allows it)");
-  for (int i = 0; i < b->nblocks; i++) {
-    std::vector<int> key(b->dims.begin() + 3 * i, b->dims.begin() + 3 * i + 3);
-    TileChoice c = choice_for(b, i);
+  for (const auto& k : choices(b)) {
+    TileChoice c = k.second;
     c.tile_x[stage] = tile_x;
     c.tile_y[stage] = tile_y;
     c.zchunk[stage] = zchunk;
-    b->tune[key] = c;
+    b->tune[k.first] = c;
   }
-  b->threads[stage] = threads ? threads : 256;
   return build_descriptors_any(b, 0);
 }
 
@@ -1272,7 +1234,6 @@ int autotune_t(mhdvlct_batch* b, int reps, std::string& json, cudaStream_t st) {
                                                const std::vector<int>& c) {
     return (long)a[0] * a[1] * a[2] > (long)c[0] * c[1] * c[2];
   });
-  const size_t smem_cap = 227 * 1024;
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
@@ -1289,41 +1250,26 @@ int autotune_t(mhdvlct_batch* b, int reps, std::string& json, cudaStream_t st) {
     }
     std::sort(shapes.begin(), shapes.end());
     shapes.erase(std::unique(shapes.begin(), shapes.end()), shapes.end());
-    int rep_block = 0;
-    for (int i = 0; i < b->nblocks; i++)
-      if (b->dims[3 * i] == cls[0] && b->dims[3 * i + 1] == cls[1] &&
-          b->dims[3 * i + 2] == cls[2]) {
-        rep_block = i;
-        break;
-      }
-    TileChoice bestc = choice_for(b, rep_block);
+    TileChoice bestc = choices(b).at(cls);
     float best_stage[2] = {0.f, 0.f};
     size_t ncand = 0;
     // the stages are tuned one after the other (each candidate is timed on
     // the whole two-stage step, the other stage at its current choice)
     for (int s = 0; s < 2; s++) {
-      // one launch serves every class, so its shared memory is sized by the
-      // largest tile extents over all classes: a candidate is kept only if
-      // that combined shape fits
-      int other_tx = 1, other_ty = 1;
-      for (int i = 0; i < b->nblocks; i++) {
-        if (b->dims[3 * i] == cls[0] && b->dims[3 * i + 1] == cls[1] &&
-            b->dims[3 * i + 2] == cls[2])
-          continue;
-        const TileChoice oc = choice_for(b, i);
-        other_tx = std::max(other_tx, oc.tile_x[s]);
-        other_ty = std::max(other_ty, oc.tile_y[s]);
-      }
       std::vector<TileChoice> cands;
       // the split FP64 stages have no tiles: the choice in force is the only
       // candidate
       if (b->d_ws) cands.push_back(bestc);
-      for (auto& sh : shapes) {
-        if (b->d_ws) break;
-        if (stage_smem<R>(b->h->solver, sp.recon[s], b->h->de != 0,
-                          std::max(sh.first, other_tx), std::max(sh.second, other_ty)) >
-            smem_cap)
-          continue;
+      // the least-work tile, then each shape, as the fused kernel takes them
+      const int m[3] = {cls[0] + 2 * b->g, cls[1] + 2 * b->g, cls[2] + 2 * b->g};
+      const Window w = stage_window(m, sp.S[s], s == 1);
+      std::vector<std::pair<int, int>> seen;
+      shapes.insert(shapes.begin(), {0, 0});
+      for (auto sh : shapes) {
+        if (b->d_ws || w.len[0] <= 0 || w.len[1] <= 0) break;
+        fit_tile(stage_kind(b->h, b->dtype, s), w.len[0], w.len[1], sh.first, sh.second);
+        if (std::find(seen.begin(), seen.end(), sh) != seen.end()) continue;
+        seen.push_back(sh);
         for (int zc : {0, 16}) {
           if (zc && zc >= cls[2]) continue;
           TileChoice c = bestc;
@@ -1333,55 +1279,60 @@ int autotune_t(mhdvlct_batch* b, int reps, std::string& json, cudaStream_t st) {
           cands.push_back(c);
         }
       }
+      if (cands.empty()) cands.push_back(bestc);
+      shapes.erase(shapes.begin());
       float best = 1e30f;
-      int best_threads = b->threads[s];
-      for (int threads : {256, 512}) {
-        if (threads > stage_max_threads<R>(sp.recon[s])) continue;
-        b->threads[s] = threads;
-        for (const auto& c : cands) {
-          ncand++;
-          b->tune[cls] = c;
-          if (int rc = build_descriptors<R>(b, st)) {
-            bfree(b, save);
-            return rc;
-          }
-          // one untimed step, then reps timed steps
-          e = launch_stages<R>(b, st);
-          cudaEventRecord(e0, st);
-          for (int r = 0; r < reps && e == cudaSuccess; r++) e = launch_stages<R>(b, st);
-          cudaEventRecord(e1, st);
-          cudaEventSynchronize(e1);
-          cudaMemcpyAsync(b->pool, save, bytes, cudaMemcpyDeviceToDevice, st);
-          if (e == cudaErrorInvalidValue || e == cudaErrorInvalidConfiguration) {
-            // a launch shape this GPU refuses (nothing ran): skip the candidate
-            e = cudaSuccess;
-            continue;
-          }
-          if (e != cudaSuccess) break;
-          float t;
-          cudaEventElapsedTime(&t, e0, e1);
-          if (t < best) {
-            best = t;
-            bestc = c;
-            best_threads = threads;
-          }
+      for (const auto& c : cands) {
+        ncand++;
+        b->tune[cls] = c;
+        if (int rc = build_descriptors<R>(b, st)) {
+          bfree(b, save);
+          return rc;
+        }
+        // one untimed step, then reps timed steps
+        e = launch_stages<R>(b, st);
+        cudaEventRecord(e0, st);
+        for (int r = 0; r < reps && e == cudaSuccess; r++) e = launch_stages<R>(b, st);
+        cudaEventRecord(e1, st);
+        cudaEventSynchronize(e1);
+        cudaMemcpyAsync(b->pool, save, bytes, cudaMemcpyDeviceToDevice, st);
+        if (e == cudaErrorInvalidValue || e == cudaErrorInvalidConfiguration) {
+          // a launch shape this GPU refuses (nothing ran): skip the candidate
+          e = cudaSuccess;
+          continue;
         }
         if (e != cudaSuccess) break;
+        float t;
+        cudaEventElapsedTime(&t, e0, e1);
+        if (t < best) {
+          best = t;
+          bestc = c;
+        }
       }
-      b->threads[s] = best_threads;
       b->tune[cls] = bestc;
       best_stage[s] = best / std::max(1, reps);
       if (e != cudaSuccess) break;
     }
+    // the tiles in force: what the fused kernel makes of the choices
+    const int m[3] = {cls[0] + 2 * b->g, cls[1] + 2 * b->g, cls[2] + 2 * b->g};
+    int shape[2][2];
+    for (int k = 0; k < 2; k++) {
+      const Window w = stage_window(m, sp.S[k], k == 1);
+      shape[k][0] = bestc.tile_x[k];
+      shape[k][1] = bestc.tile_y[k];
+      fit_tile(stage_kind(b->h, b->dtype, k), w.len[0], w.len[1], shape[k][0], shape[k][1]);
+    }
+    const int threads[2] = {stage_kind(b->h, b->dtype, 0).threads(),
+                            stage_kind(b->h, b->dtype, 1).threads()};
     char buf[512];
     std::snprintf(buf, sizeof(buf),
                   "%s\"%dx%dx%d\": {\"stage1\": {\"tile_x\": %d, \"tile_y\": %d, "
                   "\"zchunk\": %d, \"threads\": %d}, \"stage2\": {\"tile_x\": %d, "
                   "\"tile_y\": %d, \"zchunk\": %d, \"threads\": %d}, "
                   "\"ms_per_step\": %.4f, \"candidates\": %zu}",
-                  first_cls ? "" : ", ", cls[0], cls[1], cls[2], bestc.tile_x[0],
-                  bestc.tile_y[0], bestc.zchunk[0], b->threads[0], bestc.tile_x[1],
-                  bestc.tile_y[1], bestc.zchunk[1], b->threads[1], best_stage[1], ncand);
+                  first_cls ? "" : ", ", cls[0], cls[1], cls[2], shape[0][0],
+                  shape[0][1], bestc.zchunk[0], threads[0], shape[1][0],
+                  shape[1][1], bestc.zchunk[1], threads[1], best_stage[1], ncand);
     json += buf;
     first_cls = false;
     if (e != cudaSuccess) break;

@@ -71,16 +71,102 @@ static void split(int lo, int hi, int t, std::vector<std::pair<int, int>>& out) 
   }
 }
 
-void make_tiles(int block, const int m[3], int S, bool final, int tile_x,
+StageKind stage_kind(const mhdvlct_handle* h, int dtype, int i) {
+  return StageKind{dtype == MHD_DTYPE_F64, stage_plan(h).recon[i] == RECON_NN, h->mhd != 0};
+}
+
+Window stage_window(const int m[3], int S, bool final) {
+  Window w;
+  w.lo = final ? S : S + 1;
+  for (int a = 0; a < 3; a++) w.len[a] = m[a] - 2 * w.lo;
+  return w;
+}
+
+int sm_count() {
+  static const int n = [] {
+    int dev = 0, v = 0;
+    cudaGetDevice(&dev);
+    if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0)
+      v = 1;
+    return v;
+  }();
+  return n;
+}
+
+static int parts_of(int len, int t) { return (len + t - 1) / t; }
+// Warps a tile of tx x ty columns keeps busy, and about one more for its
+// barriers.
+static double tile_cost(int tx, int ty) { return ((tx + 2) * (ty + 2) + 31) / 32 + 1.0; }
+
+void fit_tile(const StageKind& k, int lx, int ly, int& tx, int& ty) {
+  const int top = k.f64 ? TileLimits<double>::TMAX : TileLimits<float>::TMAX;
+  const int mx = std::min(lx, tx > 0 ? std::min(tx, top) : top);
+  const int my = std::min(ly, ty > 0 ? std::min(ty, top) : top);
+  double best = 1e300;
+  int bx = 1, by = 1;
+  for (int y = 1; y <= my; y++)
+    for (int x = 1; x <= mx; x++) {
+      const int ax = parts_of(lx, parts_of(lx, x)), ay = parts_of(ly, parts_of(ly, y));
+      if (!k.fits(ax, ay)) continue;
+      const double c = (double)parts_of(lx, ax) * parts_of(ly, ay) * tile_cost(ax, ay);
+      if (c <= best) {  // on ties the wider tile: longer rows to load
+        best = c;
+        bx = ax;
+        by = ay;
+      }
+    }
+  tx = bx;
+  ty = by;
+}
+
+long tile_columns(const StageKind& k, int lx, int ly, int tx, int ty) {
+  if (lx <= 0 || ly <= 0) return 0;
+  fit_tile(k, lx, ly, tx, ty);
+  return (long)parts_of(lx, tx) * parts_of(ly, ty);
+}
+
+// The tile and z-chunk that minimise a simple cost model: a chunk of L planes
+// costs L planes and about two and a half more (its prologue), a plane's time
+// a fixed part (latencies, barriers) and one that grows with the tile; chunks
+// run in waves of the CTAs the GPU holds at once.
+Decomp decompose(const StageKind& k, const Window& w, long nblocks) {
+  Decomp d;
+  if (w.len[0] <= 0 || w.len[1] <= 0 || w.len[2] <= 0) return d;
+  const long resident = (long)k.ctas() * sm_count();
+  const int full = k.threads();
+  const int top = k.f64 ? TileLimits<double>::TMAX : TileLimits<float>::TMAX;
+  double best = 1e300;
+  for (int y = 1; y <= std::min(top, w.len[1]); y++)
+    for (int x = 1; x <= std::min(top, w.len[0]); x++) {
+      const int ax = parts_of(w.len[0], parts_of(w.len[0], x));
+      const int ay = parts_of(w.len[1], parts_of(w.len[1], y));
+      if (ax != x || ay != y || !k.fits(ax, ay)) continue;
+      const long cols = (long)parts_of(w.len[0], ax) * parts_of(w.len[1], ay) * nblocks;
+      const double plane = 0.35 + 0.65 * ((ax + 2) * (ay + 2)) / full;
+      for (int L : {0, 32, 24, 16, 12, 8, 6, 4, 3, 2}) {
+        if (L >= w.len[2]) continue;
+        const int nz = L > 0 ? parts_of(w.len[2], L) : 1, tz = parts_of(w.len[2], nz);
+        const double cost = (double)((cols * nz + resident - 1) / resident) * plane * (tz + 2.5);
+        if (cost < best * 0.999) {  // on ties fewer chunks
+          best = cost;
+          d.tx = ax;
+          d.ty = ay;
+          d.zchunk = L;
+        }
+      }
+    }
+  return d;
+}
+
+void make_tiles(const StageKind& k, int block, const int m[3], int S, bool final, int tile_x,
                 int tile_y, int zchunk, std::vector<StageTile>& out) {
-  const int lo = final ? S : S + 1;
-  const int hi_x = final ? m[0] - S : m[0] - S - 1;
-  const int hi_y = final ? m[1] - S : m[1] - S - 1;
-  const int hi_z = final ? m[2] - S : m[2] - S - 1;
+  const Window w = stage_window(m, S, final);
+  if (w.len[0] <= 0 || w.len[1] <= 0 || w.len[2] <= 0) return;
+  fit_tile(k, w.len[0], w.len[1], tile_x, tile_y);
   std::vector<std::pair<int, int>> xs, ys, zs;
-  split(lo, hi_x, tile_x, xs);
-  split(lo, hi_y, tile_y, ys);
-  split(lo, hi_z, zchunk > 0 ? zchunk : (hi_z - lo), zs);
+  split(w.lo, w.lo + w.len[0], tile_x, xs);
+  split(w.lo, w.lo + w.len[1], tile_y, ys);
+  split(w.lo, w.lo + w.len[2], zchunk > 0 ? zchunk : w.len[2], zs);
   for (auto& z : zs)
     for (auto& y : ys)
       for (auto& x : xs)
@@ -152,37 +238,6 @@ FieldSet<R> fieldset_of(const MhdBlockView* b) {
 }
 template FieldSet<double> fieldset_of<double>(const MhdBlockView*);
 template FieldSet<float> fieldset_of<float>(const MhdBlockView*);
-
-int default_tile(int dtype, int solver, int recon, int de) {
-  // largest square tile whose shared memory fits the CTAs an SM holds at
-  // once (227 KB per SM): one CTA for FP64, three for the FP32 NN stage, two
-  // for the other FP32 stages
-  const int cap = (dtype == MHD_DTYPE_F64) ? 200 * 1024
-                  : (recon == RECON_NN)    ? 72 * 1024
-                                           : 110 * 1024;
-  int best = 4;
-  for (int t = 4; t <= (dtype == MHD_DTYPE_F64 ? TileLimits<double>::TMAX
-                                                 : TileLimits<float>::TMAX);
-       t++) {
-    const size_t b = (dtype == MHD_DTYPE_F64)
-                         ? stage_smem<double>(solver, recon, de != 0, t, t)
-                         : stage_smem<float>(solver, recon, de != 0, t, t);
-    if (b <= (size_t)cap) best = t;
-  }
-  return best;
-}
-
-void default_tile_xy(int dtype, int solver, int recon, int de, int& tx, int& ty) {
-  if (dtype == MHD_DTYPE_F32) {
-    // the shapes the autotuner settles on for 32^3 blocks: wide in x
-    // (coalesced rows), one large tile per SM; the tile split evens them
-    // out over other block sizes.  Both fit 227 KB with dual energy.
-    tx = recon == RECON_NN ? 34 : 24;
-    ty = recon == RECON_NN ? 10 : 16;
-    return;
-  }
-  tx = ty = default_tile(dtype, solver, recon, de);
-}
 
 }  // namespace mhdint
 
@@ -566,54 +621,22 @@ cudaError_t launch_make_tiles(StageTile* out, const TileSplit& sp, cudaStream_t 
   return cudaGetLastError();
 }
 
-// Work decomposition of one stage of the per-block path: the tile extent and
-// z-chunk that minimise a simple cost model for one block alone on the GPU.
-// A tile of t x t columns and L planes costs about (t+2)^2 (L + 1.5) (its
-// halo columns and the planes of its prologue); the tiles run in waves of
-// the CTAs the GPU holds at once (one per SM for FP64, two or three for
-// FP32), so the stage takes about waves x the largest tile's cost.
+// Work decomposition of the stages of the per-block path: one block alone on
+// the GPU.
 struct PlainDecomp {
-  int tile[2] = {8, 8};
+  int tx[2] = {8, 8}, ty[2] = {8, 8};
   int zchunk[2] = {0, 0};
 };
-int sm_count() {
-  static const int n = [] {
-    int dev = 0, v = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0)
-      v = 1;
-    return v;
-  }();
-  return n;
-}
 PlainDecomp plain_decomp(const mhdvlct_handle* h, const int m[3], int dtype) {
   PlainDecomp d;
   const StagePlan sp = stage_plan(h);
   for (int i = 0; i < sp.nstages; i++) {
-    const bool final = i + 1 == sp.nstages;
-    const int tmax = default_tile(dtype, h->solver, sp.recon[i], h->de);
-    const int per_sm = dtype == MHD_DTYPE_F64 ? 1 : (sp.recon[i] == RECON_NN) ? 3 : 2;
-    const long resident = (long)per_sm * sm_count();
-    double best = 1e300;
-    for (int t = std::min(6, tmax); t <= tmax; t++) {
-      for (int L : {0, 16, 12, 8, 6, 4}) {
-        const TileSplit s = tile_split(m, sp.S[i], final, t, t, L);
-        const long n = ntiles_of(s);
-        if (n <= 0) continue;
-        const int tx = (s.len[0] + s.np[0] - 1) / s.np[0];
-        const int ty = (s.len[1] + s.np[1] - 1) / s.np[1];
-        const int tz = (s.len[2] + s.np[2] - 1) / s.np[2];
-        const double cost = (double)((n + resident - 1) / resident) * (tx + 2) * (ty + 2) *
-                            (tz + 1.5);
-        if (cost < best * 0.999) {  // on ties the smaller tile / fewer chunks stays
-          best = cost;
-          d.tile[i] = t;
-          d.zchunk[i] = L;
-        }
-      }
-    }
-    if (h->tile > 0) d.tile[i] = h->tile;  // a tile set on the handle wins
-    if (h->zchunk > 0) d.zchunk[i] = h->zchunk;
+    const Decomp c = decompose(stage_kind(h, dtype, i),
+                               stage_window(m, sp.S[i], i + 1 == sp.nstages), 1);
+    if (c.tx <= 0) continue;
+    d.tx[i] = c.tx;
+    d.ty[i] = c.ty;
+    d.zchunk[i] = c.zchunk;
   }
   return d;
 }
@@ -636,7 +659,6 @@ template <class R> struct PlainScratch {
   void* ws;                  // their workspace (null: the fused kernels)
   StageTile* d_tiles;        // stage 0 tiles then stage 1 tiles
   int ntiles[2];
-  int tile[2];               // largest tile extent of each stage
 };
 
 size_t align_up(size_t v) { return (v + 255) & ~(size_t)255; }
@@ -649,7 +671,7 @@ int ensure_scratch(mhdvlct_handle* h, const int m[3], int dtype,
   TileSplit ts[2] = {};
   long nt[2] = {0, 0};
   for (int i = 0; i < sp.nstages; i++) {
-    ts[i] = tile_split(m, sp.S[i], i + 1 == sp.nstages, dc.tile[i], dc.tile[i], dc.zchunk[i]);
+    ts[i] = tile_split(m, sp.S[i], i + 1 == sp.nstages, dc.tx[i], dc.ty[i], dc.zchunk[i]);
     nt[i] = ntiles_of(ts[i]);
   }
   const size_t M = (size_t)m[0] * m[1] * m[2];
@@ -729,8 +751,6 @@ int ensure_scratch(mhdvlct_handle* h, const int m[3], int dtype,
   S.d_tiles = (StageTile*)(base + offs[i++]);
   S.ntiles[0] = (int)nt[0];
   S.ntiles[1] = (int)nt[1];
-  S.tile[0] = dc.tile[0];
-  S.tile[1] = dc.tile[1];
   S.d_jobs = h->split ? (SplitJob*)(base + offs[i]) : nullptr;
   S.ws = h->split ? (void*)(base + offs[i + 1]) : nullptr;
   if (!same) {
@@ -839,10 +859,7 @@ int block_step_on(mhdvlct_handle* h, const MhdBlockView* b, PlainScratch<R>& S,
     info.S = sp.S[i];
     info.final_stage = (i + 1) == sp.nstages;
     info.dt_factor = sp.dt_factor[i];
-    info.tx = S.tile[i];
-    info.ty = S.tile[i];
     info.queue = nullptr;
-    info.threads = 256;
     // EnzoMHDIntegratorStageCommands.cpp:279: the gravity source enters the
     // stage with index 1 (the full-dt stage of vl; never with euler)
     info.gravity = (i == 1 && b->acceleration[0] != nullptr) ? 1 : 0;
@@ -1101,7 +1118,7 @@ int block_step_noalloc_t(mhdvlct_handle* h, const MhdBlockView* b, double dt,
   TileSplit ts[2] = {};
   long nt[2] = {0, 0};
   for (int i = 0; i < sp.nstages; i++) {
-    ts[i] = tile_split(m, sp.S[i], i + 1 == sp.nstages, dc.tile[i], dc.tile[i], dc.zchunk[i]);
+    ts[i] = tile_split(m, sp.S[i], i + 1 == sp.nstages, dc.tx[i], dc.ty[i], dc.zchunk[i]);
     nt[i] = ntiles_of(ts[i]);
     if (nt[i] > kNoAllocMaxTiles)
       return fail(h, MHD_ERR_INVALID,
@@ -1154,8 +1171,6 @@ int block_step_noalloc_t(mhdvlct_handle* h, const MhdBlockView* b, double dt,
   S.d_tiles = (StageTile*)(base + o_tl);
   S.ntiles[0] = (int)nt[0];
   S.ntiles[1] = (int)nt[1];
-  S.tile[0] = dc.tile[0];
-  S.tile[1] = dc.tile[1];
   // every call rewrites the dt slot, the descriptors and the tile lists (the
   // array keeps whatever the previous call left)
   cudaError_t e = launch_set_scalar(S.d_dt, dt, st);

@@ -30,8 +30,6 @@ struct mhdvlct_handle {
   std::vector<vlct::SplitGroup> sp_groups[2];
   size_t sp_ws = 0;
   bool split = false;
-  int tile = 0;                // tile extent used by the plain path
-  int zchunk = 0;              // z-chunk length used by the plain path
   // mesh-refresh tables (pointer table, regions, chunks), reused across calls
   void* rf_dev = nullptr;
   size_t rf_bytes = 0;
@@ -56,9 +54,32 @@ struct StagePlan {
 };
 StagePlan stage_plan(const mhdvlct_handle* h);
 
-// Split the output window of a stage into tiles.  m: ghosted extents of the
-// block, S: stale depth after reconstruction, final: last stage.
-void make_tiles(int block, const int m[3], int S, bool final, int tile_x,
+// The kind of stage i (vlct_launch.h) on fields of a dtype.
+vlct::StageKind stage_kind(const mhdvlct_handle* h, int dtype, int i);
+
+// Extents of a stage's output window.  m: ghosted extents of the block, S:
+// stale depth after reconstruction, final: last stage.
+struct Window {
+  int lo, len[3];
+};
+Window stage_window(const int m[3], int S, bool final);
+
+// A work decomposition of a stage: tile extents and z-chunk length (0: the
+// whole window).
+struct Decomp {
+  int tx = 0, ty = 0, zchunk = 0;
+};
+// The tile of at most tx x ty columns (0: any) that the fused kernel holds and
+// that covers an lx x ly window with the least work.
+void fit_tile(const vlct::StageKind& k, int lx, int ly, int& tx, int& ty);
+// Columns that fit_tile cuts an lx x ly window into.
+long tile_columns(const vlct::StageKind& k, int lx, int ly, int tx, int ty);
+// Tile and z-chunk for `nblocks` windows alone on the GPU.
+Decomp decompose(const vlct::StageKind& k, const Window& w, long nblocks);
+
+// Split the output window of a stage into tiles of at most tile_x x tile_y
+// columns (0: any) that the fused kernel holds.
+void make_tiles(const vlct::StageKind& k, int block, const int m[3], int S, bool final, int tile_x,
                 int tile_y, int zchunk, std::vector<vlct::StageTile>& out);
 
 // The jobs of a split stage over blocks of ghosted extents m (3 per block),
@@ -73,10 +94,8 @@ void split_plan(const std::vector<int>& m, const std::vector<int>& ids, int S, b
 template <class R>
 vlct::FieldSet<R> fieldset_of(const MhdBlockView* b);
 
-// Default tile extent for a precision (fits the shared-memory budget).
-int default_tile(int dtype, int solver, int recon, int de);
-// Default tile shape of the batched form (tx x ty columns).
-void default_tile_xy(int dtype, int solver, int recon, int de, int& tx, int& ty);
+// SM count of the current device (asked for once).
+int sm_count();
 
 // The batched form (batch.cu).  batch_create is mhdvlct_batch_create_ex with,
 // when ordered_stream is not null, every device allocation, free and set-up

@@ -49,13 +49,44 @@ __device__ __forceinline__ ff ff_mul(ff x, float b) {
   const ff p = two_prod(x.hi, b);
   return fast_two_sum(p.hi, __fmaf_rn(x.lo, b, p.lo));
 }
-__device__ __forceinline__ ff ff_div(ff x, float b) {
-  const float q = __fdiv_rn(x.hi, b);
+// x / b with inv_b = 1 / b to a few ulp: the quotient of the leading part, and
+// its exact remainder (FMA) divided the same way -- 2^-45 relative, as two IEEE
+// divisions give at a quarter of the instructions
+__device__ __forceinline__ ff ff_div(ff x, float b, float inv_b) {
+  const float q = __fmul_rn(x.hi, inv_b);
   const float r = __fadd_rn(__fmaf_rn(-q, b, x.hi), x.lo);
-  return fast_two_sum(q, __fdiv_rn(r, b));
+  return fast_two_sum(q, __fmul_rn(r, inv_b));
 }
 __device__ __forceinline__ ff ff_sqsum(float a, float b, float c) {
   return ff_add(ff_add(two_prod(a, a), two_prod(b, b)), two_prod(c, c));
+}
+// Two float-float sums of three squares at once, in the lanes of packed FP32
+// arithmetic: the operations, and so the bits, of ff_sqsum in each lane, at
+// half the instructions.
+struct ff2 {
+  float2 hi, lo;
+};
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
+  return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a);
+}
+__device__ __forceinline__ ff2 two_sq2(float2 a) {
+  const float2 p = __fmul2_rn(a, a);
+  return {p, __ffma2_rn(a, a, make_float2(-p.x, -p.y))};
+}
+__device__ __forceinline__ ff2 ff_add2(ff2 x, ff2 y) {
+  const float2 s = __fadd2_rn(x.hi, y.hi);
+  const float2 bb = sub2(s, x.hi);
+  float2 e = __fadd2_rn(sub2(x.hi, sub2(s, bb)), sub2(y.hi, bb));
+  e = __fadd2_rn(__fadd2_rn(e, x.lo), y.lo);
+  const float2 t = __fadd2_rn(s, e);
+  return {t, sub2(e, sub2(t, s))};
+}
+__device__ __forceinline__ void ff_sqsum_pair(float vx, float vy, float vz, float bx, float by,
+                                              float bz, ff& v2, ff& b2) {
+  const ff2 r = ff_add2(ff_add2(two_sq2(make_float2(vx, bx)), two_sq2(make_float2(vy, by))),
+                        two_sq2(make_float2(vz, bz)));
+  v2 = {r.hi.x, r.lo.x};
+  b2 = {r.hi.y, r.lo.y};
 }
 __device__ __forceinline__ float ff_round(ff x) { return __fadd_rn(x.hi, x.lo); }
 
@@ -126,9 +157,13 @@ template <bool MHD>
 __device__ __forceinline__ float pressure_ff(float gm1, float rho, float etot,
                                              float vx, float vy, float vz, float bx,
                                              float by, float bz) {
-  const ff ke = ff_scale(ff_sqsum(vx, vy, vz), 0.5f);
-  ff d = ff_mul(ff_add({etot, 0.f}, ff_neg(ke)), rho);
-  if (MHD) d = ff_add(d, ff_neg(ff_scale(ff_sqsum(bx, by, bz), 0.5f)));
+  ff v2, b2 = {0.f, 0.f};
+  if (MHD)
+    ff_sqsum_pair(vx, vy, vz, bx, by, bz, v2, b2);
+  else
+    v2 = ff_sqsum(vx, vy, vz);
+  ff d = ff_mul(ff_add({etot, 0.f}, ff_neg(ff_scale(v2, 0.5f))), rho);
+  if (MHD) d = ff_add(d, ff_neg(ff_scale(b2, 0.5f)));
   return gm1 * ff_round(d);
 }
 template <>
@@ -188,12 +223,14 @@ __device__ __forceinline__ void energy_floor_sync(const EnergyConsts<float>& ec,
   const float inv_rho = 1.f / rho;
   const float eint_floor = ec.pfloor * ec.inv_gm1 * inv_rho;
   // non-thermal energy |v|^2/2 + |B|^2/(2 rho) in float-float
-  const ff v2 = ff_sqsum(vx, vy, vz);
+  ff v2, b2 = {0.f, 0.f};
+  if (MHD)
+    ff_sqsum_pair(vx, vy, vz, bx, by, bz, v2, b2);
+  else
+    v2 = ff_sqsum(vx, vy, vz);
   ff nte = ff_scale(v2, 0.5f);
-  ff b2 = {0.f, 0.f};
   if (MHD) {
-    b2 = ff_sqsum(bx, by, bz);
-    nte = ff_add(nte, ff_div(ff_scale(b2, 0.5f), rho));
+    nte = ff_add(nte, ff_div(ff_scale(b2, 0.5f), rho, inv_rho));
   }
   if (DE) {
     const float eint_1 = ff_round(ff_add({etot, 0.f}, ff_neg(nte)));

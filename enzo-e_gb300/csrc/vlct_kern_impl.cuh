@@ -2,6 +2,7 @@
 // kernel templates for one precision R.  Included once per precision TU.
 #pragma once
 #include <algorithm>
+#include <atomic>
 #include <type_traits>
 
 #include "vlct_aux.cuh"
@@ -13,60 +14,8 @@
 namespace vlct {
 
 namespace {
-typedef void (*StageKernelFn)(const StageBlock<VLCT_REAL>*, const StageTile*, int, StageInfo,
-                              PhysParams);
-
-// Stage kernels compiled for one launch shape (FixedShape: tile, block
-// extent, stale depths as constants), for the FP32 launches of the
-// production workloads, where the constants save about 12% of a stage:
-//   - 32^3 blocks with 3 ghost zones (extent 38), MHD (HLLD), the two-stage
-//     scheme with NN then PLM: the half-dt stage's 36 x 36 columns in tiles
-//     of 18 x 9, the full-dt stage's 34 x 34 in tiles of at most 17 x 12
-//     (both the default tiles and the autotuner's choice for this block),
-//     plain and with the gravity source / passive scalars;
-//   - 32^3 blocks with 4 ghost zones (extent 40), hydro (HLLC), the default
-//     tiles: 38 x 38 columns in tiles of at most 19 x 10, and 36 x 36 in
-//     tiles of 18 x 12, with and without flux storing.
-// Returns null unless the launch has exactly one of these shapes.
-template <int SOLVER, int RECON, bool DE, int EXTRA>
-StageKernelFn fixed_shape(const StageInfo& in) {
-  if constexpr (std::is_same<VLCT_REAL, float>::value && !DE) {
-    // the launch's (tile, every-tile-full, block extent, s, S, final) against
-    // one compiled shape
-    auto is = [&](int lx, int ly, bool full, int bm, int s, int S, bool fin) {
-      return in.tx == lx && in.ty == ly && (!full || in.full_tiles) && in.block_m == bm &&
-             in.s == s && in.S == S && (in.final_stage != 0) == fin;
-    };
-    if constexpr (SOLVER == SOLVER_HLLD && RECON == RECON_NN && EXTRA != EXTRA_FC) {
-      if (is(18, 9, true, 38, 0, 0, false))
-        return stage_kernel<float, SOLVER, RECON, DE, EXTRA,
-                            FixedShape<18, 9, true, 38, 0, 0, false>>;
-    }
-    if constexpr (SOLVER == SOLVER_HLLD && RECON == RECON_PLM && EXTRA != EXTRA_FC) {
-      if (is(17, 12, false, 38, 1, 2, true))
-        return stage_kernel<float, SOLVER, RECON, DE, EXTRA,
-                            FixedShape<17, 12, false, 38, 1, 2, true>>;
-    }
-    if constexpr (SOLVER == SOLVER_HLLC && RECON == RECON_NN && EXTRA == EXTRA_NONE) {
-      if (is(19, 10, false, 40, 0, 0, false))
-        return stage_kernel<float, SOLVER, RECON, DE, EXTRA,
-                            FixedShape<19, 10, false, 40, 0, 0, false>>;
-    }
-    if constexpr (SOLVER == SOLVER_HLLC && RECON == RECON_PLM && EXTRA != EXTRA_ALL) {
-      if (is(18, 12, true, 40, 1, 2, true))
-        return stage_kernel<float, SOLVER, RECON, DE, EXTRA,
-                            FixedShape<18, 12, true, 40, 1, 2, true>>;
-    }
-  }
-  (void)in;
-  return nullptr;
-}
-
-template <int SOLVER, int RECON, bool DE, int EXTRA>
-StageKernelFn stage_fn(const StageInfo& info) {
-  const StageKernelFn f = fixed_shape<SOLVER, RECON, DE, EXTRA>(info);
-  return f ? f : stage_kernel<VLCT_REAL, SOLVER, RECON, DE, EXTRA>;
-}
+// Device ordinals a per-device cache covers.
+constexpr int kMaxDevices = 64;
 
 // One stage as the kernels of vlct_split.cuh, group after group of jobs.
 template <class R, int SOLVER, int RECON, bool DE>
@@ -102,6 +51,37 @@ cudaError_t stage_split(const StageBlock<R>* b, const SplitLaunch& sp, const Sta
   return cudaSuccess;
 }
 
+// One stage as the fused kernel, on a persistent grid: as many CTAs as fit on
+// the GPU at once (asked for once per device: the query costs as much as a
+// launch).
+template <class R, int SOLVER, int RECON, bool DE, int EXTRA>
+cudaError_t stage_fused(const StageBlock<R>* b, const StageTile* t, int nt,
+                        const StageInfo& info, const PhysParams& phys, int grid,
+                        cudaStream_t st) {
+  auto* k = stage_kernel<R, SOLVER, RECON, DE, EXTRA>;
+  constexpr size_t smem = stage_smem_bytes<R, SOLVER, RECON, DE>();
+  constexpr int threads = StageBounds<R, SOLVER, RECON>::threads;
+  static std::atomic<int> resident[kMaxDevices];
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  int fit = dev < kMaxDevices ? resident[dev].load(std::memory_order_acquire) : 0;
+  if (fit == 0) {
+    e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    int nsm = 1, per_sm = 1;
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess)
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, smem);
+    if (e != cudaSuccess) return e;
+    fit = std::max(1, per_sm) * std::max(1, nsm);
+    if (dev < kMaxDevices) resident[dev].store(fit, std::memory_order_release);
+  }
+  if (nt <= 0) return cudaSuccess;
+  if (grid <= 0) grid = fit;
+  k<<<std::min(grid, nt), threads, smem, st>>>(b, t, nt, info, phys);
+  return cudaGetLastError();
+}
+
 template <class R, int SOLVER, int RECON, bool DE>
 cudaError_t stage_one(const StageBlock<R>* b, const StageTile* t, int nt,
                       const StageInfo& info, const PhysParams& phys, int grid,
@@ -118,37 +98,19 @@ cudaError_t stage_one(const StageBlock<R>* b, const StageTile* t, int nt,
   }
   const bool all = info.gravity != 0 || info.npass > 0;
   const bool fc = info.fc != nullptr || info.block_fc != 0;
-  const size_t smem = stage_smem_bytes<R, SOLVER, RECON, DE>(info.tx, info.ty);
   // the flux-storing-only variant exists for the hydro solver (flux
   // correction is hydro only); the others take the full variant
-  StageKernelFn k = all ? stage_fn<SOLVER, RECON, DE, EXTRA_ALL>(info)
-                        : stage_fn<SOLVER, RECON, DE, EXTRA_NONE>(info);
-  if (fc && !all) {
-    if constexpr (SOLVER == SOLVER_HLLC)
-      k = stage_fn<SOLVER, RECON, DE, EXTRA_FC>(info);
-    else
-      k = stage_fn<SOLVER, RECON, DE, EXTRA_ALL>(info);
-  }
-  cudaError_t e = cudaFuncSetAttribute(
-      k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  if (nt <= 0) return cudaSuccess;
-  const int threads =
-      (info.threads == 512 && StageBounds<R, RECON>::threads >= 512) ? 512 : 256;
-  if (grid <= 0) {
-    // persistent grid: as many CTAs as fit on the GPU at once
-    int dev = 0, nsm = 1, per_sm = 1;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, smem);
-    grid = std::max(1, per_sm) * nsm;
-  }
-  if (grid > nt) grid = nt;
-  k<<<grid, threads, smem, st>>>(b, t, nt, info, phys);
-  e = cudaGetLastError();
+  cudaError_t e;
+  if (all || (fc && SOLVER != SOLVER_HLLC))
+    e = stage_fused<R, SOLVER, RECON, DE, EXTRA_ALL>(b, t, nt, info, phys, grid, st);
+  else if (fc)
+    e = stage_fused<R, SOLVER, RECON, DE, SOLVER == SOLVER_HLLC ? EXTRA_FC : EXTRA_ALL>(
+        b, t, nt, info, phys, grid, st);
+  else
+    e = stage_fused<R, SOLVER, RECON, DE, EXTRA_NONE>(b, t, nt, info, phys, grid, st);
   // the passive scalars, on the same tiles, with the density fluxes the
   // stage kernel wrote
-  if (e == cudaSuccess && info.npass > 0) {
+  if (e == cudaSuccess && info.npass > 0 && nt > 0) {
     passive_kernel<R, RECON><<<nt, 256, 0, st>>>(b, t, info, phys);
     e = cudaGetLastError();
   }
@@ -177,14 +139,6 @@ cudaError_t stage_de(int recon, bool de, const StageBlock<R>* b,
             : stage_recon<R, SOLVER, false>(recon, b, t, nt, info, phys, grid, st, split);
 }
 
-template <class R, int SOLVER, bool DE>
-size_t smem_recon(int recon, int tx, int ty) {
-  switch (recon) {
-    case RECON_NN: return stage_smem_bytes<R, SOLVER, RECON_NN, DE>(tx, ty);
-    case RECON_PLM: return stage_smem_bytes<R, SOLVER, RECON_PLM, DE>(tx, ty);
-    default: return stage_smem_bytes<R, SOLVER, RECON_PLM_ATHENA, DE>(tx, ty);
-  }
-}
 }  // namespace
 
 template <>
@@ -200,17 +154,6 @@ cudaError_t launch_stage<VLCT_REAL>(int solver, int recon, bool de,
     case SOLVER_HLLD: return stage_de<VLCT_REAL, SOLVER_HLLD>(recon, de, b, t, nt, info, phys, grid, st, split);
   }
   return cudaErrorInvalidValue;
-}
-
-template <>
-size_t stage_smem<VLCT_REAL>(int solver, int recon, bool de, int tx, int ty) {
-  // the solver changes only NF (hydro vs MHD)
-  if (solver == SOLVER_HLLC) {
-    return de ? smem_recon<VLCT_REAL, SOLVER_HLLC, true>(recon, tx, ty)
-              : smem_recon<VLCT_REAL, SOLVER_HLLC, false>(recon, tx, ty);
-  }
-  return de ? smem_recon<VLCT_REAL, SOLVER_HLLD, true>(recon, tx, ty)
-            : smem_recon<VLCT_REAL, SOLVER_HLLD, false>(recon, tx, ty);
 }
 
 template <>

@@ -11,10 +11,32 @@ namespace vlct {
 
 template <class R> struct AuxBlock;
 
-// Largest tile extent compiled for each precision.
+// Largest tile extent that can be asked for, per precision.
 template <class R> struct TileLimits;
 template <> struct TileLimits<double> { static constexpr int TMAX = 16; };
 template <> struct TileLimits<float> { static constexpr int TMAX = 40; };
+
+// The kind of a fused stage kernel, and what a CTA of it holds of a tile of
+// tx x ty columns: its columns with their halo, one a thread, and the ring of
+// cells around them that PLM's stencil reaches.  nn: nearest-neighbour
+// reconstruction.
+//
+// Threads and CTAs per SM: FP32 MHD stages want up to 166 registers a thread
+// and run at 128 (two CTAs of 256); more, smaller-register CTAs spill (256^3
+// HLLD + PLM box, cycle: 256 x 2 6.34 ms, NN at 224 x 3 and PLM at 224 x 2 6.71,
+// both at 288 x 2 7.54).  Hydro stages are lighter: NN four CTAs of 256, PLM two
+// of 320 (960-leaf HLLC mesh with flux correction, cycle: 6.23 ms; 3 x 256 and
+// 2 x 288 6.40; 3 x 256 both 6.45; 2 x 288 and 2 x 384 6.95).
+struct StageKind {
+  bool f64, nn, mhd;
+  constexpr int threads() const { return !f64 && !mhd && !nn ? 320 : 256; }
+  // CTAs an SM holds at once
+  constexpr int ctas() const { return f64 ? 1 : (mhd || !nn ? 2 : 4); }
+  static constexpr int ring = 96;
+  bool fits(int tx, int ty) const {
+    return (tx + 2) * (ty + 2) <= threads() && 2 * (tx + ty + 4) <= ring;
+  }
+};
 
 template <class R>
 cudaError_t launch_stage(int solver, int recon, bool de,
@@ -22,9 +44,6 @@ cudaError_t launch_stage(int solver, int recon, bool de,
                          int ntiles, const StageInfo& info,
                          const PhysParams& phys, int grid, cudaStream_t st,
                          const SplitLaunch& split = SplitLaunch());
-
-template <class R>
-size_t stage_smem(int solver, int recon, bool de, int tx, int ty);
 
 template <class R>
 cudaError_t launch_timestep(bool mhd, bool de, const AuxBlock<R>* d_blocks,

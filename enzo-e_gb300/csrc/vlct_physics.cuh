@@ -357,10 +357,13 @@ __device__ __forceinline__ void hlld(R g, const R* wli, const R* wri,
 // and flux as the FP64 form, with fewer instructions.  The left and right
 // states ride in the two lanes of packed FP32 arithmetic (float2: fadd2 /
 // fmul2 / ffma2 on sm_100+), so every side-wise operation is one
-// instruction for both sides; each shared denominator is inverted once
-// (rsqrt for 1/sqrt(rho*)); the flux is F_side + c1 (U* - U) + c2 (U** - U*)
-// with the coefficients chosen in the reference's case order.  Differences
-// from the FP64 form lie only in rounding.
+// instruction for both sides, down to the flux of each side,
+//   F + c1 (U* - U) + c2 (U** - U*),
+// with the coefficients chosen in the reference's case order and the same for
+// both lanes: one select per component picks the side at the end.  Each shared
+// denominator is inverted once (rsqrt for 1/sqrt(rho*)) and multiplied by; a
+// division of its own would be eight instructions.  Differences from the FP64
+// form lie only in rounding.
 namespace packed {
 __device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
 __device__ __forceinline__ float2 s2(float a) { return make_float2(a, a); }
@@ -416,15 +419,19 @@ __device__ __forceinline__ void hlld<float>(float g, const float* wli, const flo
   const float2 sd = sub(S04, u);
   const float2 sdd = mul(sd, d);
   const float2 sddu = mul(sdd, u);
-  const float spd2 = (sddu.y - sddu.x + (pt.x - pt.y)) / (sdd.y - sdd.x);
+  const float spd2 = (sddu.y - sddu.x + (pt.x - pt.y)) * (1.0f / (sdd.y - sdd.x));
   const float2 SPD2 = s2(spd2);
   const float2 sdm = sub(S04, SPD2);
-  const float2 st_d = f2(sdd.x / sdm.x, sdd.y / sdm.y);
+  const float2 sdm_inv = f2(1.0f / sdm.x, 1.0f / sdm.y);
+  const float2 st_d = mul(sdd, sdm_inv);
   const float2 isq = f2(rsqrtf(st_d.x), rsqrtf(st_d.y));
   const float2 sqrtd = mul(st_d, isq);
   const float2 st_d_inv = mul(isq, isq);
-  const float spd1 = spd2 - fabsf(bxi) * isq.x;
-  const float spd3 = spd2 + fabsf(bxi) * isq.y;
+  // (the Alfven speeds' roundings are spelled out: near B_x^2 = rho s (s - s_M)
+  // one ulp of anything above moves a flux by 1e-4, so results that are to stay
+  // the same need every bit the same)
+  const float spd1 = __fsub_rn(spd2, __fmul_rn(fabsf(bxi), isq.x));
+  const float spd3 = __fmaf_rn(fabsf(bxi), isq.y, spd2);
   const float2 ptw = fma(sdd, sub(SPD2, u), pt);
   const float ptst = 0.5f * (ptw.y + ptw.x);
   // single-star states, both sides at once: d, mx, my, mz, e, by, bz; a
@@ -448,52 +455,58 @@ __device__ __forceinline__ void hlld<float>(float g, const float* wli, const flo
   const float2 vbst = mul(fma(Us[1], BXI, fma(Us[2], Us[5], mul(Us[3], Us[6]))), st_d_inv);
   const float2 e_num =
       add(fma(SPD2, s2(ptst), sub(mul(sd, ue), mul(pt, u))), mul(BXI, sub(fma(u, BXI, vbt), vbst)));
-  Us[4] = f2(e_num.x / sdm.x, e_num.y / sdm.y);
-  // double-star states
-  float2 Ud[7];
-#pragma unroll
-  for (int k = 0; k < 7; k++) Ud[k] = Us[k];
-  if (!(0.5f * bxsq < SMALL * ptst)) {
+  Us[4] = mul(e_num, sdm_inv);
+  // F = F_side + c1 (U* - U) + c2 (U** - U*), the cases in the reference's
+  // order: F_L (spd0 >= 0), F_R (spd4 <= 0), then by the signs of spd1..spd3;
+  // both sides at once, so that one select per component picks the side
+  const bool outer = spd0 >= 0.0f || spd4 <= 0.0f;
+  const bool left = spd0 >= 0.0f || (!(spd4 <= 0.0f) && spd2 >= 0.0f);
+  const float c1 = outer ? 0.0f : (left ? spd0 : spd4);
+  const float c2v = (outer || 0.5f * bxsq < thr)
+                        ? 0.0f
+                        : (left ? (spd1 >= 0.0f ? 0.0f : spd1) : (spd3 > 0.0f ? spd3 : 0.0f));
+  const float2 C1 = s2(c1);
+  const float2 r0 = fma(C1, sub(Us[0], d), F[0]);
+  const float2 r1 = fma(C1, sub(Us[1], du), F[1]);
+  float2 r2 = fma(C1, sub(Us[2], mul(d, vj)), F[2]);
+  float2 r3 = fma(C1, sub(Us[3], mul(d, vk)), F[3]);
+  float2 r4 = fma(C1, sub(Us[4], ue), F[4]);
+  float2 r5 = fma(C1, sub(Us[5], by), F[5]);
+  float2 r6 = fma(C1, sub(Us[6], bz), F[6]);
+  if (c2v != 0.0f) {  // the double-star states (U** = U* where B_x^2 / 2 < SMALL p*)
+    const float2 C2 = s2(c2v);
     const float invsumd = 1.0f / (sqrtd.x + sqrtd.y);
     const float bxsig = bxi > 0.0f ? 1.0f : -1.0f;
     const float2 vy = mul(Us[2], st_d_inv), vz = mul(Us[3], st_d_inv);
     const float2 wvy = mul(sqrtd, vy), wvz = mul(sqrtd, vz);
     const float ty = invsumd * (wvy.x + wvy.y + bxsig * (Us[5].y - Us[5].x));
     const float tz = invsumd * (wvz.x + wvz.y + bxsig * (Us[6].y - Us[6].x));
-    Ud[2] = mul(Us[0], s2(ty));
-    Ud[3] = mul(Us[0], s2(tz));
+    const float2 dmy = mul(Us[0], s2(ty)), dmz = mul(Us[0], s2(tz));
     const float sq = bxsig * sqrtd.x * sqrtd.y;
     const float byd = invsumd * (sqrtd.x * Us[5].y + sqrtd.y * Us[5].x + sq * (vy.y - vy.x));
     const float bzd = invsumd * (sqrtd.x * Us[6].y + sqrtd.y * Us[6].x + sq * (vz.y - vz.x));
-    Ud[5] = s2(byd);
-    Ud[6] = s2(bzd);
     // v** . B** from the left side's values for both (as the scalar form)
-    const float tl = spd2 * bxi + (Ud[2].x * byd + Ud[3].x * bzd) * st_d_inv.x;
+    const float tl = spd2 * bxi + (dmy.x * byd + dmz.x * bzd) * st_d_inv.x;
     const float2 sg = mul(sqrtd, f2(-bxsig, bxsig));
-    Ud[4] = fma(sg, sub(vbst, s2(tl)), Us[4]);
+    const float2 de = fma(sg, sub(vbst, s2(tl)), Us[4]);
+    r2 = fma(C2, sub(dmy, Us[2]), r2);
+    r3 = fma(C2, sub(dmz, Us[3]), r3);
+    r4 = fma(C2, sub(de, Us[4]), r4);
+    r5 = fma(C2, sub(s2(byd), Us[5]), r5);
+    r6 = fma(C2, sub(s2(bzd), Us[6]), r6);
   }
-  // F = F_side + c1 (U* - U) + c2 (U** - U*), the cases in the reference's
-  // order: F_L (spd0 >= 0), F_R (spd4 <= 0), then by the signs of spd1..spd3
-  const bool outer = spd0 >= 0.0f || spd4 <= 0.0f;
-  const bool left = spd0 >= 0.0f || (!(spd4 <= 0.0f) && spd2 >= 0.0f);
-  const float c1 = outer ? 0.0f : (left ? spd0 : spd4);
-  const float c2v = outer ? 0.0f : (left ? (spd1 >= 0.0f ? 0.0f : spd1)
-                                         : (spd3 > 0.0f ? spd3 : 0.0f));
-  const float2 U[7] = {d, du, mul(d, vj), mul(d, vk), ue, by, bz};
-  float Fo[7];
-#pragma unroll
-  for (int k = 0; k < 7; k++) {
-    const float Fk = left ? F[k].x : F[k].y, Uk = left ? U[k].x : U[k].y;
-    const float Usk = left ? Us[k].x : Us[k].y, Udk = left ? Ud[k].x : Ud[k].y;
-    Fo[k] = Fk + c1 * (Usk - Uk) + c2v * (Udk - Usk);
-  }
-  out.f[L_RHO] = Fo[0]; out.f[L_VI] = Fo[1]; out.f[L_VJ] = Fo[2]; out.f[L_VK] = Fo[3];
-  out.f[L_E] = Fo[4]; out.f[L_BJ] = Fo[5]; out.f[L_BK] = Fo[6];
+  out.f[L_RHO] = left ? r0.x : r0.y;
+  out.f[L_VI] = left ? r1.x : r1.y;
+  out.f[L_VJ] = left ? r2.x : r2.y;
+  out.f[L_VK] = left ? r3.x : r3.y;
+  out.f[L_E] = left ? r4.x : r4.y;
+  out.f[L_BJ] = left ? r5.x : r5.y;
+  out.f[L_BK] = left ? r6.x : r6.y;
   out.f[L_BI] = 0.0f;
   out.eflux = eint_flux(g, d.x, p.x, d.y, p.y, out.f[L_RHO]);
   if (spd0 > 0.0f) out.vbar = u.x;
   else if (spd4 < 0.0f) out.vbar = u.y;
-  else out.vbar = spd2 * (spd2 >= 0.0f ? sd.x / sdm.x : sd.y / sdm.y);
+  else out.vbar = spd2 * (spd2 >= 0.0f ? sd.x * sdm_inv.x : sd.y * sdm_inv.y);
 }
 
 // conserved state from primitives (EnzoRiemannUtils.hpp:48-82)
@@ -801,18 +814,12 @@ __device__ __forceinline__ void hllc<float>(float g, const float* wl, const floa
   const float dl = dd.x, dr = -dd.y;
   const float q1 = 1.0f / (dl + dr);
   const float cw = (t.y - t.x) * q1;
-  float cp = (dl * t.y + dr * t.x) * q1;
-  float sl, sr, sm;
-  if (cw >= 0.0f) {
-    sl = cw / (cw - bm);
-    sr = 0.0f;
-    sm = -bm / (cw - bm);
-  } else {
-    sl = 0.0f;
-    sr = -cw / (bp - cw);
-    sm = bp / (bp - cw);
-  }
-  cp = smax(cp, 0.0f);
+  const float cp = smax((dl * t.y + dr * t.x) * q1, 0.0f);
+  const bool left = cw >= 0.0f;
+  const float inv_c = 1.0f / (left ? cw - bm : bp - cw);
+  const float sc = fabsf(cw) * inv_c;
+  const float sl = left ? sc : 0.0f, sr = left ? 0.0f : sc;
+  const float sm = (left ? -bm : bp) * inv_c;
   // side fluxes relative to the outer wave speeds
   const float2 B = f2(bm, bp);
   const float2 ub = sub(u, B);

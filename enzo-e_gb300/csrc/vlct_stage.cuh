@@ -2,24 +2,39 @@
 // blocks, as a z-marching CUDA kernel.
 //
 // A CTA owns a column tile [xa, xb) x [ya, yb) of one block and marches up
-// the block's z range (or one z-chunk of it).  Everything between the global
-// state read and the stage's outputs stays in shared memory: the primitives
-// and cell-centred E of a ring of z-planes, the x/y face fluxes of two
-// planes, the z-face fluxes of two faces, the edge EMFs and the new face B.
-// Per z-plane t the CTA runs three phases separated by __syncthreads():
+// the block's z range (or one z-chunk of it).  One thread owns one column of
+// the tile and its one-cell halo, (tx + 2) x (ty + 2) of them, for the whole
+// march: it loads that column's cells, solves the Riemann problems of the
+// faces on the high side of its cell, forms the three edge EMFs there and
+// updates its cell.  So a column's positions, windows and addresses are worked
+// out once per tile and not once per item; what only the owner reads (the
+// cells below and above, the z fluxes, the x-y part of the flux divergence)
+// stays in registers; and the shared memory holds one plane of primitives (and
+// of slopes) and what neighbours exchange.  Nothing depends on the tile's or
+// the block's extents at compile time.  Per z-plane t:
 //
-//   B  Riemann solves: z-faces at t+1/2, x- and y-faces of plane t+1 (when
-//      the boundary fluxes are stored, a short pass after B copies the
-//      tile's block-boundary faces out of shared memory)
-//   C  upwinded edge EMFs: E_x, E_y at t+1/2 and E_z of plane t
-//   D  per column of the tile: its constrained-transport face updates (Bz
-//      at t+1, Bx / By at both faces of cell t), then the cell update of
-//      plane t -- centred B, flux divergence + dual-energy source, density
-//      floor, energy floor / dual-energy sync, store -- and the primitives
-//      + cell-centred E of plane t+1+L (L = 1 for NN, 2 for PLM) loaded into
-//      the ring for the next plane (in the PLM stages, and in NN stages
-//      compiled for a fixed launch shape, the raw fields are copied
-//      asynchronously right after B and converted here).
+//   B  Riemann solves: the z-face at t+1/2, the x- and y-faces of plane t+1
+//   |  barrier
+//   C  upwinded edge EMFs (E_x, E_y at t+1/2, E_z of plane t); the x-y flux
+//      divergence of plane t+1, kept for its update; the next plane's cells
+//      (on their way since the start of C, with the start-of-step values that D
+//      wants) turned into primitives and published, with the cell-centred E
+//   |  barrier
+//   D  the constrained-transport face updates around cell (x, y, t) (Bz at
+//      t+1, Bx / By at both faces of the cell), the cell update: centred B,
+//      flux divergence + dual-energy source, density floor, energy floor /
+//      dual-energy sync, store
+//   A  (PLM) the x and y slopes of the plane published in C, each formed once
+//      and read by both faces of its cell; | barrier
+//
+// What bounds it: issue slots (51-55% used; FMA, ALU and LSU pipes 24-33%, DRAM
+// 10%), with 16 warps an SM, as the Riemann solvers want 128 registers.  Against
+// the form it replaced, whose threads took each phase's items in rounds (every
+// item's place worked out anew, launch shapes of one block size compiled in):
+// HLLD + PLM warp instructions per zone 129 -> 94 (half dt), 135 -> 121 (full).
+// One cycle, before -> after: 256^3 in blocks of 32^3 6.60 -> 6.29 ms; in blocks
+// of 64^3 with dual energy 11.7 -> 5.35 ms; 1000 blocks of 16^3 - 64^3
+// 29.2 -> 12.6 ms; 960 hydro leaves with flux correction 7.45 -> 6.21 ms.
 //
 // The index windows of every quantity are those of the reference's array
 // passes (EnzoMHDIntegratorStageCommands::compute_update_stage,
@@ -43,6 +58,7 @@
 #include <type_traits>
 
 #include "vlct_energy.cuh"
+#include "vlct_launch.h"
 #include "vlct_physics.cuh"
 #include "vlct_types.h"
 
@@ -57,29 +73,16 @@ __device__ __forceinline__ bool inr(int a, int lo, int hi) {
   return a >= lo && a < hi;
 }
 
-// Asynchronous global -> shared copy of one element (cp.async, cached in
-// L1), and the calls that close a group of them and wait for the calling
-// thread's own copies.
-template <class R>
-__device__ __forceinline__ void cp_async_elem(R* smem, const R* gmem) {
-  static_assert(sizeof(R) == 4 || sizeof(R) == 8, "element size");
-  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-  if (sizeof(R) == 4)
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(sa), "l"(gmem) : "memory");
-  else
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() {
-  asm volatile("cp.async.commit_group;\n" ::: "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() {
-  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-}
-
 // Upwind weight of CT from the sign of the density flux
 // (EnzoBfieldMethodCT.cpp:198-213).
 template <class R> __device__ __forceinline__ R upw(R fd) {
   return gt0(fd) ? R(1.0) : (lt0(fd) ? R(0.0) : R(0.5));
+}
+
+// In FP32 one saturating multiply-add: the product of a normal number with
+// 3e38 is beyond +-1/2 (and a NaN, whose EMF is NaN by its other terms, gives 0).
+template <> __device__ __forceinline__ float upw<float>(float fd) {
+  return __saturatef(__fmaf_rn(fd, 3e38f, 0.5f));
 }
 
 // compute_edge_<true> (EnzoBfieldMethodCT.cpp:384-457)
@@ -96,140 +99,104 @@ __device__ __forceinline__ R edge_emf(R Ej, R Ej_kp1, R Ek, R Ek_jp1, R Wj,
   R Ek_sum = Ek + Ek_jp1;
   return R(0.25) * (Ej_sum + Ek_sum + (dEdj_l - dEdj_r) + (dEdk_l - dEdk_r));
 }
+// The same in FP32, the same value bit for bit (a weight is 0, 1/2 or 1, so its
+// products are exact), with the signs of the sums folded in.
+template <>
+__device__ __forceinline__ float edge_emf<float>(float Ej, float Ej_kp1, float Ek, float Ek_jp1,
+                                                 float Wj, float Wj_kp1, float Wk, float Wk_jp1,
+                                                 float Ec, float Ec_jp1, float Ec_kp1,
+                                                 float Ec_jkp1) {
+  auto mix = [](float w, float a, float b) {
+    return __fmaf_rn(w, a, __fmul_rn(__fsub_rn(1.0f, w), b));
+  };
+  const float dj_r = mix(Wk_jp1, Ec_jp1 + Ej, Ec_jkp1 + Ej_kp1);
+  const float dj_l = mix(Wk, Ej + Ec, Ej_kp1 + Ec_kp1);  // minus dEdj_l
+  const float dk_r = mix(Wj_kp1, Ec_kp1 - Ek, Ec_jkp1 - Ek_jp1);
+  const float dk_l = mix(Wj, Ek - Ec, Ek_jp1 - Ec_jp1);
+  return 0.25f * ((((Ek + Ek_jp1) - (Ej + Ej_kp1)) - (dj_l + dj_r)) + (dk_l - dk_r));
+}
 
 template <class R, int SOLVER, int RECON, bool DE> struct StageCfg {
   static constexpr bool MHD = SOLVER != SOLVER_HLLC;
-  static constexpr int LOOK = (RECON == RECON_NN) ? 1 : 2;
-  // ring of primitive planes: the planes a step reads plus the plane loaded
-  // ahead for the next step
-  static constexpr int NRING = (RECON == RECON_NN) ? 3 : 4;
-  static constexpr int RP = (RECON == RECON_NN) ? 0 : 1;
+  static constexpr bool NN = RECON == RECON_NN;
   static constexpr int NF = DE ? 9 : (MHD ? 7 : 5);
 };
 
-// Shared-memory carve-up for a launch whose tiles are at most tx x ty.
-struct SmemLayout {
-  int PP, QP;   // primitive tile pitch / rows
-  int HP, HQ;   // halo grid pitch / rows (tile + 1 cell each side)
-  int G;        // HP * HQ
-  int o_prim, o_xf, o_yf, o_zf, o_ec, o_ex, o_ey, o_ez, o_bz;
-  int total;    // in elements of R
-  __host__ __device__ void init(int tx, int ty, int rp, int nring, int nf) {
-    PP = tx + 2 + 2 * rp;
-    QP = ty + 2 + 2 * rp;
-    HP = tx + 2;
-    HQ = ty + 2;
-    G = HP * HQ;
-    int o = 0;
-    o_prim = o; o += nring * NQ * PP * QP;
-    o_xf = o; o += 2 * nf * G;
-    o_yf = o; o += 2 * nf * G;
-    o_zf = o; o += 2 * nf * G;
-    o_ec = o; o += nring * 3 * G;
-    o_ex = o; o += 2 * G;
-    o_ey = o; o += 2 * G;
-    o_ez = o; o += G;
-    o_bz = o; o += 2 * G;
-    total = o;
-  }
+// Threads of a CTA (and the most columns a tile takes with its halo, one a
+// thread) and the CTAs the register allocation leaves room for on an SM.
+template <class R, int SOLVER, int RECON> struct StageBounds {
+  static constexpr StageKind kind = {sizeof(R) == 8, RECON == RECON_NN, SOLVER != SOLVER_HLLC};
+  static constexpr int threads = kind.threads(), min_blocks = kind.ctas();
 };
+constexpr int kStageRing = StageKind::ring;
 
-template <class R, int SOLVER, int RECON, bool DE>
-size_t stage_smem_bytes(int tx, int ty) {
+// Shared-memory arrays, in elements: of NT each but where a size is given.
+template <class R, int SOLVER, int RECON, bool DE> struct StageSmem {
   using C = StageCfg<R, SOLVER, RECON, DE>;
-  SmemLayout L;
-  L.init(tx, ty, C::RP, C::NRING, C::NF);
-  return (size_t)L.total * sizeof(R);
-}
-
-// Launch bounds per precision and reconstruction.  FP32 PLM: 256 or 512
-// threads (the tuner's choice), registers capped at 128 so that a 512-thread
-// CTA fits an SM.  FP32 NN (the half-dt stage, smaller ring and no slopes):
-// 256 threads, registers capped at 85 so that three CTAs share an SM.
-// FP64: 256 threads with up to 255 registers (the FP64 solver does not fit
-// in 128 without spilling).
-template <class R, int RECON> struct StageBounds {
-  static constexpr int threads = 256, min_blocks = 1;
+  static constexpr int NT = StageBounds<R, SOLVER, RECON>::threads;
+  static constexpr int PQ = NT + (C::NN ? 0 : kStageRing);
+  // x / y face fluxes: density and the two transverse B of two planes, the
+  // other components of one
+  static constexpr int FD = C::MHD ? 3 : 1;            // per plane, two planes
+  static constexpr int FS = 4 + (DE ? 2 : 0);          // one plane
+  static constexpr int PL = C::NN ? 0 : 1;
+  static constexpr int MH = C::MHD ? 1 : 0;
+  static constexpr int NEC = C::NN ? 3 : 2;            // planes of E
+  static constexpr int NP = C::NN ? 2 : 1;             // planes of primitives
+  static constexpr int o_p = 0;
+  static constexpr int o_h = o_p + NP * NQ * PQ;            // PLM: x, y slopes
+  static constexpr int o_xf = o_h + PL * 2 * (NQ - 1) * NT;
+  static constexpr int o_yf = o_xf + (2 * FD + FS) * NT;
+  static constexpr int o_zf = o_yf + (2 * FD + FS) * NT;
+  static constexpr int o_ec = o_zf + MH * 3 * NT;
+  static constexpr int o_ex = o_ec + MH * 3 * NEC * NT;
+  static constexpr int o_ey = o_ex + MH * 2 * NT;
+  static constexpr int o_ez = o_ey + MH * 2 * NT;
+  // a column's own values, kept here across the Riemann solves, which want the
+  // registers: PLM's plane t+2 and low z-face state, the z fluxes at t-1/2,
+  // the x-y flux divergence of the plane to be updated
+  static constexpr int o_w2 = o_ez + MH * NT;
+  static constexpr int o_lz = o_w2 + PL * NQ * NT;
+  static constexpr int o_zm = o_lz + PL * NQ * NT;
+  static constexpr int o_dx = o_zm + (DE ? 7 : 5) * NT;
+  static constexpr int total = o_dx + (DE ? 6 : 5) * NT;
 };
-template <> struct StageBounds<float, RECON_NN> {
-  static constexpr int threads = 256, min_blocks = 3;
-};
-template <> struct StageBounds<float, RECON_PLM> {
-  static constexpr int threads = 512, min_blocks = 1;
-};
-template <> struct StageBounds<float, RECON_PLM_ATHENA> {
-  static constexpr int threads = 512, min_blocks = 1;
-};
-// largest CTA a stage of this precision and reconstruction takes
-template <class R>
-inline int stage_max_threads(int recon) {
-  return recon == RECON_NN          ? StageBounds<R, RECON_NN>::threads
-         : recon == RECON_PLM       ? StageBounds<R, RECON_PLM>::threads
-                                    : StageBounds<R, RECON_PLM_ATHENA>::threads;
+template <class R, int SOLVER, int RECON, bool DE> constexpr size_t stage_smem_bytes() {
+  return (size_t)StageSmem<R, SOLVER, RECON, DE>::total * sizeof(R);
 }
 
 enum { EXTRA_NONE = 0, EXTRA_FC = 1, EXTRA_ALL = 2 };
 
-// Launch shapes of the stage kernel.  RuntimeShape takes every value from
-// the launch.  FixedShape<LX, LY, FULL, BM, s, S, FINAL> is a launch whose
-// largest tile is LX x LY (every tile exactly that when FULL), whose blocks
-// all have extent BM (ghosts included) along each axis, and whose stage has
-// stale depths s (start) and S (after reconstruction) and is the final
-// stage when FINAL.  A fixed-shape kernel runs only launches of exactly
-// that shape; its arithmetic is the run-time kernel's.
-struct RuntimeShape {
-  static constexpr int LX = 0, LY = 0, BM = 0, s = -1, S = -1;
-  static constexpr bool FULL = false, FINAL = false;
-};
-template <int LX_, int LY_, bool FULL_, int BM_, int s_, int S_, bool FINAL_>
-struct FixedShape {
-  static_assert(LX_ > 0 && LY_ > 0 && BM_ > 0 && s_ >= 0 && S_ >= s_, "fixed shape");
-  static constexpr int LX = LX_, LY = LY_, BM = BM_, s = s_, S = S_;
-  static constexpr bool FULL = FULL_, FINAL = FINAL_;
-};
+// element at a byte offset
+template <class R> __device__ __forceinline__ R ldb(const R* p, size_t o) {
+  return *reinterpret_cast<const R*>(reinterpret_cast<const char*>(p) + o);
+}
+template <class R> __device__ __forceinline__ void stb(R* p, size_t o, R v) {
+  *reinterpret_cast<R*>(reinterpret_cast<char*>(p) + o) = v;
+}
 
 // EXTRA: EXTRA_NONE compiles the optional work out (its run-time checks alone
 // cost ~4% of a stage); EXTRA_FC can store the boundary fluxes; EXTRA_ALL
 // can also add the gravity source and write the density fluxes that
 // passive_kernel advects the passive scalars with.
-// SH: the launch's shape -- RuntimeShape (everything read from the launch's
-// StageInfo and the block descriptors) or a FixedShape, whose values are
-// compile-time constants so that the index arithmetic of shared- and
-// global-memory accesses folds.
-template <class R, int SOLVER, int RECON, bool DE, int EXTRA, class SH = RuntimeShape>
-__global__ void __launch_bounds__(StageBounds<R, RECON>::threads,
-                                  StageBounds<R, RECON>::min_blocks)
+template <class R, int SOLVER, int RECON, bool DE, int EXTRA>
+__global__ void __launch_bounds__(StageBounds<R, SOLVER, RECON>::threads,
+                                  StageBounds<R, SOLVER, RECON>::min_blocks)
 stage_kernel(const StageBlock<R>* __restrict__ blocks,
              const StageTile* __restrict__ tiles, int ntiles, StageInfo info,
              PhysParams phys) {
   using C = StageCfg<R, SOLVER, RECON, DE>;
-  constexpr bool MHD = C::MHD;
-  constexpr int LOOK = C::LOOK, NRING = C::NRING, RP = C::RP, NF = C::NF;
+  using L = StageSmem<R, SOLVER, RECON, DE>;
+  constexpr bool MHD = C::MHD, NN = C::NN;
+  constexpr int NT = L::NT, PQ = L::PQ, FD = L::FD;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  R* sm = reinterpret_cast<R*>(smem_raw);
-  SmemLayout Ls;
-  Ls.init(SH::LX > 0 ? SH::LX : info.tx, SH::LY > 0 ? SH::LY : info.ty, RP, NRING, NF);
-  // passive scalars (EXTRA_ALL only) are advected by passive_kernel after
-  // this kernel, with the density flux of every face written here
-  const int PP = Ls.PP, QP = Ls.QP, HP = Ls.HP, G = Ls.G;
-  const int PQ = PP * QP;
-  R* s_prim = sm + Ls.o_prim;
-  R* s_xf = sm + Ls.o_xf;
-  R* s_yf = sm + Ls.o_yf;
-  R* s_zf = sm + Ls.o_zf;
-  R* s_ec = sm + Ls.o_ec;
-  R* s_ex = sm + Ls.o_ex;
-  R* s_ey = sm + Ls.o_ey;
-  R* s_ez = sm + Ls.o_ez;
-  R* s_bz = sm + Ls.o_bz;
-  const int tid = threadIdx.x, nthr = blockDim.x;
-  const int s = SH::S >= 0 ? SH::s : info.s, S = SH::S >= 0 ? SH::S : info.S;
-  const bool final_stage = SH::S >= 0 ? SH::FINAL : info.final_stage != 0;
-  // the physical constants in R.  In the FP32 NN stage (registers capped for
-  // three CTAs per SM, so the compiler reloads constants from the
-  // parameters) they are the values rounded on the host, which need no FP64
-  // conversion on the device; the same values as the conversions here.
-  constexpr bool F32 = std::is_same<R, float>::value && RECON == RECON_NN;
+  R* const sm = reinterpret_cast<R*>(smem_raw);
+  const int tid = threadIdx.x;
+  const int s = info.s, S = info.S;
+  const bool final_stage = info.final_stage != 0;
+  // the physical constants in R; in FP32 the values rounded on the host, which
+  // need no FP64 conversion on the device
+  constexpr bool F32 = std::is_same<R, float>::value;
   const R g = F32 ? R(phys.gamma_f) : R(phys.gamma);
   const R theta = F32 ? R(phys.theta_limiter_f) : R(phys.theta_limiter);
   const R dfloor = F32 ? R(phys.density_floor_f) : R(phys.density_floor);
@@ -238,8 +205,7 @@ stage_kernel(const StageBlock<R>* __restrict__ blocks,
   if constexpr (F32)
     econ.init_rounded(phys, DE);
   else
-    econ.init(phys.gamma, phys.pressure_floor, DE ? phys.eta : 0.0);
-  const FastDiv divPP(Ls.PP), divHP(Ls.HP);
+    econ.init(phys, DE);
 
   __shared__ int s_next;
   // the current tile's block descriptor, copied into shared memory once per
@@ -251,8 +217,19 @@ stage_kernel(const StageBlock<R>* __restrict__ blocks,
   // would first wait for its pointer
   constexpr int kFoWords = EXTRA != EXTRA_NONE ? (int)((sizeof(FluxOut<R>) + 7) / 8) : 1;
   __shared__ __align__(16) unsigned long long s_fo_raw[kFoWords];
-  __shared__ R s_dtdx[3];
-  __shared__ R s_dt;
+  // what is the same for all threads of a tile stays in shared memory too: the
+  // solves leave no registers for it
+  struct Tile {
+    R dtdx[3], dt;
+    int m0, m1, m2, HP, HQ, za, zb, olo;
+    size_t szb, fxzb, fyzb;  // plane strides of the cell, x-face, y-face arrays
+    int rowb;                // row stride of the cell arrays
+  };
+  __shared__ Tile T;
+  const StageBlock<R>& B = *reinterpret_cast<const StageBlock<R>*>(s_blk_raw);
+  const bool store_fc =
+      EXTRA != EXTRA_NONE && final_stage && (info.fc != nullptr || info.block_fc);
+
   int it = blockIdx.x;
   if (info.queue) {
     if (tid == 0) s_next = atomicAdd(info.queue, 1);
@@ -264,547 +241,630 @@ stage_kernel(const StageBlock<R>* __restrict__ blocks,
     {
       const unsigned long long* src =
           reinterpret_cast<const unsigned long long*>(blocks + tl.block);
-      for (int w = tid; w < (int)((sizeof(StageBlock<R>) + 7) / 8); w += nthr)
+      for (int w = tid; w < (int)((sizeof(StageBlock<R>) + 7) / 8); w += NT)
         s_blk_raw[w] = src[w];
-      if (EXTRA != EXTRA_NONE && final_stage && (info.fc != nullptr || info.block_fc)) {
+      if (store_fc) {
         const void* fsrc = blocks[tl.block].fc != nullptr ? blocks[tl.block].fc : info.fc;
         const unsigned long long* fw = reinterpret_cast<const unsigned long long*>(fsrc);
-        for (int w = tid; w < kFoWords; w += nthr) s_fo_raw[w] = fw[w];
+        for (int w = tid; w < kFoWords; w += NT) s_fo_raw[w] = fw[w];
       }
     }
-    const StageBlock<R>& B = *reinterpret_cast<const StageBlock<R>*>(s_blk_raw);
-    const StageBlock<R>& Bg = blocks[tl.block];
-    const int m0 = SH::BM > 0 ? SH::BM : Bg.m[0];
-    const int m1 = SH::BM > 0 ? SH::BM : Bg.m[1];
-    const int m2 = SH::BM > 0 ? SH::BM : Bg.m[2];
-    const int xa = tl.xa, xb = tl.xb, ya = tl.ya, yb = tl.yb;
-    const int tx = SH::FULL ? SH::LX : xb - xa, ty = SH::FULL ? SH::LY : yb - ya;
     // dt / dx per axis, once per tile (FP64 divisions: one thread)
     if (tid == 0) {
+      const StageBlock<R>& Bg = blocks[tl.block];
       const double dt = *Bg.dt * info.dt_factor;
-      s_dtdx[0] = R(dt / Bg.cw[0]);
-      s_dtdx[1] = R(dt / Bg.cw[1]);
-      s_dtdx[2] = R(dt / Bg.cw[2]);
-      s_dt = R(dt);
+      for (int a = 0; a < 3; a++) T.dtdx[a] = R(dt / Bg.cw[a]);
+      T.dt = R(dt);
+      T.m0 = Bg.m[0];
+      T.m1 = Bg.m[1];
+      T.m2 = Bg.m[2];
+      T.HP = tl.xb - tl.xa + 2;
+      T.HQ = tl.yb - tl.ya + 2;
+      T.za = tl.za;
+      T.zb = tl.zb;
+      T.olo = final_stage ? S : S + 1;
+      T.rowb = T.m0 * (int)sizeof(R);
+      T.szb = (size_t)T.rowb * T.m1;
+      T.fxzb = (size_t)(T.m0 + 1) * sizeof(R) * T.m1;
+      T.fyzb = (size_t)T.rowb * (T.m1 + 1);
     }
     __syncthreads();  // also publishes the descriptor copy
-    const R dtdx[3] = {s_dtdx[0], s_dtdx[1], s_dtdx[2]};
-    // output window of centred B (and the z-march range)
-    const int olo = final_stage ? S : S + 1;
-    const int ohi_x = final_stage ? m0 - S : m0 - S - 1;
-    const int ohi_y = final_stage ? m1 - S : m1 - S - 1;
-    const int za = tl.za, zb = tl.zb;  // output planes of this chunk
-    const int t0 = za - 1;
-    // prim-tile origin and halo-grid origin
-    const int px0 = xa - 1 - RP, py0 = ya - 1 - RP;
-    const int hx0 = xa - 1, hy0 = ya - 1;
-    const size_t cstr_y = (size_t)m0, cstr_z = (size_t)m0 * m1;
 
-    // offset of cell (x, y) of ring slot `slot` in s_prim (add q * PQ)
-    auto poff = [&](int slot, int x, int y) -> int {
-      return slot * NQ * PQ + (y - py0) * PP + (x - px0);
+    // ---- the thread's column and what it takes part in
+    enum {
+      CELL = 1, FX = 2, FY = 4, FZ = 8, EX = 16, EY = 32, EZ = 64, OUT = 128, UX = 256, UY = 512,
+      UPD = 1024, RING = 2048, COL = 4096, XHI = 1 << 13, YHI = 1 << 14,
+      // face B updated on the low / high side along x, y
+      XLO = 1 << 15, XUP = 1 << 16, YLO = 1 << 17, YUP = 1 << 18,
+      // first / last column and row of the halo grid
+      ILO = 1 << 19, IHI = 1 << 20, JLO = 1 << 21, JHI = 1 << 22
     };
-
-    // ---- primitives (and the cell-centred E) of plane p into its ring slot,
-    // in two steps.  With ASYNC_LOADS (the PLM stages) issue_plane starts
-    // asynchronous copies of the raw cell fields into the slot (the energy
-    // field into the pressure plane) and finish_plane, after the copies have
-    // landed, turns them into primitives in place.  Every thread finishes
-    // exactly the cells it issued, so the two need no barrier between them;
-    // in the z-march the copies of plane t+1+L go out right after phase B of
-    // plane t (the slot they overwrite, plane t-1's, is no longer read) and
-    // land while phases C and D run.  The NN stage with the run-time shape,
-    // already close to its issue limit, loads in finish_plane directly: the
-    // extra shared-memory pass costs it more than the latency it would hide.
-    // With a fixed shape it issues fewer instructions, and the asynchronous
-    // copies pay there too.
-    constexpr bool ASYNC_LOADS = RECON != RECON_NN || SH::BM > 0;
-    auto issue_plane = [&](int p) {
-      if (!ASYNC_LOADS || !inr(p, s, m2 - s)) return;
-      const int slot = p % NRING;
-      const int fe = DE ? F_EINT : F_ETOT;
-      for (int idx = tid; idx < PQ; idx += nthr) {
-        const int qy = divPP.div(idx);
-        const int x = px0 + (idx - qy * PP), y = py0 + qy;
-        if (!inr(x, s, m0 - s) || !inr(y, s, m1 - s)) continue;
-        const size_t c = (size_t)p * cstr_z + (size_t)y * cstr_y + x;
-        R* w = s_prim + poff(slot, x, y);
-        cp_async_elem(w + Q_RHO * PQ, B.cur.c[F_RHO] + c);
-        cp_async_elem(w + (Q_VX + 0) * PQ, B.cur.c[F_VX] + c);
-        cp_async_elem(w + (Q_VX + 1) * PQ, B.cur.c[F_VY] + c);
-        cp_async_elem(w + (Q_VX + 2) * PQ, B.cur.c[F_VZ] + c);
-        if (MHD) {
-          cp_async_elem(w + (Q_BX + 0) * PQ, B.cur.c[F_BX] + c);
-          cp_async_elem(w + (Q_BX + 1) * PQ, B.cur.c[F_BY] + c);
-          cp_async_elem(w + (Q_BX + 2) * PQ, B.cur.c[F_BZ] + c);
-        }
-        cp_async_elem(w + Q_P * PQ, B.cur.c[fe] + c);
+    unsigned fl = 0;
+    auto on = [&](unsigned f) { return (fl & f) == f; };
+    auto flag = [&](unsigned f, bool v) { fl |= v ? f : 0u; };
+    int cb, xb_, rcell = 0;  // byte offsets in a plane: cell and y-face arrays,
+                             // x-face arrays, ring
+    {
+      const int m0 = T.m0, m1 = T.m1, HP = T.HP, HQ = T.HQ;
+      const int tx = HP - 2, ty = HQ - 2;
+      const int j = tid / HP, i = tid - j * HP;
+      const int x = tl.xa - 1 + i, y = tl.ya - 1 + j;
+      const bool col = j < HQ;
+      const bool iny = inr(y, S, m1 - S), inx = inr(x, S, m0 - S);
+      const bool ux = inr(x, S + 1, m0 - S - 1), uy = inr(y, S + 1, m1 - S - 1);
+      const bool hx = inr(x, S, m0 - S - 1), hy = inr(y, S, m1 - S - 1);
+      const bool out = col && i >= 1 && i <= tx && j >= 1 && j <= ty;
+      flag(COL, col);
+      flag(CELL, col && inr(x, s, m0 - s) && inr(y, s, m1 - s));
+      flag(FX, col && i <= tx && hx && iny);
+      flag(FY, col && j <= ty && hy && inx);
+      flag(FZ, col && inx && iny);
+      flag(EX, col && i >= 1 && i <= tx && j <= ty && ux && hy);
+      flag(EY, col && i <= tx && j >= 1 && j <= ty && uy && hx);
+      flag(EZ, col && i <= tx && j <= ty && hx && hy);
+      flag(OUT, out);
+      flag(UX, ux);
+      flag(UY, uy);
+      flag(UPD, out && ux && uy);
+      flag(XLO, inr(x, S + 1, m0 - S));
+      flag(XUP, inr(x + 1, S + 1, m0 - S));
+      flag(YLO, inr(y, S + 1, m1 - S));
+      flag(YUP, inr(y + 1, S + 1, m1 - S));
+      flag(XHI, x + 1 == m0 - T.olo);
+      flag(YHI, y + 1 == m1 - T.olo);
+      cb = y * T.rowb + x * (int)sizeof(R);
+      xb_ = cb + y * (int)sizeof(R);
+      flag(ILO, i == 0);
+      flag(IHI, i == HP - 1);
+      flag(JLO, j == 0);
+      flag(JHI, j == HQ - 1);
+      // PLM: the plane of primitives has a second ring of cells around the
+      // halo grid, kept behind it: HP below, HP above, HQ left, HQ right; ring
+      // cell k is loaded by thread k
+      if (!NN && tid < 2 * (HP + HQ)) {
+        const int k = tid < 2 * HP ? tid : tid - 2 * HP;
+        const int ri = tid < 2 * HP ? (k < HP ? k : k - HP) : (k < HQ ? -1 : HP);
+        const int rj = tid < 2 * HP ? (k < HP ? -1 : HQ) : (k < HQ ? k : k - HQ);
+        const int rx = tl.xa - 1 + ri, ry = tl.ya - 1 + rj;
+        flag(RING, inr(rx, s, m0 - s) && inr(ry, s, m1 - s));
+        rcell = ry * T.rowb + rx * (int)sizeof(R);
       }
-      cp_async_commit();
+    }
+    const int t0 = tl.za - 1;
+    const int zb = tl.zb;
+
+    R* const s_p0 = sm + L::o_p + tid;
+    auto plane_p = [&](int p) { return s_p0 + (NN ? (p & 1) * NQ * PQ : 0); };
+    R* const s_w2 = sm + L::o_w2 + tid;
+    R* const s_h = sm + L::o_h + tid;
+    R* const s_lz = sm + L::o_lz + tid;
+    R* const s_zm = sm + L::o_zm + tid;
+    R* const s_dx = sm + L::o_dx + tid;
+    R* const s_xf = sm + L::o_xf + tid;
+    R* const s_yf = sm + L::o_yf + tid;
+    R* const s_zf = sm + L::o_zf + tid;
+    R* const s_ec = sm + L::o_ec + tid;
+    R* const s_ex = sm + L::o_ex + tid;
+    R* const s_ey = sm + L::o_ey + tid;
+    R* const s_ez = sm + L::o_ez + tid;
+    // flux components in shared memory: plane-buffered ones and single ones
+    auto fd = [&](int plane, int k) { return ((plane & 1) * FD + k) * NT; };
+    auto fs = [&](int k) { return (2 * FD + k) * NT; };
+
+    // ---- the cell at a byte offset: density, B, v and the energy field, in
+    // primitive order; then the energy turned into the pressure
+    // (EnzoComputePressure::compute_pressure, EnzoComputePressure.cpp:127-190)
+    auto load = [&](size_t at, R* w) {
+#pragma unroll
+      for (int q = 0; q < NQ; q++)
+        w[q] = q == Q_RHO ? ldb(B.cur.c[F_RHO], at)
+             : q >= Q_VX && q < Q_P ? ldb(B.cur.c[F_VX + (q - Q_VX)], at)
+             : q == Q_P ? ldb(B.cur.c[DE ? F_EINT : F_ETOT], at)
+             : MHD ? ldb(B.cur.c[F_BX + (q - Q_BX)], at) : R(0);
     };
-    auto finish_plane = [&](int p) {
-      if (!inr(p, s, m2 - s)) return;
-      if (ASYNC_LOADS) cp_async_wait_all();
-      const int slot = p % NRING;
-      const int fe = DE ? F_EINT : F_ETOT;
-      for (int idx = tid; idx < PQ; idx += nthr) {
-        const int qy = divPP.div(idx);
-        const int x = px0 + (idx - qy * PP), y = py0 + qy;
-        if (!inr(x, s, m0 - s) || !inr(y, s, m1 - s)) continue;
-        R* w = s_prim + poff(slot, x, y);
-        const size_t c = (size_t)p * cstr_z + (size_t)y * cstr_y + x;
-        // the fields: from the slot (copied there) or from global memory
-        auto field = [&](int q, int f) -> R { return ASYNC_LOADS ? w[q * PQ] : B.cur.c[f][c]; };
-        const R rho = field(Q_RHO, F_RHO);
-        const R vx = field(Q_VX + 0, F_VX), vy = field(Q_VX + 1, F_VY), vz = field(Q_VX + 2, F_VZ);
-        R bx = R(0), by = R(0), bz = R(0);
-        if (MHD) {
-          bx = field(Q_BX + 0, F_BX);
-          by = field(Q_BX + 1, F_BY);
-          bz = field(Q_BX + 2, F_BZ);
-        }
-        // EnzoComputePressure::compute_pressure (EnzoComputePressure.cpp:127-190)
-        const R e_in = field(Q_P, fe);
-        if (!ASYNC_LOADS) {
-          w[Q_RHO * PQ] = rho;
-          w[(Q_VX + 0) * PQ] = vx;
-          w[(Q_VX + 1) * PQ] = vy;
-          w[(Q_VX + 2) * PQ] = vz;
-          if (MHD) {
-            w[(Q_BX + 0) * PQ] = bx;
-            w[(Q_BX + 1) * PQ] = by;
-            w[(Q_BX + 2) * PQ] = bz;
-          }
-        }
-        R p_out;
-        if (DE) {
-          p_out = econ.gm1 * rho * e_in;
-        } else {
-          p_out = pressure_from_etot<R, MHD>(econ, rho, e_in, vx, vy, vz, bx, by, bz);
-        }
-        w[Q_P * PQ] = p_out;
-        // cell-centred E = -v x B (EnzoBfieldMethodCT.cpp:267-292), on the
-        // halo grid and inside [S, m - S)
-        const int hi = x - hx0, hj = y - hy0;
-        if (MHD && hi >= 0 && hi < HP && hj >= 0 && hj < Ls.HQ &&
-            inr(x, S, m0 - S) && inr(y, S, m1 - S) && inr(p, S, m2 - S)) {
-          R* e = s_ec + slot * 3 * G + hj * HP + hi;
-          e[0] = (-vy * bz + vz * by);
-          e[G] = (-vz * bx + vx * bz);
-          e[2 * G] = (-vx * by + vy * bx);
+    auto prims = [&](R* w) {
+      w[Q_P] = DE ? econ.gm1 * w[Q_RHO] * w[Q_P]
+                  : pressure_from_etot<R, MHD>(econ, w[Q_RHO], w[Q_P], w[Q_VX], w[Q_VX + 1],
+                                               w[Q_VX + 2], w[Q_BX], w[Q_BX + 1], w[Q_BX + 2]);
+    };
+    auto put = [&](R* dst, int pitch, const R* w) {
+#pragma unroll
+      for (int q = 0; q < NQ; q++)
+        if (MHD || q < Q_BX || q >= Q_VX) dst[q * pitch] = w[q];
+    };
+    // cell-centred E = -v x B of plane p (EnzoBfieldMethodCT.cpp:267-292)
+    auto put_ec = [&](int p, const R* w) {
+      if (MHD && on(FZ) && inr(p, S, T.m2 - S)) {
+        R* e = s_ec + (p % L::NEC) * 3 * NT;
+        const R bx = w[Q_BX], by = w[Q_BX + 1], bz = w[Q_BX + 2];
+        const R vx = w[Q_VX], vy = w[Q_VX + 1], vz = w[Q_VX + 2];
+        e[0] = (-vy * bz + vz * by);
+        e[NT] = (-vz * bx + vx * bz);
+        e[2 * NT] = (-vx * by + vy * bx);
+      }
+    };
+    // PLM: half the slopes of the published plane along x (not of Bx) and y
+    // (not of By), in the slots that hslot says
+    auto hslot = [](int dir, int q) { return dir * (NQ - 1) + (q > Q_BX + dir ? q - 1 : q); };
+    auto slopes = [&]() {
+      const R* const s_p = s_p0;
+      if (on(COL)) {
+        const int HP = T.HP, HQ = T.HQ;
+        const int j = tid / HP, i = tid - j * HP;
+        const int lft = on(ILO) ? NT + 2 * HP + j - tid : -1;
+        const int rgt = on(IHI) ? NT + 2 * HP + HQ + j - tid : 1;
+        const int dwn = on(JLO) ? NT + i - tid : -HP;
+        const int upp = on(JHI) ? NT + HP + i - tid : HP;
+#pragma unroll
+        for (int q = 0; q < NQ; q++) {
+          if (!MHD && q >= Q_BX && q < Q_VX) continue;
+          const R* w = s_p + q * PQ;
+          const R c = w[0];
+          if (q != Q_BX)
+            s_h[hslot(0, q) * NT] = half_slope<R, RECON>(w[lft], c, w[rgt], theta);
+          if (q != Q_BX + 1)
+            s_h[hslot(1, q) * NT] = half_slope<R, RECON>(w[dwn], c, w[upp], theta);
         }
       }
     };
 
-    // ---- Riemann solves: z-faces at t+1/2 (if zfaces) and the x- and
-    // y-faces of plane pl.  One code path for all three directions.
-    auto phase_b = [&](int t, bool zfaces, int pl) {
-      const int HQv = Ls.HQ;
-      const FastDiv divX(tx + 1);
-      const int nz = zfaces ? HP * HQv : 0;
-      const int nx = (tx + 1) * HQv;
-      const int ny = HP * (ty + 1);
-      const bool plane_ok = inr(pl, S, m2 - S);
-      for (int idx = tid; idx < nz + nx + ny; idx += nthr) {
-        int d, i, j;
-        if (idx < nz) {
-          d = 2; j = divHP.div(idx); i = idx - j * HP;
-        } else if (idx < nz + nx) {
-          const int q = idx - nz;
-          d = 0; j = divX.div(q); i = q - j * (tx + 1);
-        } else {
-          const int q = idx - nz - nx;
-          d = 1; j = divHP.div(q); i = q - j * HP;
+    // ---- column state.  NN: the primitives of planes t and t+1 stay in shared
+    // memory.  PLM, at iteration t: w1 the primitives of plane t+1, hz half
+    // their z slope; in shared memory the state on the low side of the z-face
+    // t+1/2 (s_lz) and plane t+2's primitives (s_w2)
+    R w1[NQ], hz[NQ];
+    R zp[7];  // z fluxes at t+1/2: rho, mom, E, eint, vbar
+    R bz_lo = R(0);
+    R p_t = R(0), p_n = R(0);  // floored pressure of plane t, t+1 (dual energy)
+#pragma unroll
+    for (int q = 0; q < NQ; q++) w1[q] = hz[q] = R(0);
+#pragma unroll
+    for (int k = 0; k < 7; k++) zp[k] = R(0);
+
+    // ---- prologue: plane t0 published (PLM: and t0 - 1, t0 + 1 held)
+    {
+      R wa[NQ], wc[NQ];
+#pragma unroll
+      for (int q = 0; q < NQ; q++) wa[q] = wc[q] = R(0);
+      auto have = [&](int p) { return inr(p, s, T.m2 - s); };
+      auto fetch = [&](int p, R* w) {
+        if (on(CELL) && have(p)) {
+          load((size_t)p * T.szb + cb, w);
+          prims(w);
         }
-        const int x = hx0 + i, y = hy0 + j;
-        // face index f along d: the face between cells f and f+1
-        int off[4];  // s_prim offsets of the cells f-1 .. f+2 along d
-        const R* bface;
-        R* dst;
-        const int r = j * HP + i;
-        if (d == 2) {
-          const int fz = t;
-          if (!inr(fz, S, m2 - 1 - S) || !inr(x, S, m0 - S) || !inr(y, S, m1 - S))
-            continue;
+      };
+      fetch(t0, w1);
+      if (on(CELL) && have(t0)) {
+        put(plane_p(t0), PQ, w1);
+        put_ec(t0, w1);
+      }
+      if constexpr (!NN) {
+        fetch(t0 - 1, wa);
+        fetch(t0 + 1, wc);
+        if (on(CELL) && have(t0 + 1)) put(s_w2, NT, wc);
 #pragma unroll
-          for (int k = 0; k < 4; k++) off[k] = poff((fz - 1 + k + NRING) % NRING, x, y);
-          bface = B.cur.f[2] + ((size_t)(fz + 1) * cstr_z + (size_t)y * cstr_y + x);
-          dst = s_zf + (size_t)(fz & 1) * NF * G + r;
-        } else {
-          if (!plane_ok) continue;
-          const int slot = pl % NRING;
-          if (d == 0) {
-            if (!inr(x, S, m0 - 1 - S) || !inr(y, S, m1 - S)) continue;
-#pragma unroll
-            for (int k = 0; k < 4; k++) off[k] = poff(slot, x - 1 + k, y);
-            bface = B.cur.f[0] + ((size_t)pl * ((size_t)m1 * (m0 + 1)) +
-                                  (size_t)y * (m0 + 1) + (x + 1));
-            dst = s_xf + (size_t)(pl & 1) * NF * G + r;
-          } else {
-            if (!inr(y, S, m1 - 1 - S) || !inr(x, S, m0 - S)) continue;
-#pragma unroll
-            for (int k = 0; k < 4; k++) off[k] = poff(slot, x, y - 1 + k);
-            bface = B.cur.f[1] + ((size_t)pl * ((size_t)(m1 + 1) * m0) +
-                                  (size_t)(y + 1) * m0 + x);
-            dst = s_yf + (size_t)(pl & 1) * NF * G + r;
-          }
+        for (int q = 0; q < NQ; q++) hz[q] = half_slope<R, RECON>(wa[q], w1[q], wc[q], theta);
+        if (on(RING) && have(t0)) {
+          load((size_t)t0 * T.szb + rcell, wa);
+          prims(wa);
+          put(s_p0 + NT, PQ, wa);
         }
-        // reconstruction (EnzoReconstructorNN.cpp:14-49,
-        // EnzoReconstructorPLM.hpp:167-345), in the face frame
+        __syncthreads();
+        slopes();
+      }
+      __syncthreads();
+    }
+
+    // face B along x, y (plane t+1) and z (face t+1), loaded ahead of their use
+    R bfx = R(0), bfy = R(0), bfz = R(0);
+    auto load_bface = [&](int t) {
+      if (!MHD) return;
+      const int pl = t + 1;
+      if (inr(pl, S, T.m2 - S)) {
+        if (on(FX)) bfx = ldb(B.cur.f[0], (size_t)pl * T.fxzb + (xb_ + (int)sizeof(R)));
+        if (on(FY)) bfy = ldb(B.cur.f[1], (size_t)pl * T.fyzb + (cb + T.rowb));
+      }
+      if (on(FZ) && inr(t, S, T.m2 - 1 - S)) bfz = ldb(B.cur.f[2], (size_t)pl * T.szb + cb);
+    };
+    load_bface(t0 - 1);
+
+    for (int t = t0 - 1; t < zb; t++) {
+      const bool first = t < t0;  // only the x- and y-faces of plane t0
+      const int pl = t + 1;
+      // the cells of the plane after next (NN: the next one)
+      const int nxt = NN ? t + 2 : t + 3;
+      const bool more = t + 1 < zb;
+      // ---- B: Riemann solves
+      // (EnzoReconstructorNN.cpp:14-49, EnzoReconstructorPLM.hpp:167-345);
+      // the longitudinal B is the face's own (EnzoBfieldMethodCT.cpp:122-166)
+      FaceFlux<R> F;
+      auto solve = [&](auto dir, R bf, auto left, auto right) {
+        constexpr int d = decltype(dir)::value, d1 = (d + 1) % 3, d2 = (d + 2) % 3;
         R wl[8], wr[8];
-        const int d1 = (d + 1) % 3, d2 = (d + 2) % 3;
+        constexpr int q_of[8] = {Q_RHO, Q_BX + d, Q_BX + d1, Q_BX + d2,
+                                 Q_VX + d, Q_VX + d1, Q_VX + d2, Q_P};
 #pragma unroll
         for (int k = 0; k < 8; k++) {
-          if (!MHD && (k == L_BI || k == L_BJ || k == L_BK)) {
+          if (k == L_BI) {
+            wl[k] = wr[k] = MHD ? bf : R(0);
+          } else if (!MHD && (k == L_BJ || k == L_BK)) {
             wl[k] = wr[k] = R(0);
-            continue;
-          }
-          const int q = (k == L_RHO) ? Q_RHO
-                      : (k == L_BI) ? Q_BX + d : (k == L_BJ) ? Q_BX + d1
-                      : (k == L_BK) ? Q_BX + d2 : (k == L_VI) ? Q_VX + d
-                      : (k == L_VJ) ? Q_VX + d1 : (k == L_VK) ? Q_VX + d2 : Q_P;
-          const R* w = s_prim + q * PQ;
-          if (RECON == RECON_NN) {
-            wl[k] = w[off[1]];
-            wr[k] = w[off[2]];
           } else {
-            const R a = w[off[0]], b0 = w[off[1]], b1 = w[off[2]], c = w[off[3]];
-            R dl, dr;
-            if (RECON == RECON_PLM) {
-              dl = limiter_enzo_rk(a, b0, b1, theta);
-              dr = limiter_enzo_rk(b0, b1, c, theta);
-            } else {
-              dl = limiter_athena(a, b0, b1);
-              dr = limiter_athena(b0, b1, c);
-            }
-            R lv = b0 + dl * R(0.5), rv = b1 - dr * R(0.5);
-            if (k == L_RHO) {
-              lv = smax(lv, dfloor);
-              rv = smax(rv, dfloor);
-            } else if (k == L_E) {
-              lv = smax(lv, pfloor);
-              rv = smax(rv, pfloor);
-            }
-            wl[k] = lv;
-            wr[k] = rv;
+            wl[k] = left(q_of[k]);
+            wr[k] = right(q_of[k]);
           }
         }
-        if (MHD) {  // correct_reconstructed_bfield (EnzoBfieldMethodCT.cpp:122-166)
-          const R bf = *bface;
-          wl[L_BI] = bf;
-          wr[L_BI] = bf;
+        if (!NN) {
+          wl[L_RHO] = smax(wl[L_RHO], dfloor);
+          wr[L_RHO] = smax(wr[L_RHO], dfloor);
+          wl[L_E] = smax(wl[L_E], pfloor);
+          wr[L_E] = smax(wr[L_E], pfloor);
         }
-        FaceFlux<R> F;
         riemann<SOLVER, R>(g, wl, wr, F);
-        dst[S_RHO * G] = F.f[L_RHO];
-        dst[(S_MX + d) * G] = F.f[L_VI];
-        dst[(S_MX + d1) * G] = F.f[L_VJ];
-        dst[(S_MX + d2) * G] = F.f[L_VK];
-        dst[S_E * G] = F.f[L_E];
-        if (MHD) {
-          dst[S_BJ * G] = F.f[L_BJ];
-          dst[S_BK * G] = F.f[L_BK];
-        }
-        if (DE) {
-          dst[S_EINT * G] = F.eflux;
-          dst[S_VBAR * G] = F.vbar;
-        }
-      }
-    };
-
-    // ---- store_fluxes_for_corrections (EnzoMethodMHDVlct.cpp:250-330): on
-    // the final stage, dt/dx times the fluxes through the block's active
-    // boundary faces, read back from the face fluxes phase B left in shared
-    // memory (valid until phase B overwrites that plane parity two steps
-    // later).  Every face is written by exactly one tile: the tile (and
-    // z-chunk) that owns the cells on its high side.
-    // (the outputs are looked up inside the pass: nothing extra stays live
-    // across the z-march)
-    const bool store_fc =
-        EXTRA != EXTRA_NONE && final_stage && (info.fc != nullptr || info.block_fc);
-    auto store_fluxes = [&](int t, bool zfaces, int pl) {
-      const FluxOut<R>* fo = reinterpret_cast<const FluxOut<R>*>(s_fo_raw);
-      const int gg = info.fc_g;
-      // f: the face's fluxes (the passive scalars' are stored by
-      // passive_kernel)
-      auto put = [&](int d, int side, size_t at, const R* f) {
-        const R sc = dtdx[d];
+      };
+      // boundary fluxes for flux correction (EnzoMethodMHDVlct.cpp:250-330):
+      // on the final stage, dt/dx times the flux through the block's active
+      // boundary faces, each by the tile (and z-chunk) that owns the cell on
+      // its high side
+      auto store_face = [&](int d, int side, size_t at) {
+        const FluxOut<R>* fo = reinterpret_cast<const FluxOut<R>*>(s_fo_raw);
+        const R sc = T.dtdx[d];
+        const R v[6] = {F.f[L_RHO], F.f[L_VI + (3 - d) % 3], F.f[L_VI + (4 - d) % 3],
+                        F.f[L_VI + (5 - d) % 3], F.f[L_E], DE ? F.eflux : R(0)};
 #pragma unroll
         for (int q = 0; q < 6; q++) {
           R* p = fo->f[d][side][q];
-          if (!p) continue;
-          const R v = q == 0 ? f[S_RHO * G]
-                    : q <= 3 ? f[(S_MX + q - 1) * G]
-                    : q == 4 ? f[S_E * G] : (DE ? f[S_EINT * G] : R(0));
-          p[at] = sc * v;
+          if (p) p[at] = sc * v[q];
         }
       };
-      const int xlo = xa > gg ? xa : gg, xhi = xb < m0 - gg ? xb : m0 - gg;
-      const int ylo = ya > gg ? ya : gg, yhi = yb < m1 - gg ? yb : m1 - gg;
-      if (pl >= za && pl < zb && inr(pl, gg, m2 - gg)) {
-        const R* xf = s_xf + (size_t)(pl & 1) * NF * G;
-        const R* yf = s_yf + (size_t)(pl & 1) * NF * G;
-        for (int side = 0; side < 2; side++) {
-          const int x = side == 0 ? gg - 1 : m0 - gg - 1;  // x faces
-          if (x >= xa - 1 && x < xb - 1)
-            for (int y = ylo + tid; y < yhi; y += nthr) {
-              const int r = (y - hy0) * HP + (x - hx0);
-              put(0, side, (size_t)(pl - gg) * (m1 - 2 * gg) + (y - gg), xf + r);
-            }
-          const int y = side == 0 ? gg - 1 : m1 - gg - 1;  // y faces
-          if (y >= ya - 1 && y < yb - 1)
-            for (int x2 = xlo + tid; x2 < xhi; x2 += nthr) {
-              const int r = (y - hy0) * HP + (x2 - hx0);
-              put(1, side, (size_t)(pl - gg) * (m0 - 2 * gg) + (x2 - gg), yf + r);
-            }
+      const int gg = info.fc_g;
+      // the column's (and its tile's) place again, only where fluxes are stored
+      auto place = [&](int& x, int& y, int& i, int& j) {
+        j = tid / T.HP;
+        i = tid - j * T.HP;
+        x = tl.xa - 1 + i;
+        y = tl.ya - 1 + j;
+      };
+      // x- and y-faces of plane t+1
+      auto put_face = [&](R* f, int d) {
+        f[fd(pl, 0)] = F.f[L_RHO];
+        if (MHD) {
+          f[fd(pl, 1)] = F.f[L_BJ];
+          f[fd(pl, 2)] = F.f[L_BK];
+        }
+        f[fs(0)] = F.f[L_VI + (3 - d) % 3];
+        f[fs(1)] = F.f[L_VI + (4 - d) % 3];
+        f[fs(2)] = F.f[L_VI + (5 - d) % 3];
+        f[fs(3)] = F.f[L_E];
+        if (DE) {
+          f[fs(4)] = F.eflux;
+          f[fs(5)] = F.vbar;
+        }
+      };
+      const bool plane_ok = inr(pl, S, T.m2 - S);
+      const R* const s_p = plane_p(pl);
+      if (plane_ok && on(FX)) {
+        const R* w = s_p + 1;
+        solve(std::integral_constant<int, 0>{}, bfx,
+              [&](int q) { return NN ? s_p[q * PQ] : w1[q] + s_h[hslot(0, q) * NT]; },
+              [&](int q) { return NN ? w[q * PQ] : w[q * PQ] - s_h[hslot(0, q) * NT + 1]; });
+        put_face(s_xf, 0);
+        if (EXTRA != EXTRA_NONE && store_fc) {
+          int x, y, i, j;
+          place(x, y, i, j);
+          const int side = x == gg - 1 ? 0 : (x == T.m0 - gg - 1 ? 1 : -1);
+          if (side >= 0 && i < T.HP - 2 && j >= 1 && j <= tl.yb - tl.ya && inr(y, gg, T.m1 - gg) &&
+              pl >= T.za && pl < zb && inr(pl, gg, T.m2 - gg))
+            store_face(0, side, (size_t)(pl - gg) * (T.m1 - 2 * gg) + (y - gg));
         }
       }
-      const int side = t == gg - 1 ? 0 : (t == m2 - gg - 1 ? 1 : -1);  // z faces at t+1/2
-      if (zfaces && side >= 0 && t >= za - 1 && t < zb - 1) {
-        const R* zf = s_zf + (size_t)(t & 1) * NF * G;
-        const int w = xhi - xlo;
-        for (int k = tid; k < w * (yhi - ylo); k += nthr) {
-          const int y = ylo + k / w, x = xlo + k % w;
-          const int r = (y - hy0) * HP + (x - hx0);
-          put(2, side, (size_t)(y - gg) * (m0 - 2 * gg) + (x - gg), zf + r);
+      if (plane_ok && on(FY)) {
+        const R* w = s_p + T.HP;
+        const R* h = s_h + T.HP;
+        solve(std::integral_constant<int, 1>{}, bfy,
+              [&](int q) { return NN ? s_p[q * PQ] : w1[q] + s_h[hslot(1, q) * NT]; },
+              [&](int q) { return NN ? w[q * PQ] : w[q * PQ] - h[hslot(1, q) * NT]; });
+        put_face(s_yf, 1);
+        if (EXTRA != EXTRA_NONE && store_fc) {
+          int x, y, i, j;
+          place(x, y, i, j);
+          const int side = y == gg - 1 ? 0 : (y == T.m1 - gg - 1 ? 1 : -1);
+          if (side >= 0 && j < tl.yb - tl.ya && i >= 1 && i <= T.HP - 2 && inr(x, gg, T.m0 - gg) &&
+              pl >= T.za && pl < zb && inr(pl, gg, T.m2 - gg))
+            store_face(1, side, (size_t)(pl - gg) * (T.m0 - 2 * gg) + (x - gg));
         }
       }
-    };
-
-    // ---------------------------------------------------------- prologue --
-    for (int p = t0 - (LOOK - 1); p <= t0 + LOOK; p++) issue_plane(p);
-    for (int p = t0 - (LOOK - 1); p <= t0 + LOOK; p++) finish_plane(p);
-    __syncthreads();
-    phase_b(t0 - 1, false, t0);
-    __syncthreads();
-    if (store_fc) store_fluxes(t0 - 1, false, t0);
-
-    for (int t = t0; t < zb; t++) {
-      // ---- B: z-faces at t+1/2, x/y faces of plane t+1
-      phase_b(t, true, t + 1);
-      __syncthreads();
-      // plane t+1+L's fields start towards the ring slot phase B just
-      // released (plane t-1's)
-      if (t + 1 < zb) issue_plane(t + 1 + LOOK);
-      if (store_fc) store_fluxes(t, true, t + 1);
-      // ---- C: edge EMFs (EnzoBfieldMethodCT.cpp:480-590)
-      if (MHD) {
-        const R* xf0 = s_xf + (size_t)(t & 1) * NF * G;
-        const R* xf1 = s_xf + (size_t)((t + 1) & 1) * NF * G;
-        const R* yf0 = s_yf + (size_t)(t & 1) * NF * G;
-        const R* yf1 = s_yf + (size_t)((t + 1) & 1) * NF * G;
-        const R* zf = s_zf + (size_t)(t & 1) * NF * G;
-        const R* ec0 = s_ec + (size_t)(t % NRING) * 3 * G;
-        const R* ec1 = s_ec + (size_t)((t + 1) % NRING) * 3 * G;
-        for (int idx = tid; idx < 3 * G; idx += nthr) {
-          const int kind = idx < G ? 0 : (idx < 2 * G ? 1 : 2), r = idx - kind * G;
-          const int j = divHP.div(r), i = r - j * HP;
-          const int x = hx0 + i, y = hy0 + j;
-          if (kind == 0) {  // E_x at (x, y+1/2, t+1/2)
-            if (i < 1 || i > tx || j > ty) continue;
-            if (!inr(x, S + 1, m0 - S - 1) || !inr(y, S, m1 - S - 1) ||
-                !inr(t, S, m2 - S - 1))
-              continue;
-            s_ex[(t & 1) * G + r] = edge_emf<R>(
-                yf0[S_BJ * G + r], yf1[S_BJ * G + r], zf[S_BK * G + r],
-                zf[S_BK * G + r + HP], upw(yf0[r]), upw(yf1[r]), upw(zf[r]),
-                upw(zf[r + HP]), ec0[r], ec0[r + HP], ec1[r], ec1[r + HP]);
-          } else if (kind == 1) {  // E_y at (x+1/2, y, t+1/2)
-            if (i > tx || j < 1 || j > ty) continue;
-            if (!inr(x, S, m0 - S - 1) || !inr(y, S + 1, m1 - S - 1) ||
-                !inr(t, S, m2 - S - 1))
-              continue;
-            s_ey[(t & 1) * G + r] = edge_emf<R>(
-                zf[S_BJ * G + r], zf[S_BJ * G + r + 1], xf0[S_BK * G + r],
-                xf1[S_BK * G + r], upw(zf[r]), upw(zf[r + 1]), upw(xf0[r]),
-                upw(xf1[r]), ec0[G + r], ec1[G + r], ec0[G + r + 1],
-                ec1[G + r + 1]);
-          } else {  // E_z at (x+1/2, y+1/2, t)
-            if (i > tx || j > ty) continue;
-            if (!inr(x, S, m0 - S - 1) || !inr(y, S, m1 - S - 1) ||
-                !inr(t, S + 1, m2 - S - 1))
-              continue;
-            s_ez[r] = edge_emf<R>(
-                xf0[S_BJ * G + r], xf0[S_BJ * G + r + HP], yf0[S_BK * G + r],
-                yf0[S_BK * G + r + 1], upw(xf0[r]), upw(xf0[r + HP]),
-                upw(yf0[r]), upw(yf0[r + 1]), ec0[2 * G + r],
-                ec0[2 * G + r + 1], ec0[2 * G + r + HP], ec0[2 * G + r + HP + 1]);
+      // z-face at t+1/2
+      if (!first && on(FZ) && inr(t, S, T.m2 - 1 - S)) {
+        solve(std::integral_constant<int, 2>{}, bfz,
+              [&](int q) { return NN ? plane_p(t)[q * PQ] : s_lz[q * NT]; },
+              [&](int q) { return NN ? s_p[q * PQ] : w1[q] - hz[q]; });
+        zp[0] = F.f[L_RHO];
+        zp[1] = F.f[L_VJ];
+        zp[2] = F.f[L_VK];
+        zp[3] = F.f[L_VI];
+        zp[4] = F.f[L_E];
+        if (DE) {
+          zp[5] = F.eflux;
+          zp[6] = F.vbar;
+        }
+        if (MHD) {
+          s_zf[0] = F.f[L_RHO];
+          s_zf[NT] = F.f[L_BJ];
+          s_zf[2 * NT] = F.f[L_BK];
+        }
+        if (EXTRA != EXTRA_NONE && store_fc && on(OUT)) {
+          const int side = t == gg - 1 ? 0 : (t == T.m2 - gg - 1 ? 1 : -1);
+          if (side >= 0 && t >= T.za - 1 && t < zb - 1) {
+            int x, y, i, j;
+            place(x, y, i, j);
+            if (inr(x, gg, T.m0 - gg) && inr(y, gg, T.m1 - gg))
+              store_face(2, side, (size_t)(y - gg) * (T.m0 - 2 * gg) + (x - gg));
           }
         }
-        __syncthreads();
       }
-      // ---- D: per column (x, y) of the tile, the constrained-transport
-      // face updates it needs (EnzoBfieldMethodCT.cpp:617-687) -- Bz at the
-      // face t+1 above it and, when plane t is output, Bx at faces x, x+1 and
-      // By at faces y, y+1 of plane t -- then the update of cell (x, y, t).
-      // A face between two cells of the tile is computed by both (the same
-      // expression) and written by the one that owns it: the cell on its high
-      // side, or the cell below the block's outermost written face.  A face
-      // not updated in this stage keeps its start-of-step value.  Bz at t+1
-      // stays in shared memory for the same column's next plane, so the
-      // mapping of columns to threads is the same for every plane.  The
-      // primitives of plane t+1+LOOK are finished into the ring in the same
-      // phase.
-      {
-        const bool do_plane = t >= za;
-        // the lowest face of a chunk is written by the chunk below it
-        const bool own_bz = t >= za || za == olo;
-        const bool in_t = inr(t, S + 1, m2 - S - 1);
-        // Bx at face kx of row y, plane t; rx: the halo index of face kx
-        auto face_x = [&](int kx, int y, int rx, bool own) -> R {
-          const size_t fi = (size_t)t * ((size_t)m1 * (m0 + 1)) + (size_t)y * (m0 + 1) + kx;
-          if (!(inr(kx, S + 1, m0 - S) && inr(y, S + 1, m1 - S - 1) && in_t))
-            return B.base.f[0][fi];
-          // E_z at (kx-1/2, y -+ 1/2), E_y at (kx-1/2, t -+ 1/2)
-          const int re = rx - 1;  // edge ex = kx - 1
-          const R Ek_term = dtdx[1] * (s_ez[re] - s_ez[re - HP]);
-          const R Ej_term = dtdx[2] * (s_ey[(t & 1) * G + re] - s_ey[((t - 1) & 1) * G + re]);
-          const R v = B.base.f[0][fi] - Ek_term + Ej_term;
-          if (own) B.out.f[0][fi] = v;
-          return v;
-        };
-        // By at face ky of column x, plane t; ry: the halo index of face ky
-        auto face_y = [&](int ky, int x, int ry, bool own) -> R {
-          const size_t fi = (size_t)t * ((size_t)(m1 + 1) * m0) + (size_t)ky * m0 + x;
-          if (!(inr(ky, S + 1, m1 - S) && inr(x, S + 1, m0 - S - 1) && in_t))
-            return B.base.f[1][fi];
-          // E_x at (x, ky-1/2, t -+ 1/2), E_z at (x -+ 1/2, ky-1/2)
-          const int re = ry - HP;  // edge ey = ky - 1
-          const R Ek_term = dtdx[2] * (s_ex[(t & 1) * G + re] - s_ex[((t - 1) & 1) * G + re]);
-          const R Ej_term = dtdx[0] * (s_ez[re] - s_ez[re - 1]);
-          const R v = B.base.f[1][fi] - Ek_term + Ej_term;
-          if (own) B.out.f[1][fi] = v;
-          return v;
-        };
-        const R* xf0 = s_xf + (size_t)(t & 1) * NF * G;
-        const R* yf0 = s_yf + (size_t)(t & 1) * NF * G;
-        const R* zfm = s_zf + (size_t)((t - 1) & 1) * NF * G;
-        const R* zfp = s_zf + (size_t)(t & 1) * NF * G;
-        const int slot = t % NRING;
-        const FastDiv divT(tx);
-        for (int idx = tid; idx < tx * ty; idx += nthr) {
-          const int qy = divT.div(idx);
-          const int x = xa + (idx - qy * tx), y = ya + qy;
-          const int r = (y - hy0) * HP + (x - hx0);
-          R bcx = R(0), bcy = R(0), bcz = R(0);
+      if constexpr (!NN) {
+#pragma unroll
+        for (int q = 0; q < NQ; q++)
+          if (MHD || q < Q_BX || q >= Q_VX) s_lz[q * NT] = w1[q] + hz[q];
+      }
+      __syncthreads();
+
+      // ---- C.  First the loads: the next cells, and plane t's start-of-step
+      // values for its update in D; their latency passes under the rest of C
+      const int HP = T.HP;
+      R in[NQ], rin[NQ];
+      const bool in_on = more && on(CELL) && inr(nxt, s, T.m2 - s);
+      const bool rin_on = !NN && more && on(RING) && inr(t + 2, s, T.m2 - s);
+      if (in_on) load((size_t)nxt * T.szb + cb, in);
+      if constexpr (!NN) {
+        if (rin_on) load((size_t)(t + 2) * T.szb + rcell, rin);
+      }
+      R base[6], bf[5];  // rho, v, etot, eint; face B: x, x+1, y, y+1, z+1
+      if (!first && on(OUT)) {
+        const size_t c = (size_t)t * T.szb + cb;
+        if (MHD) bf[4] = ldb(B.base.f[2], c + T.szb);
+        if (t >= T.za) {  // (plane za - 1 may lie below the block)
           if (MHD) {
-            // Bz at face kz = t+1 of column (x, y)
-            const int kz = t + 1;
-            R bz_hi = R(0);
-            if (kz <= m2) {
-              const size_t fi = (size_t)kz * cstr_z + (size_t)y * cstr_y + x;
-              const bool upd = inr(kz, S + 1, m2 - S) && inr(x, S + 1, m0 - S - 1) &&
-                               inr(y, S + 1, m1 - S - 1);
-              if (upd) {
-                const R Ek_term = dtdx[0] * (s_ey[(t & 1) * G + r] - s_ey[(t & 1) * G + r - 1]);
-                const R Ej_term = dtdx[1] * (s_ex[(t & 1) * G + r] - s_ex[(t & 1) * G + r - HP]);
-                bz_hi = B.base.f[2][fi] - Ek_term + Ej_term;
-                if (own_bz) B.out.f[2][fi] = bz_hi;
-              } else {
-                bz_hi = B.base.f[2][fi];
+            const size_t xo = (size_t)t * T.fxzb + xb_, yo = (size_t)t * T.fyzb + cb;
+            bf[0] = ldb(B.base.f[0], xo);
+            bf[1] = ldb(B.base.f[0], xo + sizeof(R));
+            bf[2] = ldb(B.base.f[1], yo);
+            bf[3] = ldb(B.base.f[1], yo + T.rowb);
+          }
+#pragma unroll
+          for (int k = 0; k < 5; k++) base[k] = ldb(B.base.c[F_RHO + k], c);
+          if (DE) base[5] = ldb(B.base.c[F_EINT], c);
+        }
+      }
+      // edge EMFs (EnzoBfieldMethodCT.cpp:480-590)
+      if (MHD && !first) {
+        const R *xf0 = s_xf + fd(t, 0), *xf1 = s_xf + fd(pl, 0);
+        const R *yf0 = s_yf + fd(t, 0), *yf1 = s_yf + fd(pl, 0);
+        const R *bj = s_zf + NT, *bk = s_zf + 2 * NT;
+        const R* ec0 = s_ec + (t % L::NEC) * 3 * NT;
+        const R* ec1 = s_ec + (pl % L::NEC) * 3 * NT;
+        const bool zt = inr(t, S, T.m2 - S - 1);
+        const R Wx0 = upw(xf0[0]), Wx1 = upw(xf1[0]), Wy0 = upw(yf0[0]), Wy1 = upw(yf1[0]),
+                Wz = upw(s_zf[0]);
+        if (on(EX) && zt)  // E_x at (x, y+1/2, t+1/2)
+          s_ex[(t & 1) * NT] = edge_emf<R>(yf0[NT], yf1[NT], bk[0], bk[HP], Wy0, Wy1, Wz,
+                                           upw(s_zf[HP]), ec0[0], ec0[HP], ec1[0], ec1[HP]);
+        if (on(EY) && zt)  // E_y at (x+1/2, y, t+1/2)
+          s_ey[(t & 1) * NT] =
+              edge_emf<R>(bj[0], bj[1], xf0[2 * NT], xf1[2 * NT], Wz, upw(s_zf[1]), Wx0, Wx1,
+                          ec0[NT], ec1[NT], ec0[NT + 1], ec1[NT + 1]);
+        if (on(EZ) && inr(t, S + 1, T.m2 - S - 1))  // E_z at (x+1/2, y+1/2, t)
+          s_ez[0] = edge_emf<R>(xf0[NT], xf0[NT + HP], yf0[2 * NT], yf0[2 * NT + 1], Wx0,
+                                upw(xf0[HP]), Wy0, upw(yf0[1]), ec0[2 * NT], ec0[2 * NT + 1],
+                                ec0[2 * NT + HP], ec0[2 * NT + HP + 1]);
+      }
+      // flux divergence of plane t+1 along x, then y
+      // (EnzoIntegrationQuanUpdate.cpp:105-147, EnzoSourceInternalEnergy.cpp:16-92);
+      // plane t's moves to registers, for its update
+      R dxy[6];
+      if (on(UPD) && plane_ok) {
+#pragma unroll
+        for (int k = 0; k < (DE ? 6 : 5); k++) dxy[k] = s_dx[k * NT];
+        const R dtdx0 = T.dtdx[0], dtdx1 = T.dtdx[1];
+        const R *xr = s_xf + fd(pl, 0), *yr = s_yf + fd(pl, 0);
+        R a = R(0.0);
+        a -= dtdx0 * (xr[0] - xr[-1]);
+        a -= dtdx1 * (yr[0] - *(yr - HP));
+        s_dx[0] = a;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          const R *xk = s_xf + fs(k), *yk = s_yf + fs(k);
+          a = R(0.0);
+          a -= dtdx0 * (xk[0] - xk[-1]);
+          a -= dtdx1 * (yk[0] - *(yk - HP));
+          s_dx[(1 + k) * NT] = a;
+        }
+        if (DE) {
+          p_n = smax(NN ? s_p[Q_P * PQ] : w1[Q_P], pfloor);
+          const R *xe = s_xf + fs(4), *xv = s_xf + fs(5), *ye = s_yf + fs(4), *yv = s_yf + fs(5);
+          a = R(0.0);
+          a -= dtdx0 * (xe[0] - xe[-1]);
+          a -= dtdx0 * p_n * (xv[0] - xv[-1]);
+          a -= dtdx1 * (ye[0] - *(ye - HP));
+          a -= dtdx1 * p_n * (yv[0] - *(yv - HP));
+          s_dx[5 * NT] = a;
+        }
+        // the passive scalars' advection (passive_kernel) needs the density
+        // flux of both faces of every updated cell along each axis: the low
+        // faces, and the high ones at the region's edges
+        if (EXTRA == EXTRA_ALL && info.npass > 0 && pl >= T.za && pl < zb &&
+            inr(pl, S + 1, T.m2 - S - 1)) {
+          const size_t c = (size_t)pl * T.szb + cb;
+          stb(B.dflux[0], c, xr[-1]);
+          stb(B.dflux[1], c, *(yr - HP));
+          int x, y, i, j;
+          place(x, y, i, j);
+          if (x + 1 == T.m0 - S - 1) stb(B.dflux[0], c + sizeof(R), xr[0]);
+          if (y + 1 == T.m1 - S - 1) stb(B.dflux[1], c + T.rowb, yr[0]);
+        }
+      }
+      // the next plane's primitives and cell-centred E; plane t+1 is no
+      // longer read
+      if (more) {
+        if constexpr (NN) {
+          if (in_on) {
+            prims(in);
+            put(plane_p(nxt), PQ, in);
+            put_ec(nxt, in);
+          }
+        } else {
+          R w2[NQ];
+#pragma unroll
+          for (int q = 0; q < NQ; q++)
+            w2[q] = (!MHD && q >= Q_BX && q < Q_VX) ? R(0) : s_w2[q * NT];
+          if (on(CELL) && inr(t + 2, s, T.m2 - s)) put(s_p0, PQ, w2);
+          if (in_on) {
+            prims(in);
+            put(s_w2, NT, in);
+#pragma unroll
+            for (int q = 0; q < NQ; q++)
+              hz[q] = half_slope<R, RECON>(w1[q], w2[q], in[q], theta);
+          }
+#pragma unroll
+          for (int q = 0; q < NQ; q++) w1[q] = w2[q];
+          if (rin_on) {
+            prims(rin);
+            put(s_p0 + NT, PQ, rin);
+          }
+        }
+        load_bface(t + 1);
+      }
+      __syncthreads();
+
+      // ---- D: the constrained-transport face updates around cell (x, y, t)
+      // (EnzoBfieldMethodCT.cpp:617-687) -- Bz at the face t+1 above it and,
+      // when plane t is output, Bx at faces x, x+1 and By at faces y, y+1 --
+      // then the cell's update.  A face between two cells of the tile is
+      // computed by both (the same expression) and written by the one that
+      // owns it: the cell on its high side, or the cell below the block's
+      // outermost written face.  A face not updated in this stage keeps its
+      // start-of-step value.
+      if (on(OUT) && !first) {
+        const bool do_plane = t >= T.za;
+        const bool in_t = inr(t, S + 1, T.m2 - S - 1);
+        const size_t c = (size_t)t * T.szb + cb;
+        const R dtdx0 = T.dtdx[0], dtdx1 = T.dtdx[1], dtdx2 = T.dtdx[2];
+        R bcx = R(0), bcy = R(0), bcz = R(0);
+        if (MHD) {
+          const R *ex = s_ex + (t & 1) * NT, *exm = s_ex + ((t - 1) & 1) * NT;
+          const R *ey = s_ey + (t & 1) * NT, *eym = s_ey + ((t - 1) & 1) * NT;
+          // Bz at face t+1
+          R bz_hi = bf[4];
+          if (on(UPD) && inr(t + 1, S + 1, T.m2 - S)) {
+            const R Ek_term = dtdx0 * (ey[0] - ey[-1]);
+            const R Ej_term = dtdx1 * (ex[0] - *(ex - HP));
+            bz_hi = bz_hi - Ek_term + Ej_term;
+            // the lowest face of a chunk is written by the chunk below it
+            if (do_plane || T.za == T.olo) stb(B.out.f[2], c + T.szb, bz_hi);
+          }
+          if (do_plane) {
+            const size_t xo = (size_t)t * T.fxzb + xb_, yo = (size_t)t * T.fyzb + cb;
+            // Bx at faces x, x+1: E_z at (kx-1/2, y -+ 1/2), E_y at (kx-1/2, t -+ 1/2)
+            R b[2];
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+              b[k] = bf[k];
+              if (on(k == 0 ? XLO : XUP) && on(UY) && in_t) {
+                const R Ek_term = dtdx1 * (s_ez[k - 1] - *(s_ez + (k - 1) - HP));
+                const R Ej_term = dtdx2 * (ey[k - 1] - eym[k - 1]);
+                b[k] = b[k] - Ek_term + Ej_term;
+                if (k == 0 || on(XHI)) stb(B.out.f[0], xo + k * sizeof(R), b[k]);
               }
             }
-            const R bz_lo = s_bz[(t & 1) * G + r];  // face t, from the previous plane
-            s_bz[((t + 1) & 1) * G + r] = bz_hi;
-            if (do_plane) {
-              // compute_center_bfield (EnzoBfieldMethodCT.cpp:702-728)
-              const R bx_lo = face_x(x, y, r, true);
-              const R bx_hi = face_x(x + 1, y, r + 1, x + 1 == xb && xb == ohi_x);
-              const R by_lo = face_y(y, x, r, true);
-              const R by_hi = face_y(y + 1, x, r + HP, y + 1 == yb && yb == ohi_y);
-              bcx = R(0.5) * (bx_lo + bx_hi);
-              bcy = R(0.5) * (by_lo + by_hi);
-              bcz = R(0.5) * (bz_lo + bz_hi);
+            bcx = R(0.5) * (b[0] + b[1]);
+            // By at faces y, y+1: E_x at (x, ky-1/2, t -+ 1/2), E_z at (x -+ 1/2, ky-1/2)
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+              const size_t o = yo + k * T.rowb;
+              b[k] = bf[2 + k];
+              if (on(k == 0 ? YLO : YUP) && on(UX) && in_t) {
+                const int e = (k - 1) * HP;
+                const R Ek_term = dtdx2 * (ex[e] - exm[e]);
+                const R Ej_term = dtdx0 * (s_ez[e] - s_ez[e - 1]);
+                b[k] = b[k] - Ek_term + Ej_term;
+                if (k == 0 || on(YHI)) stb(B.out.f[1], o, b[k]);
+              }
             }
+            bcy = R(0.5) * (b[0] + b[1]);
+            // compute_center_bfield (EnzoBfieldMethodCT.cpp:702-728)
+            bcz = R(0.5) * (bz_lo + bz_hi);
+            stb(B.out.c[F_BX], c, bcx);
+            stb(B.out.c[F_BY], c, bcy);
+            stb(B.out.c[F_BZ], c, bcz);
           }
-          if (!do_plane) continue;
-          const size_t c = (size_t)t * cstr_z + (size_t)y * cstr_y + x;
-          if (MHD) {
-            B.out.c[F_BX][c] = bcx;
-            B.out.c[F_BY][c] = bcy;
-            B.out.c[F_BZ][c] = bcz;
-          }
-          if (!inr(x, S + 1, m0 - S - 1) || !inr(y, S + 1, m1 - S - 1) ||
-              !inr(t, S + 1, m2 - S - 1))
-            continue;
-          // flux divergence, x then y then z
-          // (EnzoIntegrationQuanUpdate.cpp:105-147, EnzoSourceInternalEnergy.cpp:16-92)
+          bz_lo = bz_hi;
+        }
+        if (do_plane && on(UPD) && in_t) {
           R du[6];
 #pragma unroll
-          for (int k = 0; k < 5; k++) {
-            R a = R(0.0);
-            a -= dtdx[0] * (xf0[k * G + r] - xf0[k * G + r - 1]);
-            a -= dtdx[1] * (yf0[k * G + r] - yf0[k * G + r - HP]);
-            a -= dtdx[2] * (zfp[k * G + r] - zfm[k * G + r]);
-            du[k] = a;
-          }
+          for (int k = 0; k < 5; k++) du[k] = dxy[k] - dtdx2 * (zp[k] - s_zm[k * NT]);
           if (DE) {
-            const R p = smax(s_prim[poff(slot, x, y) + Q_P * PQ], pfloor);
-            R a = R(0.0);
-            a -= dtdx[0] * (xf0[S_EINT * G + r] - xf0[S_EINT * G + r - 1]);
-            a -= dtdx[0] * p * (xf0[S_VBAR * G + r] - xf0[S_VBAR * G + r - 1]);
-            a -= dtdx[1] * (yf0[S_EINT * G + r] - yf0[S_EINT * G + r - HP]);
-            a -= dtdx[1] * p * (yf0[S_VBAR * G + r] - yf0[S_VBAR * G + r - HP]);
-            a -= dtdx[2] * (zfp[S_EINT * G + r] - zfm[S_EINT * G + r]);
-            a -= dtdx[2] * p * (zfp[S_VBAR * G + r] - zfm[S_VBAR * G + r]);
+            R a = dxy[5];
+            a -= dtdx2 * (zp[5] - s_zm[5 * NT]);
+            a -= dtdx2 * p_t * (zp[6] - s_zm[6 * NT]);
             du[5] = a;
           }
+          const R old_rho = base[0], ovx = base[1], ovy = base[2], ovz = base[3], oet = base[4];
+          R eint = DE ? base[5] : R(0);
           // gravity source on the full-dt stage (EnzoSourceGravity.cpp:17-69,
           // EnzoMHDIntegratorStageCommands.cpp:267-297): start-of-step
           // density and velocity
           if (EXTRA == EXTRA_ALL && info.gravity) {
-            const R dt = s_dt;
-            const R rho0 = B.base.c[F_RHO][c];
-            const R ax = B.accel[0][c], ay = B.accel[1][c], az = B.accel[2][c];
-            du[1] += dt * rho0 * ax;
-            du[2] += dt * rho0 * ay;
-            du[3] += dt * rho0 * az;
-            du[4] += dt * rho0 * ((B.base.c[F_VX][c] * ax) + (B.base.c[F_VY][c] * ay) +
-                                  (B.base.c[F_VZ][c] * az));
+            const R dt = T.dt;
+            const R ax = ldb(B.accel[0], c), ay = ldb(B.accel[1], c), az = ldb(B.accel[2], c);
+            du[1] += dt * old_rho * ax;
+            du[2] += dt * old_rho * ay;
+            du[3] += dt * old_rho * az;
+            du[4] += dt * old_rho * ((ovx * ax) + (ovy * ay) + (ovz * az));
           }
           // update_quantities (EnzoIntegrationQuanUpdate.cpp:183-231)
-          const R old_rho = B.base.c[F_RHO][c];
           R new_rho = old_rho + du[0];
           new_rho = smax(new_rho, dfloor);
           const R inv_new_rho = R(1.) / new_rho;
-          R vx = (B.base.c[F_VX][c] * old_rho + du[1]) * inv_new_rho;
-          R vy = (B.base.c[F_VY][c] * old_rho + du[2]) * inv_new_rho;
-          R vz = (B.base.c[F_VZ][c] * old_rho + du[3]) * inv_new_rho;
-          R etot = (B.base.c[F_ETOT][c] * old_rho + du[4]) * inv_new_rho;
-          R eint = R(0);
-          if (DE) eint = (B.base.c[F_EINT][c] * old_rho + du[5]) * inv_new_rho;
+          const R vx = (ovx * old_rho + du[1]) * inv_new_rho;
+          const R vy = (ovy * old_rho + du[2]) * inv_new_rho;
+          const R vz = (ovz * old_rho + du[3]) * inv_new_rho;
+          R etot = (oet * old_rho + du[4]) * inv_new_rho;
+          if (DE) eint = (eint * old_rho + du[5]) * inv_new_rho;
           // apply_floor_to_energy_and_sync (EnzoPhysicsFluidProps.cpp:162-290)
-          energy_floor_sync<MHD, DE>(econ, new_rho, vx, vy, vz, bcx, bcy, bcz, etot,
-                                     eint);
-          B.out.c[F_RHO][c] = new_rho;
-          B.out.c[F_VX][c] = vx;
-          B.out.c[F_VY][c] = vy;
-          B.out.c[F_VZ][c] = vz;
-          B.out.c[F_ETOT][c] = etot;
-          if (DE) B.out.c[F_EINT][c] = eint;
-          // the passive scalars' advection (passive_kernel) needs the
-          // density flux of both faces of every updated cell along each
-          // axis: the low faces here, the high faces at the region's edges
+          energy_floor_sync<MHD, DE>(econ, new_rho, vx, vy, vz, bcx, bcy, bcz, etot, eint);
+          stb(B.out.c[F_RHO], c, new_rho);
+          stb(B.out.c[F_VX], c, vx);
+          stb(B.out.c[F_VY], c, vy);
+          stb(B.out.c[F_VZ], c, vz);
+          stb(B.out.c[F_ETOT], c, etot);
+          if (DE) stb(B.out.c[F_EINT], c, eint);
           if (EXTRA == EXTRA_ALL && info.npass > 0) {
-            R* const* D = B.dflux;
-            D[0][c] = xf0[S_RHO * G + r - 1];
-            D[1][c] = yf0[S_RHO * G + r - HP];
-            D[2][c] = zfm[S_RHO * G + r];
-            if (x + 1 == m0 - S - 1) D[0][c + 1] = xf0[S_RHO * G + r];
-            if (y + 1 == m1 - S - 1) D[1][c + cstr_y] = yf0[S_RHO * G + r];
-            if (t + 1 == m2 - S - 1) D[2][c + cstr_z] = zfp[S_RHO * G + r];
+            stb(B.dflux[2], c, s_zm[0]);
+            if (t + 1 == T.m2 - S - 1) stb(B.dflux[2], c + T.szb, zp[0]);
           }
         }
+#pragma unroll
+        for (int k = 0; k < (DE ? 7 : 5); k++) s_zm[k * NT] = zp[k];
       }
-      if (t + 1 < zb) finish_plane(t + 1 + LOOK);
-      __syncthreads();
+      p_t = p_n;
+      // ---- A: the slopes of plane t+2, for the next plane's faces, and its
+      // cell-centred E (in the buffer of plane t, no longer read)
+      if constexpr (!NN) {
+        if (more) {
+          put_ec(t + 2, w1);
+          slopes();
+          __syncthreads();
+        }
+      }
     }
     // next tile: dynamic queue (persistent grid) or static grid stride
+    __syncthreads();
     if (info.queue) {
       if (tid == 0) s_next = atomicAdd(info.queue, 1);
       __syncthreads();
       it = s_next;
-      __syncthreads();
     } else {
       it += gridDim.x;
     }

@@ -111,21 +111,14 @@ struct StageInfo {
   int S;            // stale depth after reconstruction (s + immediate rate)
   int final_stage;  // 1 on the last stage (writes layer S of centred B)
   double dt_factor; // 0.5 for the half step, 1 for the full step
-  int tx, ty;       // maximum tile extent of the launch (sizes shared memory)
   int* queue;       // work counter (zeroed before the launch) for a persistent
                     // grid pulling tiles dynamically; null = static grid stride
-  int threads;      // CTA size (256 or 512); 0 = 256
   int gravity = 0;           // 1: add the gravity source (the blocks' accel)
   int npass = 0;             // passive scalars advected (0..4)
   const void* fc = nullptr;  // FluxOut<R> (device) on the final stage when the
                              // boundary fluxes are stored; null otherwise
   int block_fc = 0;          // 1: the blocks carry their own FluxOut (StageBlock::fc)
   int fc_g = 0;              // ghost depth of the blocks whose fluxes are stored
-  // shape of the launch, for the stage kernels compiled with it as constants
-  // (zero: not known, the run-time shape is used)
-  int full_tiles = 0;        // 1: every tile of the launch is tx x ty
-  int block_m = 0;           // every block's extent (ghosts included) along all
-                             // three axes, when they are all equal
 };
 
 // Boundary fluxes for flux correction (EnzoMethodMHDVlct.cpp:250-330):
