@@ -45,6 +45,10 @@ template <> struct SpeedBits<float> {
   static __device__ float val(T b) { return __uint_as_float(b); }
 };
 
+// fmax, in FP64 off the FP64 pipe
+__device__ __forceinline__ float speed_max(float a, float b) { return fmaxf(a, b); }
+__device__ __forceinline__ double speed_max(double a, double b) { return fmax_i(a, b); }
+
 template <class R, bool MHD, bool DE>
 __global__ void __launch_bounds__(256)
 timestep_kernel(const AuxBlock<R>* __restrict__ blocks, int nblocks,
@@ -126,9 +130,9 @@ timestep_kernel(const AuxBlock<R>* __restrict__ blocks, int nblocks,
       } else {
         cf = sqrt(cs2(g, rho[u], p));
       }
-      s[0] = fmax(s[0], fabs(vx[u]) + cf);
-      s[1] = fmax(s[1], fabs(vy[u]) + cf);
-      s[2] = fmax(s[2], fabs(vz[u]) + cf);
+      s[0] = speed_max(s[0], fabs(vx[u]) + cf);
+      s[1] = speed_max(s[1], fabs(vy[u]) + cf);
+      s[2] = speed_max(s[2], fabs(vz[u]) + cf);
     }
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;

@@ -36,21 +36,75 @@ template <class R> __device__ __forceinline__ bool ge0(R x) { return x >= R(0); 
 template <class R> __device__ __forceinline__ bool le0(R x) { return x <= R(0); }
 constexpr long long kInfBits = 0x7ff0000000000000LL;
 constexpr long long kAbsBits = 0x7fffffffffffffffLL;
+// (through a move that the compiler cannot see through: it would turn the
+// patterns below back into floating-point comparisons)
+__device__ __forceinline__ long long bits_of(double x) {
+  long long i;
+  asm("mov.b64 %0, %1;" : "=l"(i) : "d"(x));
+  return i;
+}
+__device__ __forceinline__ double abs_i(double x) {
+  return __longlong_as_double(bits_of(x) & kAbsBits);
+}
 template <> __device__ __forceinline__ bool gt0<double>(double x) {
-  const long long i = __double_as_longlong(x);
+  const long long i = bits_of(x);
   return i > 0 && i <= kInfBits;
 }
 template <> __device__ __forceinline__ bool lt0<double>(double x) {
-  const long long i = __double_as_longlong(x), a = i & kAbsBits;
+  const long long i = bits_of(x), a = i & kAbsBits;
   return i < 0 && a != 0 && a <= kInfBits;
 }
 template <> __device__ __forceinline__ bool ge0<double>(double x) {
-  const long long i = __double_as_longlong(x), a = i & kAbsBits;
+  const long long i = bits_of(x), a = i & kAbsBits;
   return (i >= 0 || a == 0) && a <= kInfBits;
 }
 template <> __device__ __forceinline__ bool le0<double>(double x) {
-  const long long i = __double_as_longlong(x), a = i & kAbsBits;
+  const long long i = bits_of(x), a = i & kAbsBits;
   return (i < 0 || a == 0) && a <= kInfBits;
+}
+// a < b, the larger and smaller of two with std::max / std::min's choice on
+// ties and NaN (below), fmax / fmin's, and products by powers of two and by
+// signs, all likewise off the FP64 pipe.
+__device__ __forceinline__ bool is_nan(double x) {
+  return (bits_of(x) & kAbsBits) > kInfBits;
+}
+__device__ __forceinline__ bool is_finite(double x) {
+  return (bits_of(x) & kAbsBits) < kInfBits;
+}
+__device__ __forceinline__ bool lt(double a, double b) {
+  const long long ia = bits_of(a), ib = bits_of(b);
+  // two's-complement order of the sign-magnitude patterns; zeros are equal
+  const long long ka = ia ^ ((ia >> 63) & kAbsBits), kb = ib ^ ((ib >> 63) & kAbsBits);
+  return ka < kb && ((ia | ib) & kAbsBits) != 0 && !is_nan(a) && !is_nan(b);
+}
+template <>
+__device__ __forceinline__ double smin<double>(double a, double b) {
+  return lt(b, a) ? b : a;
+}
+template <>
+__device__ __forceinline__ double smax<double>(double a, double b) {
+  return lt(a, b) ? b : a;
+}
+__device__ __forceinline__ double fmax_i(double a, double b) {
+  return is_nan(a) ? b : (lt(a, b) ? b : a);
+}
+__device__ __forceinline__ double fmin_i(double a, double b) {
+  return is_nan(a) ? b : (lt(b, a) ? b : a);
+}
+// Kept in a branch: without it the compiler would compute the rare case always
+// and select.
+__device__ __forceinline__ void rare_path() { asm volatile(""); }
+// x 2^K: a step of the exponent where x and the product are normal
+template <int K> __device__ __forceinline__ double scale2(double x) {
+  const int hi = __double2hiint(x), e = (hi >> 20) & 0x7ff;
+  if (e >= (K < 0 ? 1 - K : 1) && e <= (K > 0 ? 2046 - K : 2046))
+    return __hiloint2double(hi + K * (1 << 20), __double2loint(x));
+  if ((bits_of(x) & kAbsBits) == 0) return x;
+  rare_path();
+  return x * (K < 0 ? 1.0 / (1 << -K) : (double)(1 << K));
+}
+__device__ __forceinline__ double neg_if(double x, bool n) {
+  return n ? __longlong_as_double(bits_of(x) ^ ~kAbsBits) : x;
 }
 // enzo_utils::min of three values (utils.hpp:82-89)
 template <class R> __device__ __forceinline__ R min3(R a, R b, R c) {
@@ -65,28 +119,53 @@ template <class R> __device__ __forceinline__ R sqmag(R i, R j, R k) {
 template <class R> __device__ __forceinline__ R cs2(R g, R d, R p) {
   return g * p / d;
 }
-// fast_magnetosonic_speed, generic cos^2 branch (EnzoEOSIdeal.hpp:133-139)
-template <class R>
-__device__ __forceinline__ R cfast(R g, R d, R p, R bi, R bj, R bk) {
-  const R B2 = sqmag(bi, bj, bk);
-  const R c2 = cs2(g, d, p);
-  const R inv_density = R(1.0) / d;
-  const R va2 = B2 * inv_density;
-  const R va2_cos2 = (bi * bi) * inv_density;
-  const R s = c2 + va2;
-  return sqrt(R(0.5) * (va2 + c2 + sqrt(s * s - R(4.) * c2 * va2_cos2)));
-}
 // specific internal energy p / ((gamma-1) rho) (EnzoEOSIdeal.hpp:79-82)
-template <class R> __device__ __forceinline__ R specific_eint(R g, R d, R p) {
-  return p / ((g - R(1.0)) * d);
+template <class R> __device__ __forceinline__ R specific_eint(R gm1, R d, R p) {
+  return p / (gm1 * d);
 }
 // passive upwinding of the internal energy (EnzoRiemannUtils.hpp:224-249)
 template <class R>
-__device__ __forceinline__ R eint_flux(R g, R dl, R pl, R dr, R pr, R fd) {
-  const R el = specific_eint(g, dl, pl);
-  const R er = specific_eint(g, dr, pr);
-  const R up = ((fd > R(0)) ? R(1) : R(0)) * el + ((fd <= R(0)) ? R(1) : R(0)) * er;
+__device__ __forceinline__ R eint_flux(R gm1, R dl, R pl, R dr, R pr, R fd) {
+  const R el = specific_eint(gm1, dl, pl);
+  const R er = specific_eint(gm1, dr, pr);
+  const R up = (gt0(fd) ? R(1) : R(0)) * el + (le0(fd) ? R(1) : R(0)) * er;
   return up * fd;
+}
+
+// What the FP64 solvers take from a cell's density and pressure alone, divisions
+// and square roots: sound speed squared gamma p / rho (HLLC: the sound speed)
+// and 1 / rho for the fast speed, sqrt(rho) and p / (gamma - 1) for the Einfeldt
+// speeds.  With nearest-neighbour reconstruction a face's states are the cells'
+// own, and the six faces of a cell share them.
+struct Gas {
+  double g, gm1, igm1;  // gamma, gamma - 1, 1 / (gamma - 1)
+};
+template <int SOLVER> struct CellGas {
+  // values kept per cell
+  static constexpr int N = SOLVER == SOLVER_HLLD ? 2 : (SOLVER == SOLVER_HLLC ? 3 : 4);
+  double v[N];
+  __device__ __forceinline__ void init(const Gas& gas, double d, double p) {
+    const double c2 = cs2(gas.g, d, p);
+    v[0] = SOLVER == SOLVER_HLLC ? sqrt(c2) : c2;
+    if (SOLVER == SOLVER_HLLC) {
+      v[1] = sqrt(d);
+      v[2] = p / gas.gm1;
+    } else {
+      v[1] = 1.0 / d;
+      if (SOLVER == SOLVER_HLLE) {
+        v[2 % N] = sqrt(d);
+        v[3 % N] = p / gas.gm1;
+      }
+    }
+  }
+};
+// fast_magnetosonic_speed, generic cos^2 branch (EnzoEOSIdeal.hpp:133-139), from
+// gamma p / rho, 1 / rho, B^2 and B_i^2
+__device__ __forceinline__ double cfast_of(double c2, double inv_density, double B2, double bi2) {
+  const double va2 = B2 * inv_density;
+  const double va2_cos2 = bi2 * inv_density;
+  const double s = c2 + va2;
+  return sqrt(scale2<-1>(va2 + c2 + sqrt(s * s - scale2<2>(c2) * va2_cos2)));
 }
 
 // ------------------------------------------------------------ limiters ----
@@ -144,17 +223,19 @@ __device__ __forceinline__ R half_slope(R vm1, R v, R vp1, R theta) {
 template <>
 __device__ __forceinline__ double half_slope<double, RECON_PLM>(double vm1, double v,
                                                                 double vp1, double theta) {
-  const double dv_c = 0.5 * (vp1 - vm1);
+  const double dv_c = scale2<-1>(vp1 - vm1);
   const double dv_l = (v - vm1) * theta;
   const double dv_r = (vp1 - v) * theta;
-  const long long il = __double_as_longlong(dv_l), ir = __double_as_longlong(dv_r);
+  const long long il = bits_of(dv_l), ir = bits_of(dv_r);
   const long long al = il & kAbsBits, ar = ir & kAbsBits,
-                  ac = __double_as_longlong(dv_c) & kAbsBits;
+                  ac = bits_of(dv_c) & kAbsBits;
   long long m = al < ar ? al : ar;
   const long long most = al < ar ? ar : al;
   m = ac < m ? ac : m;
-  if ((most < ac ? ac : most) >= kInfBits || (m != 0 && m < 0x0020000000000000LL))
+  if ((most < ac ? ac : most) >= kInfBits || (m != 0 && m < 0x0020000000000000LL)) {
+    rare_path();
     return limiter_enzo_rk(vm1, v, vp1, theta) * 0.5;
+  }
   const bool opposite = al != 0 && ar != 0 && (il ^ ir) < 0;
   const long long sign = (al != 0 ? il : (ar != 0 ? ir : 0)) & ~kAbsBits;
   if (m != 0) m -= 0x0010000000000000LL;
@@ -178,26 +259,25 @@ template <class R> struct FaceFlux {
 // that is formed is the reference's expression on the same operands, so the
 // result is the same bit for bit; on GB300, whose FP64 pipe bounds the FP64
 // stages, the operands' selection by integer moves is free.
-template <class R> struct HlldSide {
-  R d, u, vj, vk, by, bz, pt, e, sd, sdm_inv, sdm;  // left or right state
-  R st_d, st_inv;                                   // star density and 1 / it
+struct HlldSide {
+  double d, u, vj, vk, by, bz, pt, e, sd, sdd, sdm_inv, sdm;  // left or right state
+  double st_d, st_inv;                                        // star density and 1 / it
 };
-template <class R> struct HlldStar {
-  R mx, my, mz, e, by, bz, vb;
+struct HlldStar {
+  double mx, my, mz, e, by, bz, vb;
 };
-template <class R>
-__device__ __forceinline__ HlldStar<R> hlld_star(const HlldSide<R>& W, R bxi, R bxsq, R spd2,
-                                                 R ptst, R thr) {
-  HlldStar<R> s;
+__device__ __forceinline__ HlldStar hlld_star(const HlldSide& W, double bxi, double bxsq,
+                                              double spd2, double ptst, double thr) {
+  HlldStar s;
   s.mx = W.st_d * spd2;
-  const R den = W.d * W.sd * W.sdm - bxsq;
-  if (fabs(den) < thr) {
+  const double den = W.sdd * W.sdm - bxsq;
+  if (lt(abs_i(den), thr)) {
     s.my = W.st_d * W.vj;
     s.mz = W.st_d * W.vk;
     s.by = W.by;
     s.bz = W.bz;
   } else {
-    R tmp = bxi * (W.sd - W.sdm) / den;
+    double tmp = bxi * (W.sd - W.sdm) / den;
     s.my = W.st_d * (W.vj - W.by * tmp);
     s.mz = W.st_d * (W.vk - W.bz * tmp);
     tmp = (W.d * (W.sd * W.sd) - bxsq) / den;
@@ -211,35 +291,35 @@ __device__ __forceinline__ HlldStar<R> hlld_star(const HlldSide<R>& W, R bxi, R 
   return s;
 }
 
-template <class R>
-__device__ __forceinline__ void hlld(R g, const R* wli, const R* wri,
-                                     FaceFlux<R>& out) {
-  const R SMALL = R(1.0e-8);
-  const R igm1 = R(1.0) / (g - R(1.0));
-  const R pressure_l = wli[L_E], pressure_r = wri[L_E];
-  const R bxi = wli[L_BI];
-  const R bxsq = bxi * bxi;
-  const R pbl = R(0.5) * (bxsq + (wli[L_BJ] * wli[L_BJ] + wli[L_BK] * wli[L_BK]));
-  const R pbr = R(0.5) * (bxsq + (wri[L_BJ] * wri[L_BJ] + wri[L_BK] * wri[L_BK]));
+__device__ __forceinline__ void hlld(const Gas& gas, const double* wli, const double* wri,
+                                     const CellGas<SOLVER_HLLD>& cl,
+                                     const CellGas<SOLVER_HLLD>& cr, FaceFlux<double>& out) {
+  const double SMALL = 1.0e-8;
+  const double pressure_l = wli[L_E], pressure_r = wri[L_E];
+  const double bxi = wli[L_BI];
+  const double bxsq = bxi * bxi;
+  const double b2l = bxsq + (wli[L_BJ] * wli[L_BJ] + wli[L_BK] * wli[L_BK]);
+  const double b2r = bxsq + (wri[L_BJ] * wri[L_BJ] + wri[L_BK] * wri[L_BK]);
+  const double pbl = scale2<-1>(b2l), pbr = scale2<-1>(b2r);
 
-  const R cfl = cfast(g, wli[L_RHO], pressure_l, wli[L_BI], wli[L_BJ], wli[L_BK]);
-  const R cfr = cfast(g, wri[L_RHO], pressure_r, wri[L_BI], wri[L_BJ], wri[L_BK]);
-  const R spd0 = smin(wli[L_VI] - cfl, wri[L_VI] - cfr);
-  const R spd4 = smax(wli[L_VI] + cfl, wri[L_VI] + cfr);
-  const R uld = wli[L_RHO], urd = wri[L_RHO];
-  const R ptl = pressure_l + pbl;
-  const R ptr = pressure_r + pbr;
-  const R sdl = spd0 - wli[L_VI];
-  const R sdr = spd4 - wri[L_VI];
-  const R sddl = uld * sdl, sddr = urd * sdr;
-  const R spd2 = (sdr * (wri[L_VI] * urd) - sdl * (wli[L_VI] * uld) + (ptl - ptr)) /
-                 (sdr * urd - sdl * uld);
+  const double cfl = cfast_of(cl.v[0], cl.v[1], b2l, bxsq);
+  const double cfr = cfast_of(cr.v[0], cr.v[1], b2r, bxsq);
+  const double spd0 = smin(wli[L_VI] - cfl, wri[L_VI] - cfr);
+  const double spd4 = smax(wli[L_VI] + cfl, wri[L_VI] + cfr);
+  const double uld = wli[L_RHO], urd = wri[L_RHO];
+  const double ptl = pressure_l + pbl;
+  const double ptr = pressure_r + pbr;
+  const double sdl = spd0 - wli[L_VI];
+  const double sdr = spd4 - wri[L_VI];
+  const double sddl = uld * sdl, sddr = urd * sdr;
+  const double spd2 = (sdr * (wri[L_VI] * urd) - sdl * (wli[L_VI] * uld) + (ptl - ptr)) /
+                      (sddr - sddl);
   // the reference's order of the cases: F_L (spd0 >= 0), F_R (spd4 <= 0), then
   // left star states for spd2 >= 0 and right ones otherwise
   const bool sup_l = ge0(spd0), outer = sup_l || le0(spd4);
   const bool left = sup_l || (!outer && ge0(spd2));
 
-  HlldSide<R> W;  // the side whose flux this is
+  HlldSide W;  // the side whose flux this is
   W.d = left ? uld : urd;
   W.u = left ? wli[L_VI] : wri[L_VI];
   W.vj = left ? wli[L_VJ] : wri[L_VJ];
@@ -248,12 +328,13 @@ __device__ __forceinline__ void hlld(R g, const R* wli, const R* wri,
   W.bz = left ? wli[L_BK] : wri[L_BK];
   W.pt = left ? ptl : ptr;
   W.sd = left ? sdl : sdr;
-  const R mx = W.u * W.d, my = W.vj * W.d, mz = W.vk * W.d;
+  W.sdd = left ? sddl : sddr;
+  const double mx = W.u * W.d, my = W.vj * W.d, mz = W.vk * W.d;
   {
-    const R ke = R(0.5) * W.d * (W.u * W.u + (W.vj * W.vj + W.vk * W.vk));
-    W.e = (left ? pressure_l : pressure_r) * igm1 + ke + (left ? pbl : pbr);
+    const double ke = scale2<-1>(W.d) * (W.u * W.u + (W.vj * W.vj + W.vk * W.vk));
+    W.e = (left ? pressure_l : pressure_r) * gas.igm1 + ke + (left ? pbl : pbr);
   }
-  R f[7];
+  double f[7];
   f[0] = mx;
   f[1] = mx * W.u + W.pt - bxsq;
   f[2] = my * W.u - bxi * W.by;
@@ -263,20 +344,20 @@ __device__ __forceinline__ void hlld(R g, const R* wli, const R* wri,
   f[6] = W.bz * W.u - bxi * W.vk;
 
   if (!outer) {
-    const R ptstl = ptl + sddl * (spd2 - wli[L_VI]);
-    const R ptstr = ptr + sddr * (spd2 - wri[L_VI]);
-    const R ptst = R(0.5) * (ptstr + ptstl);
-    const R thr = SMALL * ptst;
-    const R spdo = left ? spd0 : spd4;  // the side's outermost speed
+    const double ptstl = ptl + sddl * (spd2 - wli[L_VI]);
+    const double ptstr = ptr + sddr * (spd2 - wri[L_VI]);
+    const double ptst = scale2<-1>(ptstr + ptstl);
+    const double thr = SMALL * ptst;
+    const double spdo = left ? spd0 : spd4;  // the side's outermost speed
     W.sdm = spdo - spd2;
-    W.sdm_inv = R(1.0) / W.sdm;
-    W.st_d = W.d * W.sd * W.sdm_inv;
-    W.st_inv = R(1.0) / W.st_d;
-    const R sq = sqrt(W.st_d);
-    const R va = fabs(bxi) / sq;
-    const R spdi = spd2 + (left ? -va : va);  // its Alfven speed (spd1 / spd3)
+    W.sdm_inv = 1.0 / W.sdm;
+    W.st_d = W.sdd * W.sdm_inv;
+    W.st_inv = 1.0 / W.st_d;
+    const double sq = sqrt(W.st_d);
+    const double va = abs_i(bxi) / sq;
+    const double spdi = spd2 + neg_if(va, left);  // its Alfven speed (spd1 / spd3)
     const bool two = left ? !ge0(spdi) : gt0(spdi);
-    const HlldStar<R> st = hlld_star(W, bxi, bxsq, spd2, ptst, thr);
+    const HlldStar st = hlld_star(W, bxi, bxsq, spd2, ptst, thr);
     f[0] = f[0] + spdo * (W.st_d - W.d);
     f[1] = f[1] + spdo * (st.mx - mx);
     f[2] = f[2] + spdo * (st.my - my);
@@ -285,9 +366,9 @@ __device__ __forceinline__ void hlld(R g, const R* wli, const R* wri,
     f[5] = f[5] + spdo * (st.by - W.by);
     f[6] = f[6] + spdo * (st.bz - W.bz);
     if (two) {
-      R dy = st.my, dz = st.mz, de = st.e, dby = st.by, dbz = st.bz;
-      if (!(R(0.5) * bxsq < thr)) {
-        HlldSide<R> V;  // the other side
+      double dy = st.my, dz = st.mz, de = st.e, dby = st.by, dbz = st.bz;
+      if (!lt(scale2<-1>(bxsq), thr)) {
+        HlldSide V;  // the other side
         V.d = left ? urd : uld;
         V.u = left ? wri[L_VI] : wli[L_VI];
         V.vj = left ? wri[L_VJ] : wli[L_VJ];
@@ -295,38 +376,47 @@ __device__ __forceinline__ void hlld(R g, const R* wli, const R* wri,
         V.by = left ? wri[L_BJ] : wli[L_BJ];
         V.bz = left ? wri[L_BK] : wli[L_BK];
         V.sd = left ? sdr : sdl;
+        V.sdd = left ? sddr : sddl;
         V.sdm = (left ? spd4 : spd0) - spd2;
-        V.sdm_inv = R(1.0) / V.sdm;
-        V.st_d = V.d * V.sd * V.sdm_inv;
-        V.st_inv = R(1.0) / V.st_d;
-        V.pt = V.e = R(0);  // its energy is not needed
-        const R sqv = sqrt(V.st_d);
-        const HlldStar<R> sv = hlld_star(V, bxi, bxsq, spd2, ptst, thr);
-        // left and right values, in the reference's expressions
-        const R sqrtdl = left ? sq : sqv, sqrtdr = left ? sqv : sq;
-        const R invsumd = R(1.0) / (sqrtdl + sqrtdr);
-        const R bxsig = gt0(bxi) ? R(1.0) : R(-1.0);
-        const R vy = st.my * W.st_inv, vz = st.mz * W.st_inv;
-        const R oy = sv.my * V.st_inv, oz = sv.mz * V.st_inv;
-        const R lvy = left ? vy : oy, rvy = left ? oy : vy;
-        const R lvz = left ? vz : oz, rvz = left ? oz : vz;
-        const R lby = left ? st.by : sv.by, rby = left ? sv.by : st.by;
-        const R lbz = left ? st.bz : sv.bz, rbz = left ? sv.bz : st.bz;
-        const R lst_d = left ? W.st_d : V.st_d;
-        const R ty = invsumd * (sqrtdl * lvy + sqrtdr * rvy + bxsig * (rby - lby));
-        const R tz = invsumd * (sqrtdl * lvz + sqrtdr * rvz + bxsig * (rbz - lbz));
-        const R sqlr = bxsig * sqrtdl * sqrtdr;
+        V.sdm_inv = 1.0 / V.sdm;
+        V.st_d = V.sdd * V.sdm_inv;
+        V.st_inv = 1.0 / V.st_d;
+        V.pt = V.e = 0.0;  // its energy is not needed
+        const double sqv = sqrt(V.st_d);
+        const HlldStar sv = hlld_star(V, bxi, bxsq, spd2, ptst, thr);
+        // left and right values, in the reference's expressions; the sign of
+        // B_x multiplies by flipping signs
+        const double sqrtdl = left ? sq : sqv, sqrtdr = left ? sqv : sq;
+        const double invsumd = 1.0 / (sqrtdl + sqrtdr);
+        const bool bneg = !gt0(bxi);
+        const double vy = st.my * W.st_inv, vz = st.mz * W.st_inv;
+        const double oy = sv.my * V.st_inv, oz = sv.mz * V.st_inv;
+        const double lvy = left ? vy : oy, rvy = left ? oy : vy;
+        const double lvz = left ? vz : oz, rvz = left ? oz : vz;
+        const double lby = left ? st.by : sv.by, rby = left ? sv.by : st.by;
+        const double lbz = left ? st.bz : sv.bz, rbz = left ? sv.bz : st.bz;
+        const double lst_d = left ? W.st_d : V.st_d;
+        const double ty =
+            invsumd * (sqrtdl * lvy + sqrtdr * rvy + neg_if(rby - lby, bneg));
+        const double tz =
+            invsumd * (sqrtdl * lvz + sqrtdr * rvz + neg_if(rbz - lbz, bneg));
+        const double sqlr = neg_if(sqrtdl * sqrtdr, bneg);
         dby = invsumd * (sqrtdl * rby + sqrtdr * lby + sqlr * (rvy - lvy));
         dbz = invsumd * (sqrtdl * rbz + sqrtdr * lbz + sqlr * (rvz - lvz));
         dy = W.st_d * ty;
         dz = W.st_d * tz;
         // v** . B**, from the left side's values for both sides
-        const R vb = spd2 * bxi + ((lst_d * ty) * dby + (lst_d * tz) * dbz) / lst_d;
-        const R t = sq * bxsig * (st.vb - vb);
-        de = st.e + (left ? -t : t);
+        const double vb = spd2 * bxi + ((lst_d * ty) * dby + (lst_d * tz) * dbz) / lst_d;
+        const double t = neg_if(sq, bneg) * (st.vb - vb);
+        de = st.e + neg_if(t, left);
       }
-      f[0] = f[0] + spdi * (W.st_d - W.st_d);
-      f[1] = f[1] + spdi * (st.mx - st.mx);
+      // (the density and the normal momentum do not jump there: a zero, but
+      // where a value is not finite)
+      if (!is_finite(W.st_d) || !is_finite(st.mx) || !is_finite(spdi)) {
+        rare_path();
+        f[0] = f[0] + spdi * (W.st_d - W.st_d);
+        f[1] = f[1] + spdi * (st.mx - st.mx);
+      }
       f[2] = f[2] + spdi * (dy - st.my);
       f[3] = f[3] + spdi * (dz - st.mz);
       f[4] = f[4] + spdi * (de - st.e);
@@ -335,14 +425,14 @@ __device__ __forceinline__ void hlld(R g, const R* wli, const R* wri,
     }
   }
   out.f[L_RHO] = f[0];
-  out.f[L_BI] = R(0.0);
+  out.f[L_BI] = 0.0;
   out.f[L_BJ] = f[5];
   out.f[L_BK] = f[6];
   out.f[L_VI] = f[1];
   out.f[L_VJ] = f[2];
   out.f[L_VK] = f[3];
   out.f[L_E] = f[4];
-  out.eflux = eint_flux(g, wli[L_RHO], pressure_l, wri[L_RHO], pressure_r, f[0]);
+  out.eflux = eint_flux(gas.gm1, wli[L_RHO], pressure_l, wri[L_RHO], pressure_r, f[0]);
   if (gt0(spd0)) {
     out.vbar = wli[L_VI];
   } else if (lt0(spd4)) {
@@ -376,9 +466,8 @@ __device__ __forceinline__ float2 sub(float2 a, float2 b) {
 }
 }  // namespace packed
 
-template <>
-__device__ __forceinline__ void hlld<float>(float g, const float* wli, const float* wri,
-                                            FaceFlux<float>& out) {
+__device__ __forceinline__ void hlld(float g, const float* wli, const float* wri,
+                                     FaceFlux<float>& out) {
   using namespace packed;
   const float SMALL = 1.0e-8f;
   const float igm1 = 1.0f / (g - 1.0f);
@@ -503,193 +592,191 @@ __device__ __forceinline__ void hlld<float>(float g, const float* wli, const flo
   out.f[L_BJ] = left ? r5.x : r5.y;
   out.f[L_BK] = left ? r6.x : r6.y;
   out.f[L_BI] = 0.0f;
-  out.eflux = eint_flux(g, d.x, p.x, d.y, p.y, out.f[L_RHO]);
+  out.eflux = eint_flux(g - 1.0f, d.x, p.x, d.y, p.y, out.f[L_RHO]);
   if (spd0 > 0.0f) out.vbar = u.x;
   else if (spd4 < 0.0f) out.vbar = u.y;
   else out.vbar = spd2 * (spd2 >= 0.0f ? sd.x * sdm_inv.x : sd.y * sdm_inv.y);
 }
 
-// conserved state from primitives (EnzoRiemannUtils.hpp:48-82)
-template <class R, bool MHD>
-__device__ __forceinline__ void conserved(R g, const R* w, R* u) {
-  u[L_RHO] = w[L_RHO];
-  u[L_BI] = w[L_BI]; u[L_BJ] = w[L_BJ]; u[L_BK] = w[L_BK];
-  u[L_VI] = w[L_VI] * w[L_RHO];
-  u[L_VJ] = w[L_VJ] * w[L_RHO];
-  u[L_VK] = w[L_VK] * w[L_RHO];
-  const R density = w[L_RHO], pressure = w[L_E];
-  const R internal_edens = pressure / (g - R(1.0));
-  const R kinetic_edens = R(0.5) * density * sqmag(w[L_VI], w[L_VJ], w[L_VK]);
-  const R magnetic_edens = MHD ? R(0.5) * sqmag(w[L_BI], w[L_BJ], w[L_BK])
-                               : R(0.5) * sqmag(R(0), R(0), R(0));
-  u[L_E] = internal_edens + kinetic_edens + magnetic_edens;
+// Conserved total energy (EnzoRiemannUtils.hpp:48-82); pg: p / (gamma - 1).
+// Hydro adds a magnetic energy of zero, which changes no value.
+template <bool MHD>
+__device__ __forceinline__ double energy_of(const double* w, double pg, double b2) {
+  const double ke = scale2<-1>(w[L_RHO]) * sqmag(w[L_VI], w[L_VJ], w[L_VK]);
+  return MHD ? pg + ke + scale2<-1>(b2) : pg + ke;
 }
 
-// ideal-MHD fluxes (EnzoRiemannUtils.hpp:111-149)
-template <class R, bool MHD>
-__device__ __forceinline__ void physical_flux(const R* w, const R* u, R pressure,
-                                              R* f) {
-  const R vi = w[L_VI], vj = w[L_VJ], vk = w[L_VK];
-  const R Bi = MHD ? w[L_BI] : R(0), Bj = MHD ? w[L_BJ] : R(0),
-          Bk = MHD ? w[L_BK] : R(0);
-  const R etot = u[L_E];
-  const R ptot = pressure + R(0.5) * sqmag(Bi, Bj, Bk);
-  const R mom_i = u[L_VI];
-  f[L_RHO] = mom_i;
-  f[L_VI] = mom_i * vi - Bi * Bi + ptot;
-  f[L_VJ] = mom_i * vj - Bj * Bi;
-  f[L_VK] = mom_i * vk - Bk * Bi;
-  f[L_E] = ((etot + ptot) * vi - (Bi * vi + (Bj * vj + Bk * vk)) * Bi);
-  f[L_BI] = R(0);
-  f[L_BJ] = Bj * vi - Bi * vj;
-  f[L_BK] = Bk * vi - Bi * vk;
-}
-
-// Einfeldt wave speeds with Roe averages (EnzoRiemannHLL.hpp:44-172)
-template <class R, bool MHD>
-__device__ __forceinline__ void einfeldt(R g, const R* wl, const R* wr,
-                                         const R* Ul, const R* Ur, R pl, R pr,
-                                         R* bp, R* bm) {
-  R c_l, c_r;
+// Einfeldt wave speeds with Roe averages (EnzoRiemannHLL.hpp:44-172).  c: sound
+// (hydro) or fast (MHD) speeds, sq: sqrt(rho), U: total energies, b2: B^2.
+template <bool MHD>
+__device__ __forceinline__ void einfeldt(const Gas& gas, const double* wl, const double* wr,
+                                         double c_l, double c_r, double sqrtrho_l,
+                                         double sqrtrho_r, double El, double Er, double b2l,
+                                         double b2r, double* bp, double* bm) {
+  const double left_speed = (wl[L_VI] - c_l);
+  const double right_speed = (wr[L_VI] + c_r);
+  const double inv_tot = 1.0 / (sqrtrho_l + sqrtrho_r);
+  const double vi_roe = (sqrtrho_l * wl[L_VI] + sqrtrho_r * wr[L_VI]) * inv_tot;
+  const double vj_roe = (sqrtrho_l * wl[L_VJ] + sqrtrho_r * wr[L_VJ]) * inv_tot;
+  const double vk_roe = (sqrtrho_l * wl[L_VK] + sqrtrho_r * wr[L_VK]) * inv_tot;
+  const double v_roe2 = vi_roe * vi_roe + vj_roe * vj_roe + vk_roe * vk_roe;
+  double ptot_l = wl[L_E], ptot_r = wr[L_E];
   if (MHD) {
-    c_l = cfast(g, wl[L_RHO], pl, wl[L_BI], wl[L_BJ], wl[L_BK]);
-    c_r = cfast(g, wr[L_RHO], pr, wr[L_BI], wr[L_BJ], wr[L_BK]);
-  } else {
-    c_l = sqrt(cs2(g, wl[L_RHO], pl));
-    c_r = sqrt(cs2(g, wr[L_RHO], pr));
+    ptot_l += scale2<-1>(b2l);
+    ptot_r += scale2<-1>(b2r);
   }
-  const R left_speed = (wl[L_VI] - c_l);
-  const R right_speed = (wr[L_VI] + c_r);
-  const R sqrtrho_l = sqrt(wl[L_RHO]);
-  const R sqrtrho_r = sqrt(wr[L_RHO]);
-  const R inv_tot = R(1.0) / (sqrtrho_l + sqrtrho_r);
-  const R vi_roe = (sqrtrho_l * wl[L_VI] + sqrtrho_r * wr[L_VI]) * inv_tot;
-  const R vj_roe = (sqrtrho_l * wl[L_VJ] + sqrtrho_r * wr[L_VJ]) * inv_tot;
-  const R vk_roe = (sqrtrho_l * wl[L_VK] + sqrtrho_r * wr[L_VK]) * inv_tot;
-  const R v_roe2 = vi_roe * vi_roe + vj_roe * vj_roe + vk_roe * vk_roe;
-  R ptot_l = pl, ptot_r = pr;
-  if (MHD) {
-    ptot_l += R(0.5) * sqmag(wl[L_BI], wl[L_BJ], wl[L_BK]);
-    ptot_r += R(0.5) * sqmag(wr[L_BI], wr[L_BJ], wr[L_BK]);
-  }
-  const R h_l = (Ul[L_E] + ptot_l) / wl[L_RHO];
-  const R h_r = (Ur[L_E] + ptot_r) / wr[L_RHO];
-  const R h_roe = (sqrtrho_l * h_l + sqrtrho_r * h_r) * inv_tot;
-  R c_roe;
+  const double h_l = (El + ptot_l) / wl[L_RHO];
+  const double h_r = (Er + ptot_r) / wr[L_RHO];
+  const double h_roe = (sqrtrho_l * h_l + sqrtrho_r * h_r) * inv_tot;
+  double c_roe;
   if (MHD) {  // roe_cfast_ (:134-172)
-    const R rho_roe = sqrtrho_l * sqrtrho_r;
-    const R bi_roe = wl[L_BI];
-    const R bj_roe = (sqrtrho_l * wr[L_BJ] + sqrtrho_r * wl[L_BJ]) * inv_tot;
-    const R bk_roe = (sqrtrho_l * wr[L_BK] + sqrtrho_r * wl[L_BK]) * inv_tot;
-    const R b_roe2 = bi_roe * bi_roe + bj_roe * bj_roe + bk_roe * bk_roe;
-    const R gamma_prime = g - R(1.);
-    const R dbj = wl[L_BJ] - wr[L_BJ];
-    const R dbk = wl[L_BK] - wr[L_BK];
-    const R x_prime =
-        ((dbj * dbj + dbk * dbk) * R(0.5) * (gamma_prime - R(1)) * inv_tot);
-    const R y_prime =
-        ((gamma_prime - R(1)) * (wl[L_RHO] + wr[L_RHO]) * R(0.5) / rho_roe);
-    const R tilde_a2 =
-        (gamma_prime * (h_roe - R(0.5) * v_roe2 - b_roe2 / rho_roe) - x_prime);
-    const R tilde_vai2 = bi_roe * bi_roe / rho_roe;
-    const R tilde_va2 = (tilde_vai2 + (gamma_prime - y_prime) *
-                                          (bj_roe * bj_roe + bk_roe * bk_roe) /
-                                          rho_roe);
-    const R s = tilde_a2 + tilde_va2;
-    c_roe = sqrt(R(0.5) * (tilde_a2 + tilde_va2 +
-                           sqrt(s * s - R(4) * tilde_a2 * tilde_vai2)));
+    const double rho_roe = sqrtrho_l * sqrtrho_r;
+    const double bi_roe = wl[L_BI];
+    const double bj_roe = (sqrtrho_l * wr[L_BJ] + sqrtrho_r * wl[L_BJ]) * inv_tot;
+    const double bk_roe = (sqrtrho_l * wr[L_BK] + sqrtrho_r * wl[L_BK]) * inv_tot;
+    const double bi2 = bi_roe * bi_roe;
+    const double b_roe2 = bi2 + bj_roe * bj_roe + bk_roe * bk_roe;
+    const double gamma_prime = gas.gm1;
+    const double gp1 = gamma_prime - 1.;
+    const double dbj = wl[L_BJ] - wr[L_BJ];
+    const double dbk = wl[L_BK] - wr[L_BK];
+    const double x_prime = (scale2<-1>(dbj * dbj + dbk * dbk) * gp1 * inv_tot);
+    const double y_prime = (scale2<-1>(gp1 * (wl[L_RHO] + wr[L_RHO])) / rho_roe);
+    const double tilde_a2 =
+        (gamma_prime * (h_roe - scale2<-1>(v_roe2) - b_roe2 / rho_roe) - x_prime);
+    const double tilde_vai2 = bi2 / rho_roe;
+    const double tilde_va2 =
+        (tilde_vai2 + (gamma_prime - y_prime) * (bj_roe * bj_roe + bk_roe * bk_roe) / rho_roe);
+    const double s = tilde_a2 + tilde_va2;
+    c_roe = sqrt(scale2<-1>(tilde_a2 + tilde_va2 +
+                            sqrt(s * s - scale2<2>(tilde_a2) * tilde_vai2)));
   } else {  // roe_cs_ (:123-130)
-    const R temp = h_roe - R(0.5) * v_roe2;
-    c_roe = sqrt((g - R(1)) * smax(temp, R(0.)));
+    const double temp = h_roe - scale2<-1>(v_roe2);
+    c_roe = sqrt(gas.gm1 * smax(temp, 0.));
   }
-  *bp = fmax(vi_roe + c_roe, right_speed);
-  *bm = fmin(vi_roe - c_roe, left_speed);
+  *bp = fmax_i(vi_roe + c_roe, right_speed);
+  *bm = fmin_i(vi_roe - c_roe, left_speed);
 }
 
-// HLLE for MHD (EnzoRiemannHLL.hpp:238-345)
-template <class R>
-__device__ __forceinline__ void hlle(R g, const R* wl, const R* wr,
-                                     FaceFlux<R>& out) {
-  const R pl = wl[L_E], pr = wr[L_E];
-  R Ul[8], Ur[8], Fl[8], Fr[8];
-  conserved<R, true>(g, wl, Ul);
-  conserved<R, true>(g, wr, Ur);
-  physical_flux<R, true>(wl, Ul, pl, Fl);
-  physical_flux<R, true>(wr, Ur, pr, Fr);
-  R bp, bm;
-  einfeldt<R, true>(g, wl, wr, Ul, Ur, pl, pr, &bp, &bm);
-  bp = fmax(bp, R(0.0));
-  bm = fmin(bm, R(0.0));
-  const R inv_speed_diff = R(1.) / (bp - bm);
+// HLLE for MHD (EnzoRiemannHLL.hpp:238-345), physical fluxes as in
+// EnzoRiemannUtils.hpp:111-149
+__device__ __forceinline__ void hlle(const Gas& gas, const double* wl, const double* wr,
+                                     const CellGas<SOLVER_HLLE>& cl,
+                                     const CellGas<SOLVER_HLLE>& cr, FaceFlux<double>& out) {
+  const double bi2 = wl[L_BI] * wl[L_BI];  // the face's own B_i on both sides
+  double Ul[8], Ur[8], Fl[8], Fr[8], b2[2], c[2];
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    const double* w = k == 0 ? wl : wr;
+    const CellGas<SOLVER_HLLE>& cg = k == 0 ? cl : cr;
+    double *U = k == 0 ? Ul : Ur, *F = k == 0 ? Fl : Fr;
+    const double vi = w[L_VI], vj = w[L_VJ], vk = w[L_VK];
+    const double Bi = w[L_BI], Bj = w[L_BJ], Bk = w[L_BK];
+    b2[k] = bi2 + (Bj * Bj + Bk * Bk);
+    c[k] = cfast_of(cg.v[0], cg.v[1], b2[k], bi2);
+    U[L_RHO] = w[L_RHO];
+    U[L_BJ] = Bj;
+    U[L_BK] = Bk;
+    U[L_VI] = vi * w[L_RHO];
+    U[L_VJ] = vj * w[L_RHO];
+    U[L_VK] = vk * w[L_RHO];
+    U[L_E] = energy_of<true>(w, cg.v[3], b2[k]);
+    const double ptot = w[L_E] + scale2<-1>(b2[k]);
+    const double mom_i = U[L_VI];
+    F[L_RHO] = mom_i;
+    F[L_VI] = mom_i * vi - bi2 + ptot;
+    F[L_VJ] = mom_i * vj - Bj * Bi;
+    F[L_VK] = mom_i * vk - Bk * Bi;
+    F[L_E] = ((U[L_E] + ptot) * vi - (Bi * vi + (Bj * vj + Bk * vk)) * Bi);
+    F[L_BJ] = Bj * vi - Bi * vj;
+    F[L_BK] = Bk * vi - Bi * vk;
+  }
+  double bp, bm;
+  einfeldt<true>(gas, wl, wr, c[0], c[1], cl.v[2], cr.v[2], Ul[L_E], Ur[L_E], b2[0], b2[1], &bp,
+                 &bm);
+  bp = fmax_i(bp, 0.0);
+  bm = fmin_i(bm, 0.0);
+  const double inv_speed_diff = 1. / (bp - bm);
 #pragma unroll
   for (int k = 0; k < 8; k++) {
-    out.f[k] = ((bp * Fl[k] - bm * Fr[k] + (Ur[k] - Ul[k]) * bp * bm) *
-                inv_speed_diff);
+    out.f[k] = k == L_BI ? 0.0
+                         : ((bp * Fl[k] - bm * Fr[k] + (Ur[k] - Ul[k]) * bp * bm) *
+                            inv_speed_diff);
   }
-  out.eflux = eint_flux(g, wl[L_RHO], pl, wr[L_RHO], pr, out.f[L_RHO]);
+  out.eflux = eint_flux(gas.gm1, wl[L_RHO], wl[L_E], wr[L_RHO], wr[L_E], out.f[L_RHO]);
   out.vbar = (bp * wl[L_VI] - bm * wr[L_VI]) * inv_speed_diff;
 }
 
-// HLLC for hydrodynamics (EnzoRiemannHLLC.hpp:34-172)
-template <class R>
-__device__ __forceinline__ void hllc(R g, const R* wl, const R* wr,
-                                     FaceFlux<R>& out) {
-  const R pl = wl[L_E], pr = wr[L_E];
-  R Ul[8], Ur[8];
-  conserved<R, false>(g, wl, Ul);
-  conserved<R, false>(g, wr, Ur);
-  R cs_l, cs_r;
-  einfeldt<R, false>(g, wl, wr, Ul, Ur, pl, pr, &cs_r, &cs_l);
-  const R bm = fmin(cs_l, R(0.0));
-  const R bp = fmax(cs_r, R(0.0));
-  const R tl = (pl - (cs_l - wl[L_VI]) * wl[L_RHO] * wl[L_VI]);
-  const R tr = (pr - (cs_r - wr[L_VI]) * wr[L_RHO] * wr[L_VI]);
-  const R dl = wl[L_RHO] * (cs_l - wl[L_VI]);
-  const R dr = -wr[L_RHO] * (cs_r - wr[L_VI]);
-  const R q1 = R(1.0) / (dl + dr);
-  const R cw = (tr - tl) * q1;
-  R cp = (dl * tr + dr * tl) * q1;
-  R sl, sr, sm;
-  if (cw >= R(0.)) {
-    sl = cw / (cw - bm);
-    sr = R(0.);
-    sm = -bm / (cw - bm);
-  } else {
-    sl = R(0.);
-    sr = -cw / (bp - cw);
-    sm = bp / (bp - cw);
+// HLLC for hydrodynamics (EnzoRiemannHLLC.hpp:34-172).  One of the two sides has
+// the weight zero; its products are zero, and left out, where its state is
+// finite.
+__device__ __forceinline__ void hllc(const Gas& gas, const double* wl, const double* wr,
+                                     const CellGas<SOLVER_HLLC>& cl,
+                                     const CellGas<SOLVER_HLLC>& cr, FaceFlux<double>& out) {
+  const double pl = wl[L_E], pr = wr[L_E];
+  const double El = energy_of<false>(wl, cl.v[2], 0.0), Er = energy_of<false>(wr, cr.v[2], 0.0);
+  double cs_l, cs_r;
+  einfeldt<false>(gas, wl, wr, cl.v[0], cr.v[0], cl.v[1], cr.v[1], El, Er, 0.0, 0.0, &cs_r, &cs_l);
+  const double bm = fmin_i(cs_l, 0.0);
+  const double bp = fmax_i(cs_r, 0.0);
+  const double ul = cs_l - wl[L_VI], ur = cs_r - wr[L_VI];
+  const double tl = (pl - ul * wl[L_RHO] * wl[L_VI]);
+  const double tr = (pr - ur * wr[L_RHO] * wr[L_VI]);
+  const double dl = wl[L_RHO] * ul;
+  const double dr = neg_if(wr[L_RHO], true) * ur;
+  const double q1 = 1.0 / (dl + dr);
+  const double cw = (tr - tl) * q1;
+  const double cp = smax((dl * tr + dr * tl) * q1, 0.);
+  const bool left = ge0(cw);
+  const double den = left ? cw - bm : bp - cw;
+  const double sd = neg_if(cw, !left) / den;      // the side's weight
+  const double sm = (left ? neg_if(bm, true) : bp) / den;
+  // the side's momentum, energy, relative speed and fluxes
+  auto side = [&](const double* w, double E, double b, double* f, double& ub) {
+    const double mi = w[L_VI] * w[L_RHO];
+    ub = w[L_VI] - b;
+    f[0] = mi - b * w[L_RHO];
+    f[1] = mi * ub + w[L_E];
+    f[2] = (w[L_RHO] * w[L_VJ] * ub);
+    f[3] = (w[L_RHO] * w[L_VK] * ub);
+    f[4] = (E * ub + w[L_E] * w[L_VI]);
+  };
+  double w[8], f[5], ub;
+#pragma unroll
+  for (int k = 0; k < 8; k++) w[k] = left ? wl[k] : wr[k];
+  side(w, left ? El : Er, left ? bm : bp, f, ub);
+#pragma unroll
+  for (int k = 0; k < 5; k++) f[k] = sd * f[k];
+  ub = sd * ub;
+  double o[8];
+#pragma unroll
+  for (int k = 0; k < 8; k++) o[k] = left ? wr[k] : wl[k];
+  const double Eo = left ? Er : El, bo = left ? bp : bm;
+  if (!is_finite(o[L_RHO]) || !is_finite(o[L_VI]) || !is_finite(o[L_VJ]) ||
+      !is_finite(o[L_VK]) || !is_finite(o[L_E]) || !is_finite(Eo) || !is_finite(bo)) {
+    rare_path();
+    double fo[5], uo;
+    side(o, Eo, bo, fo, uo);
+#pragma unroll
+    for (int k = 0; k < 5; k++) f[k] += 0.0 * fo[k];
+    ub += 0.0 * uo;
   }
-  cp = smax(cp, R(0.));
-  const R momentumi_l = Ul[L_VI], momentumi_r = Ur[L_VI];
-  const R dfl = momentumi_l - bm * wl[L_RHO];
-  const R dfr = momentumi_r - bp * wr[L_RHO];
-  const R ufl = momentumi_l * (wl[L_VI] - bm) + pl;
-  const R ufr = momentumi_r * (wr[L_VI] - bp) + pr;
-  const R vfl = (wl[L_RHO] * wl[L_VJ] * (wl[L_VI] - bm));
-  const R vfr = (wr[L_RHO] * wr[L_VJ] * (wr[L_VI] - bp));
-  const R wfl = (wl[L_RHO] * wl[L_VK] * (wl[L_VI] - bm));
-  const R wfr = (wr[L_RHO] * wr[L_VK] * (wr[L_VI] - bp));
-  const R efl = (Ul[L_E] * (wl[L_VI] - bm) + pl * wl[L_VI]);
-  const R efr = (Ur[L_E] * (wr[L_VI] - bp) + pr * wr[L_VI]);
-  out.f[L_RHO] = sl * dfl + sr * dfr;
-  out.f[L_VI] = sl * ufl + sr * ufr;
-  out.f[L_VJ] = sl * vfl + sr * vfr;
-  out.f[L_VK] = sl * wfl + sr * wfr;
-  out.f[L_E] = sl * efl + sr * efr;
-  out.f[L_VI] += (sm * cp);
-  out.f[L_E] += (sm * cp * cw);
-  out.f[L_BI] = out.f[L_BJ] = out.f[L_BK] = R(0);
-  out.eflux = eint_flux(g, wl[L_RHO], pl, wr[L_RHO], pr, out.f[L_RHO]);
-  out.vbar = (sl * (wl[L_VI] - bm) + sr * (wr[L_VI] - bp));
+  out.f[L_RHO] = f[0];
+  out.f[L_VI] = f[1] + (sm * cp);
+  out.f[L_VJ] = f[2];
+  out.f[L_VK] = f[3];
+  out.f[L_E] = f[4] + (sm * cp * cw);
+  out.f[L_BI] = out.f[L_BJ] = out.f[L_BK] = 0.0;
+  out.eflux = eint_flux(gas.gm1, wl[L_RHO], pl, wr[L_RHO], pr, out.f[L_RHO]);
+  out.vbar = ub;
 }
 
 // HLLE in FP32 (EnzoRiemannHLL.hpp:44-345): the same states, Einfeldt
 // speeds and flux as the FP64 form, the left and right states in the two
 // lanes of packed FP32 arithmetic.  Differences from the FP64 form lie only
 // in rounding.
-template <>
-__device__ __forceinline__ void hlle<float>(float g, const float* wl, const float* wr,
-                                            FaceFlux<float>& out) {
+__device__ __forceinline__ void hlle(float g, const float* wl, const float* wr,
+                                     FaceFlux<float>& out) {
   using namespace packed;
   const float2 HALF = s2(0.5f);
   const float2 p = f2(wl[L_E], wr[L_E]);
@@ -767,7 +854,7 @@ __device__ __forceinline__ void hlle<float>(float g, const float* wl, const floa
     const float2 t = mul(BPM, F[k]);
     out.f[k] = ((t.x + t.y) + (U[k].y - U[k].x) * bpbm) * inv_speed_diff;
   }
-  out.eflux = eint_flux(g, d.x, p.x, d.y, p.y, out.f[L_RHO]);
+  out.eflux = eint_flux(g - 1.0f, d.x, p.x, d.y, p.y, out.f[L_RHO]);
   out.vbar = (bp * u.x - bm * u.y) * inv_speed_diff;
 }
 
@@ -775,9 +862,8 @@ __device__ __forceinline__ void hlle<float>(float g, const float* wl, const floa
 // EnzoRiemannHLL.hpp:44-172): the same states, speeds and flux as the FP64
 // form, the left and right states in the two lanes of packed FP32
 // arithmetic.  Differences from the FP64 form lie only in rounding.
-template <>
-__device__ __forceinline__ void hllc<float>(float g, const float* wl, const float* wr,
-                                            FaceFlux<float>& out) {
+__device__ __forceinline__ void hllc(float g, const float* wl, const float* wr,
+                                     FaceFlux<float>& out) {
   using namespace packed;
   const float2 HALF = s2(0.5f);
   const float2 p = f2(wl[L_E], wr[L_E]);
@@ -837,16 +923,34 @@ __device__ __forceinline__ void hllc<float>(float g, const float* wl, const floa
   out.f[L_VK] = fw.x + fw.y;
   out.f[L_E] = (fe.x + fe.y) + sm * cp * cw;
   out.f[L_BI] = out.f[L_BJ] = out.f[L_BK] = 0.0f;
-  out.eflux = eint_flux(g, d.x, p.x, d.y, p.y, out.f[L_RHO]);
+  out.eflux = eint_flux(g - 1.0f, d.x, p.x, d.y, p.y, out.f[L_RHO]);
   out.vbar = fvb.x + fvb.y;
 }
 
-template <int SOLVER, class R>
-__device__ __forceinline__ void riemann(R g, const R* wl, const R* wr,
-                                        FaceFlux<R>& out) {
-  if (SOLVER == SOLVER_HLLD) hlld<R>(g, wl, wr, out);
-  else if (SOLVER == SOLVER_HLLE) hlle<R>(g, wl, wr, out);
-  else hllc<R>(g, wl, wr, out);
+// The face flux of SOLVER: FP32 from gamma, FP64 from the gas constants and the
+// cells' (or face states') own quantities.
+template <int SOLVER>
+__device__ __forceinline__ void riemann(float g, const float* wl, const float* wr,
+                                        FaceFlux<float>& out) {
+  if (SOLVER == SOLVER_HLLD) hlld(g, wl, wr, out);
+  else if (SOLVER == SOLVER_HLLE) hlle(g, wl, wr, out);
+  else hllc(g, wl, wr, out);
+}
+template <int SOLVER>
+__device__ __forceinline__ void riemann(const Gas& gas, const double* wl, const double* wr,
+                                        const CellGas<SOLVER>& cl, const CellGas<SOLVER>& cr,
+                                        FaceFlux<double>& out) {
+  if constexpr (SOLVER == SOLVER_HLLD) hlld(gas, wl, wr, cl, cr, out);
+  else if constexpr (SOLVER == SOLVER_HLLE) hlle(gas, wl, wr, cl, cr, out);
+  else hllc(gas, wl, wr, cl, cr, out);
+}
+template <int SOLVER>
+__device__ __forceinline__ void riemann(const Gas& gas, const double* wl, const double* wr,
+                                        FaceFlux<double>& out) {
+  CellGas<SOLVER> cl, cr;
+  cl.init(gas, wl[L_RHO], wl[L_E]);
+  cr.init(gas, wr[L_RHO], wr[L_E]);
+  riemann<SOLVER>(gas, wl, wr, cl, cr, out);
 }
 
 }  // namespace vlct

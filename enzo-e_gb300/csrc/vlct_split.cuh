@@ -30,11 +30,12 @@ namespace vlct {
 
 // Workspace arrays of one job, in the ghosted block's x and y extents and the
 // planes [za - 2, zb + 2): pressure, cell-centred E (3), face fluxes (3 x NF),
-// edge EMFs (3).  A face or edge value sits at the cell on its low side.
+// edge EMFs (3), the cells' gas quantities (CellGas: up to 4, NN stages).  A face
+// or edge value sits at the cell on its low side.
 template <bool MHD, bool DE> struct SplitLayout {
   static constexpr int NF = DE ? 9 : (MHD ? 7 : 5);
   static constexpr int P = 0, EC = 1, F = EC + (MHD ? 3 : 0), EMF = F + 3 * NF,
-                       N = EMF + (MHD ? 3 : 0);
+                       CG = EMF + (MHD ? 3 : 0), N = CG + 4;
   static_assert(N == split_arrays(MHD, DE), "workspace arrays");
 };
 
@@ -64,13 +65,14 @@ __device__ __forceinline__ SplitCtx<R> split_ctx(const StageBlock<R>& B, const S
   return C;
 }
 
-// ---- primitives: the pressure of every cell the fluxes read, and the
-// cell-centred E = -v x B (EnzoComputePressure.cpp:127-190,
-// EnzoBfieldMethodCT.cpp:267-292)
-template <class R, bool MHD, bool DE>
+// ---- primitives: the pressure of every cell the fluxes read, the gas
+// quantities that the faces of a cell share in an NN stage, and the cell-centred
+// E = -v x B (EnzoComputePressure.cpp:127-190, EnzoBfieldMethodCT.cpp:267-292)
+template <class R, int SOLVER, bool NN, bool DE>
 __global__ void __launch_bounds__(128)
 split_prim_kernel(const StageBlock<R>* __restrict__ blocks, const SplitJob* __restrict__ jobs,
                   R* __restrict__ ws, StageInfo info, PhysParams phys) {
+  constexpr bool MHD = SOLVER != SOLVER_HLLC;
   using L = SplitLayout<MHD, DE>;
   const SplitJob J = jobs[blockIdx.y];
   const StageBlock<R>& B = blocks[J.block];
@@ -98,9 +100,15 @@ split_prim_kernel(const StageBlock<R>* __restrict__ blocks, const SplitJob* __re
       bz = B.cur.c[F_BZ][c];
     }
     const R e = B.cur.c[DE ? F_EINT : F_ETOT][c];
-    C.ws[L::P * C.M + w] =
-        DE ? econ.gm1 * rho * e
-           : pressure_from_etot<R, MHD>(econ, rho, e, vx, vy, vz, bx, by, bz);
+    const R p = DE ? econ.gm1 * rho * e
+                   : pressure_from_etot<R, MHD>(econ, rho, e, vx, vy, vz, bx, by, bz);
+    C.ws[L::P * C.M + w] = p;
+    if (NN) {
+      CellGas<SOLVER> cg;
+      cg.init(Gas{phys.gamma, phys.gm1, phys.inv_gm1}, rho, p);
+#pragma unroll
+      for (int k = 0; k < CellGas<SOLVER>::N; k++) C.ws[(L::CG + k) * C.M + w] = cg.v[k];
+    }
     if (MHD && inr(x, S, C.m0 - S) && inr(y, S, C.m1 - S) && inr(z, S, C.m2 - S)) {
       C.ws[(L::EC + 0) * C.M + w] = (-vy * bz + vz * by);
       C.ws[(L::EC + 1) * C.M + w] = (-vz * bx + vx * bz);
@@ -180,7 +188,8 @@ split_flux_kernel(const StageBlock<R>* __restrict__ blocks, const SplitJob* __re
   const int e2 = d == 0 ? hi[2] - lo[2] : nch;
   const int n = e0 * e1 * e2;
   const size_t stride = d == 0 ? 1 : (d == 1 ? C.sy : C.sz);
-  const R g = R(phys.gamma), theta = R(phys.theta_limiter);
+  const R theta = R(phys.theta_limiter);
+  const Gas gas = {phys.gamma, phys.gm1, phys.inv_gm1};
   const R dfloor = R(phys.density_floor), pfloor = R(phys.pressure_floor);
   // face B along d: its own strides
   const R* bf = MHD ? B.cur.f[d] : nullptr;
@@ -250,7 +259,18 @@ split_flux_kernel(const StageBlock<R>* __restrict__ blocks, const SplitJob* __re
         wl[L_BI] = wr[L_BI] = *bface;
       }
       FaceFlux<R> F;
-      riemann<SOLVER, R>(g, wl, wr, F);
+      if (NN) {
+        CellGas<SOLVER> cl, cr;
+        const R* cg = C.ws + (size_t)L::CG * C.M + w;
+#pragma unroll
+        for (int k = 0; k < CellGas<SOLVER>::N; k++) {
+          cl.v[k] = cg[k * C.M];
+          cr.v[k] = cg[k * C.M + stride];
+        }
+        riemann<SOLVER>(gas, wl, wr, cl, cr, F);
+      } else {
+        riemann<SOLVER>(gas, wl, wr, F);
+      }
       R* dst = C.ws + (size_t)(L::F + d * L::NF) * C.M + w;
       dst[S_RHO * C.M] = F.f[L_RHO];
       dst[(S_MX + d) * C.M] = F.f[L_VI];

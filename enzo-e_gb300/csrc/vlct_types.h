@@ -63,9 +63,9 @@ struct SplitGroup {
   size_t cells, total;
 };
 // Workspace arrays of a split stage: pressure, cell-centred E, the face fluxes
-// of three directions, edge EMFs.
+// of three directions, edge EMFs, gas quantities.
 constexpr int split_arrays(bool mhd, bool de) {
-  return 1 + (mhd ? 6 : 0) + 3 * (de ? 9 : (mhd ? 7 : 5));
+  return 1 + (mhd ? 6 : 0) + 3 * (de ? 9 : (mhd ? 7 : 5)) + 4;
 }
 // A split stage's work as the host launches it (ngroups = 0: the fused kernel).
 struct SplitLaunch {
