@@ -125,15 +125,20 @@ long tile_columns(const StageKind& k, int lx, int ly, int tx, int ty) {
   return (long)parts_of(lx, tx) * parts_of(ly, ty);
 }
 
-// The tile and z-chunk that minimise a simple cost model: a chunk of L planes
-// costs L planes and about two and a half more (its prologue), a plane's time
-// a fixed part (latencies, barriers) and one that grows with the tile; chunks
-// run in waves of the CTAs the GPU holds at once.
+// The tile and z-chunk that minimise a simple cost model, measured on single
+// FP32 blocks of 8^3 - 96^3 at tiles of 3 x 3 - 20 x 8 and chunks of 1 - 24
+// planes: a chunk of L planes takes the time of L planes and two and a half more
+// (its prologue); a plane's time is a latency (3.4 us with NN, 3.9 with PLM
+// MHD), or, where the warps of an SM's CTAs fill its issue slots, grows with
+// them (two CTAs of 8 warps: 1.4 times).  CTAs run in waves of those the GPU
+// holds at once.  Best of the sweep / this model's choice / the first model's
+// (fixed part + tile): 16^3 HLLD, stage 1 16.3 / 17.4 / 31.7 us; 48^3, stage 2
+// 43 / 45 / 62 us; 96^3, stage 2 156 / 160 / 238 us.
 Decomp decompose(const StageKind& k, const Window& w, long nblocks) {
   Decomp d;
   if (w.len[0] <= 0 || w.len[1] <= 0 || w.len[2] <= 0) return d;
-  const long resident = (long)k.ctas() * sm_count();
-  const int full = k.threads();
+  const int nsm = sm_count();
+  const long resident = (long)k.ctas() * nsm;
   const int top = k.f64 ? TileLimits<double>::TMAX : TileLimits<float>::TMAX;
   double best = 1e300;
   for (int y = 1; y <= std::min(top, w.len[1]); y++)
@@ -142,11 +147,17 @@ Decomp decompose(const StageKind& k, const Window& w, long nblocks) {
       const int ay = parts_of(w.len[1], parts_of(w.len[1], y));
       if (ax != x || ay != y || !k.fits(ax, ay)) continue;
       const long cols = (long)parts_of(w.len[0], ax) * parts_of(w.len[1], ay) * nblocks;
-      const double plane = 0.35 + 0.65 * ((ax + 2) * (ay + 2)) / full;
-      for (int L : {0, 32, 24, 16, 12, 8, 6, 4, 3, 2}) {
+      const int warps = ((ax + 2) * (ay + 2) + 31) / 32;
+      // the time of a plane with n CTAs on an SM
+      auto plane = [&](long n) {
+        return std::max(1.0 + 0.02 * warps, 0.35 + 0.065 * (double)n * warps);
+      };
+      for (int L : {0, 32, 24, 16, 12, 10, 8, 7, 6, 5, 4, 3, 2, 1}) {
         if (L >= w.len[2]) continue;
         const int nz = L > 0 ? parts_of(w.len[2], L) : 1, tz = parts_of(w.len[2], nz);
-        const double cost = (double)((cols * nz + resident - 1) / resident) * plane * (tz + 2.5);
+        const long n = cols * nz, rest = n % resident;
+        const double cost = ((double)(n / resident) * plane(k.ctas()) +
+                             (rest ? plane((rest + nsm - 1) / nsm) : 0.0)) * (tz + 2.5);
         if (cost < best * 0.999) {  // on ties fewer chunks
           best = cost;
           d.tx = ax;
