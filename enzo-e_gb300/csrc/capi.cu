@@ -125,15 +125,18 @@ long tile_columns(const StageKind& k, int lx, int ly, int tx, int ty) {
   return (long)parts_of(lx, tx) * parts_of(ly, ty);
 }
 
-// The tile and z-chunk that minimise a simple cost model, measured on single
+// The tile and z-chunk that minimise a simple cost model, measured on 1 - 30
 // FP32 blocks of 8^3 - 96^3 at tiles of 3 x 3 - 20 x 8 and chunks of 1 - 24
 // planes: a chunk of L planes takes the time of L planes and two and a half more
-// (its prologue); a plane's time is a latency (3.4 us with NN, 3.9 with PLM
+// (its prologue); a plane's time is a latency (3.5 us with NN, 4.8 with PLM
 // MHD), or, where the warps of an SM's CTAs fill its issue slots, grows with
-// them (two CTAs of 8 warps: 1.4 times).  CTAs run in waves of those the GPU
-// holds at once.  Best of the sweep / this model's choice / the first model's
-// (fixed part + tile): 16^3 HLLD, stage 1 16.3 / 17.4 / 31.7 us; 48^3, stage 2
-// 43 / 45 / 62 us; 96^3, stage 2 156 / 160 / 238 us.
+// them.  There a CTA counts as the next multiple of four warps, one for each
+// scheduler: 6 warps take 6.6 us a plane, 8 take 7.0 (PLM, two CTAs).  CTAs run
+// in waves of those the GPU holds at once.
+// Measured stage times (us), the first model (a fixed part and one that grows
+// with the tile) / this one: one 16^3 block, HLLD, half dt 31.7 / 17.4; one 96^3,
+// HLLD, full dt 238 / 154; not everywhere better: one 48^3, HLLD, full dt 61.6 /
+// 64.2.
 Decomp decompose(const StageKind& k, const Window& w, long nblocks) {
   Decomp d;
   if (w.len[0] <= 0 || w.len[1] <= 0 || w.len[2] <= 0) return d;
@@ -147,10 +150,10 @@ Decomp decompose(const StageKind& k, const Window& w, long nblocks) {
       const int ay = parts_of(w.len[1], parts_of(w.len[1], y));
       if (ax != x || ay != y || !k.fits(ax, ay)) continue;
       const long cols = (long)parts_of(w.len[0], ax) * parts_of(w.len[1], ay) * nblocks;
-      const int warps = ((ax + 2) * (ay + 2) + 31) / 32;
+      const int warps = ((ax + 2) * (ay + 2) + 31) / 32, even = (warps + 3) / 4 * 4;
       // the time of a plane with n CTAs on an SM
       auto plane = [&](long n) {
-        return std::max(1.0 + 0.02 * warps, 0.35 + 0.065 * (double)n * warps);
+        return std::max(1.0 + 0.02 * warps, 0.35 + 0.065 * (double)n * even);
       };
       for (int L : {0, 32, 24, 16, 12, 10, 8, 7, 6, 5, 4, 3, 2, 1}) {
         if (L >= w.len[2]) continue;
@@ -633,23 +636,23 @@ cudaError_t launch_make_tiles(StageTile* out, const TileSplit& sp, cudaStream_t 
 }
 
 // Work decomposition of the stages of the per-block path: one block alone on
-// the GPU.
-struct PlainDecomp {
-  int tx[2] = {8, 8}, ty[2] = {8, 8};
-  int zchunk[2] = {0, 0};
-};
-PlainDecomp plain_decomp(const mhdvlct_handle* h, const int m[3], int dtype) {
-  PlainDecomp d;
+// the GPU.  Kept while extents and dtype repeat: the search takes tens of
+// microseconds of the host, as long as a small block's step.
+const PlainDecomp& plain_decomp(mhdvlct_handle* h, const int m[3], int dtype) {
+  if (h->dc_dtype == dtype && std::equal(m, m + 3, h->dc_m)) return h->dc;
   const StagePlan sp = stage_plan(h);
+  h->dc = PlainDecomp();
   for (int i = 0; i < sp.nstages; i++) {
     const Decomp c = decompose(stage_kind(h, dtype, i),
                                stage_window(m, sp.S[i], i + 1 == sp.nstages), 1);
     if (c.tx <= 0) continue;
-    d.tx[i] = c.tx;
-    d.ty[i] = c.ty;
-    d.zchunk[i] = c.zchunk;
+    h->dc.tx[i] = c.tx;
+    h->dc.ty[i] = c.ty;
+    h->dc.zchunk[i] = c.zchunk;
   }
-  return d;
+  h->dc_dtype = dtype;
+  std::copy(m, m + 3, h->dc_m);
+  return h->dc;
 }
 
 // Scratch of the plain path, carved from one allocation.
@@ -678,7 +681,7 @@ template <class R>
 int ensure_scratch(mhdvlct_handle* h, const int m[3], int dtype,
                    PlainScratch<R>& S, cudaStream_t st, int np = 0) {
   const StagePlan sp = stage_plan(h);
-  const PlainDecomp dc = plain_decomp(h, m, dtype);
+  const PlainDecomp& dc = plain_decomp(h, m, dtype);
   TileSplit ts[2] = {};
   long nt[2] = {0, 0};
   for (int i = 0; i < sp.nstages; i++) {
@@ -1124,12 +1127,20 @@ int block_step_noalloc_t(mhdvlct_handle* h, const MhdBlockView* b, double dt,
   const int m[3] = {b->n[0] + 2 * g, b->n[1] + 2 * g, b->n[2] + 2 * g};
   const StagePlan sp = stage_plan(h);
   const int np = b->npassive;
-  // the same work decomposition as mhdvlct_block_step
-  const PlainDecomp dc = plain_decomp(h, m, b->dtype);
+  // the same work decomposition as mhdvlct_block_step, or whole columns where
+  // its chunks are too many for the fixed tile list
+  const PlainDecomp& dc = plain_decomp(h, m, b->dtype);
   TileSplit ts[2] = {};
   long nt[2] = {0, 0};
   for (int i = 0; i < sp.nstages; i++) {
-    ts[i] = tile_split(m, sp.S[i], i + 1 == sp.nstages, dc.tx[i], dc.ty[i], dc.zchunk[i]);
+    const bool final = i + 1 == sp.nstages;
+    ts[i] = tile_split(m, sp.S[i], final, dc.tx[i], dc.ty[i], dc.zchunk[i]);
+    if (ntiles_of(ts[i]) > kNoAllocMaxTiles) {
+      const Window w = stage_window(m, sp.S[i], final);
+      int tx = 0, ty = 0;
+      fit_tile(stage_kind(h, b->dtype, i), w.len[0], w.len[1], tx, ty);
+      ts[i] = tile_split(m, sp.S[i], final, tx, ty, 0);
+    }
     nt[i] = ntiles_of(ts[i]);
     if (nt[i] > kNoAllocMaxTiles)
       return fail(h, MHD_ERR_INVALID,

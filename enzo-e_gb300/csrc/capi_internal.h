@@ -9,6 +9,14 @@
 #include "vlct_launch.h"
 #include "vlct_types.h"
 
+namespace mhdint {
+// Tiles and z-chunks of the per-block path's stages.
+struct PlainDecomp {
+  int tx[2] = {8, 8}, ty[2] = {8, 8};
+  int zchunk[2] = {0, 0};
+};
+}  // namespace mhdint
+
 struct mhdvlct_handle {
   MhdVlctParams params;
   int solver = 2;        // vlct::Solver
@@ -22,6 +30,10 @@ struct mhdvlct_handle {
   int cache_dtype = -1;
   int cache_m[3] = {0, 0, 0};
   int cache_np = 0;            // passive-scalar scratch fields in the cache
+  // the per-block path's decomposition of the last extents and dtype
+  mhdint::PlainDecomp dc;
+  int dc_dtype = -1;
+  int dc_m[3] = {0, 0, 0};
   void* scratch = nullptr;     // one device allocation
   size_t scratch_bytes = 0;
   // the split stages' jobs of that geometry (FP64): per stage, and the
