@@ -49,8 +49,17 @@ template <> struct SpeedBits<float> {
 __device__ __forceinline__ float speed_max(float a, float b) { return fmaxf(a, b); }
 __device__ __forceinline__ double speed_max(double a, double b) { return fmax_i(a, b); }
 
+//
+// FP32 is bound by the bytes in flight: with 4 cells a thread (120 registers, 2
+// CTAs on an SM) DRAM was 59% busy, as an SM's loads came in two bursts with
+// arithmetic between; with 2 cells and 64 registers 4 CTAs overlap (512 blocks of
+// 32^3, MHD 223 -> 194 us; 5 CTAs, which spill, 252; 3 CTAs 214).  FP64 is bound
+// by its pipe and keeps 4 cells (64 blocks of 32^3 366 us).
+template <class R> struct TimestepTune { static constexpr int U = 4, ctas = 1; };
+template <> struct TimestepTune<float> { static constexpr int U = 2, ctas = 4; };
+
 template <class R, bool MHD, bool DE>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, TimestepTune<R>::ctas)
 timestep_kernel(const AuxBlock<R>* __restrict__ blocks, int nblocks,
                 int chunks_per_block, PhysParams phys,
                 typename SpeedBits<R>::T* __restrict__ smax_out) {
@@ -81,7 +90,7 @@ timestep_kernel(const AuxBlock<R>* __restrict__ blocks, int nblocks,
   R* __restrict__ const f_p = B.pressure;
   // U cells per thread per pass, every load of the pass issued before the
   // arithmetic (the pass's stores would otherwise hold later loads back)
-  constexpr int U = 4;
+  constexpr int U = TimestepTune<R>::U;
   const size_t stride = (size_t)chunks_per_block * blockDim.x;
   for (size_t c0 = (size_t)chunk * blockDim.x + threadIdx.x; c0 < ncell; c0 += U * stride) {
     R rho[U], vx[U], vy[U], vz[U], bx[U], by[U], bz[U], et[U], ei[U];
