@@ -180,7 +180,7 @@ TileChoice choice_for(const mhdvlct_batch* b, const std::vector<int>& cls, const
   for (int s = 0; s < 2; s++) {
     const StageKind k = stage_kind(b->h, b->dtype, s);
     if (columns[s] >= 2L * k.ctas() * sm_count()) continue;
-    const Decomp d = decompose(k, stage_window(m, sp.S[s], s == 1), b->nblocks);
+    const Decomp d = decompose(k, stage_window(m, sp.S[s]), b->nblocks);
     c.tile_x[s] = d.tx;
     c.tile_y[s] = d.ty;
     c.zchunk[s] = d.zchunk;
@@ -201,7 +201,7 @@ std::map<std::vector<int>, TileChoice> choices(const mhdvlct_batch* b) {
   for (const auto& k : count)
     for (int s = 0; s < 2; s++) {
       const int m[3] = {k.first[0] + 2 * b->g, k.first[1] + 2 * b->g, k.first[2] + 2 * b->g};
-      const Window w = stage_window(m, sp.S[s], s == 1);
+      const Window w = stage_window(m, sp.S[s]);
       columns[s] += k.second * tile_columns(stage_kind(b->h, b->dtype, s), w.len[0], w.len[1], 0, 0);
     }
   std::map<std::vector<int>, TileChoice> out;
@@ -279,7 +279,7 @@ int build_descriptors(mhdvlct_batch* b, cudaStream_t st) {
     const TileChoice& c = choice.at(class_of(b, i));
     for (int s = 0; s < 2; s++) {
       std::vector<StageTile> t;
-      make_tiles(kind[s], i, O.m, sp.S[s], s == 1, c.tile_x[s], c.tile_y[s], c.zchunk[s], t);
+      make_tiles(kind[s], i, O.m, sp.S[s], c.tile_x[s], c.tile_y[s], c.zchunk[s], t);
       for (auto& x : t) {
         const double cost = (double)(x.xb - x.xa + 2) * (x.yb - x.ya + 2) *
                             (x.zb - x.za + 2);
@@ -1273,7 +1273,7 @@ int autotune_t(mhdvlct_batch* b, int reps, std::string& json, cudaStream_t st) {
       if (b->d_ws) cands.push_back(bestc);
       // the least-work tile, then each shape, as the fused kernel takes them
       const int m[3] = {cls[0] + 2 * b->g, cls[1] + 2 * b->g, cls[2] + 2 * b->g};
-      const Window w = stage_window(m, sp.S[s], s == 1);
+      const Window w = stage_window(m, sp.S[s]);
       std::vector<std::pair<int, int>> seen;
       shapes.insert(shapes.begin(), {0, 0});
       for (auto sh : shapes) {
@@ -1328,7 +1328,7 @@ int autotune_t(mhdvlct_batch* b, int reps, std::string& json, cudaStream_t st) {
     const int m[3] = {cls[0] + 2 * b->g, cls[1] + 2 * b->g, cls[2] + 2 * b->g};
     int shape[2][2];
     for (int k = 0; k < 2; k++) {
-      const Window w = stage_window(m, sp.S[k], k == 1);
+      const Window w = stage_window(m, sp.S[k]);
       shape[k][0] = bestc.tile_x[k];
       shape[k][1] = bestc.tile_y[k];
       fit_tile(stage_kind(b->h, b->dtype, k), w.len[0], w.len[1], shape[k][0], shape[k][1]);

@@ -75,9 +75,9 @@ StageKind stage_kind(const mhdvlct_handle* h, int dtype, int i) {
   return StageKind{dtype == MHD_DTYPE_F64, stage_plan(h).recon[i] == RECON_NN, h->mhd != 0};
 }
 
-Window stage_window(const int m[3], int S, bool final) {
+Window stage_window(const int m[3], int S) {
   Window w;
-  w.lo = final ? S : S + 1;
+  w.lo = S + 1;
   for (int a = 0; a < 3; a++) w.len[a] = m[a] - 2 * w.lo;
   return w;
 }
@@ -94,9 +94,12 @@ int sm_count() {
 }
 
 static int parts_of(int len, int t) { return (len + t - 1) / t; }
-// Warps a tile of tx x ty columns keeps busy, and about one more for its
-// barriers.
-static double tile_cost(int tx, int ty) { return ((tx + 2) * (ty + 2) + 31) / 32 + 1.0; }
+// What a plane of a tile of tx x ty columns costs on a full GPU, in warps: those
+// of its halo grid, and about six for the barriers and latencies that two CTAs
+// on an SM do not hide.  Measured a plane and tile (us): MHD PLM, 64^3 blocks 13
+// x 10 (6 warps) 97, 16 x 10 (7) 99, 16 x 11 (8) 107; hydro PLM 14 x 14 (8) 50, 22 x
+// 10 (9) 53, 22 x 11 (10) 60.
+static double tile_cost(int tx, int ty) { return ((tx + 2) * (ty + 2) + 31) / 32 + 6.0; }
 
 void fit_tile(const StageKind& k, int lx, int ly, int& tx, int& ty) {
   const int top = k.f64 ? TileLimits<double>::TMAX : TileLimits<float>::TMAX;
@@ -104,12 +107,14 @@ void fit_tile(const StageKind& k, int lx, int ly, int& tx, int& ty) {
   const int my = std::min(ly, ty > 0 ? std::min(ty, top) : top);
   double best = 1e300;
   int bx = 1, by = 1;
-  for (int y = 1; y <= my; y++)
-    for (int x = 1; x <= mx; x++) {
+  for (int x = 1; x <= mx; x++)
+    for (int y = 1; y <= my; y++) {
       const int ax = parts_of(lx, parts_of(lx, x)), ay = parts_of(ly, parts_of(ly, y));
       if (!k.fits(ax, ay)) continue;
       const double c = (double)parts_of(lx, ax) * parts_of(ly, ay) * tile_cost(ax, ay);
-      if (c <= best) {  // on ties the wider tile: longer rows to load
+      // on ties the wider tile, with longer rows to load: 512 hydro blocks of
+      // 32^3 16 x 11 1169 us, 11 x 16 1204; MHD 1309, 1431
+      if (c <= best) {
         best = c;
         bx = ax;
         by = ay;
@@ -172,9 +177,9 @@ Decomp decompose(const StageKind& k, const Window& w, long nblocks) {
   return d;
 }
 
-void make_tiles(const StageKind& k, int block, const int m[3], int S, bool final, int tile_x,
+void make_tiles(const StageKind& k, int block, const int m[3], int S, int tile_x,
                 int tile_y, int zchunk, std::vector<StageTile>& out) {
-  const Window w = stage_window(m, S, final);
+  const Window w = stage_window(m, S);
   if (w.len[0] <= 0 || w.len[1] <= 0 || w.len[2] <= 0) return;
   fit_tile(k, w.len[0], w.len[1], tile_x, tile_y);
   std::vector<std::pair<int, int>> xs, ys, zs;
@@ -611,12 +616,12 @@ __global__ void make_tiles_kernel(StageTile* out, TileSplit sp) {
 // The split of one stage's output window into tiles of at most tx x ty
 // columns and z-chunks of zchunk planes (0: whole window); ntiles() = 0 when
 // the window is empty.
-TileSplit tile_split(const int m[3], int S, bool final, int tx, int ty, int zchunk) {
+TileSplit tile_split(const int m[3], int S, int tx, int ty, int zchunk) {
   TileSplit sp{};
-  sp.lo = final ? S : S + 1;
+  sp.lo = S + 1;
   const int t[3] = {tx, ty, zchunk};
   for (int a = 0; a < 3; a++) {
-    sp.len[a] = (final ? m[a] - S : m[a] - S - 1) - sp.lo;
+    sp.len[a] = m[a] - S - 1 - sp.lo;
     int ta = t[a];
     if (sp.len[a] <= 0) {
       sp.np[0] = sp.np[1] = sp.np[2] = 0;
@@ -643,8 +648,7 @@ const PlainDecomp& plain_decomp(mhdvlct_handle* h, const int m[3], int dtype) {
   const StagePlan sp = stage_plan(h);
   h->dc = PlainDecomp();
   for (int i = 0; i < sp.nstages; i++) {
-    const Decomp c = decompose(stage_kind(h, dtype, i),
-                               stage_window(m, sp.S[i], i + 1 == sp.nstages), 1);
+    const Decomp c = decompose(stage_kind(h, dtype, i), stage_window(m, sp.S[i]), 1);
     if (c.tx <= 0) continue;
     h->dc.tx[i] = c.tx;
     h->dc.ty[i] = c.ty;
@@ -685,7 +689,7 @@ int ensure_scratch(mhdvlct_handle* h, const int m[3], int dtype,
   TileSplit ts[2] = {};
   long nt[2] = {0, 0};
   for (int i = 0; i < sp.nstages; i++) {
-    ts[i] = tile_split(m, sp.S[i], i + 1 == sp.nstages, dc.tx[i], dc.ty[i], dc.zchunk[i]);
+    ts[i] = tile_split(m, sp.S[i], dc.tx[i], dc.ty[i], dc.zchunk[i]);
     nt[i] = ntiles_of(ts[i]);
   }
   const size_t M = (size_t)m[0] * m[1] * m[2];
@@ -1133,13 +1137,12 @@ int block_step_noalloc_t(mhdvlct_handle* h, const MhdBlockView* b, double dt,
   TileSplit ts[2] = {};
   long nt[2] = {0, 0};
   for (int i = 0; i < sp.nstages; i++) {
-    const bool final = i + 1 == sp.nstages;
-    ts[i] = tile_split(m, sp.S[i], final, dc.tx[i], dc.ty[i], dc.zchunk[i]);
+    ts[i] = tile_split(m, sp.S[i], dc.tx[i], dc.ty[i], dc.zchunk[i]);
     if (ntiles_of(ts[i]) > kNoAllocMaxTiles) {
-      const Window w = stage_window(m, sp.S[i], final);
+      const Window w = stage_window(m, sp.S[i]);
       int tx = 0, ty = 0;
       fit_tile(stage_kind(h, b->dtype, i), w.len[0], w.len[1], tx, ty);
-      ts[i] = tile_split(m, sp.S[i], final, tx, ty, 0);
+      ts[i] = tile_split(m, sp.S[i], tx, ty, 0);
     }
     nt[i] = ntiles_of(ts[i]);
     if (nt[i] > kNoAllocMaxTiles)

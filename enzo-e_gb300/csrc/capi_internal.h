@@ -69,12 +69,12 @@ StagePlan stage_plan(const mhdvlct_handle* h);
 // The kind of stage i (vlct_launch.h) on fields of a dtype.
 vlct::StageKind stage_kind(const mhdvlct_handle* h, int dtype, int i);
 
-// Extents of a stage's output window.  m: ghosted extents of the block, S:
-// stale depth after reconstruction, final: last stage.
+// The cells that a stage updates, which its tiles cover.  m: ghosted extents of
+// the block, S: stale depth after reconstruction.
 struct Window {
   int lo, len[3];
 };
-Window stage_window(const int m[3], int S, bool final);
+Window stage_window(const int m[3], int S);
 
 // A work decomposition of a stage: tile extents and z-chunk length (0: the
 // whole window).
@@ -91,7 +91,7 @@ Decomp decompose(const vlct::StageKind& k, const Window& w, long nblocks);
 
 // Split the output window of a stage into tiles of at most tile_x x tile_y
 // columns (0: any) that the fused kernel holds.
-void make_tiles(const vlct::StageKind& k, int block, const int m[3], int S, bool final, int tile_x,
+void make_tiles(const vlct::StageKind& k, int block, const int m[3], int S, int tile_x,
                 int tile_y, int zchunk, std::vector<vlct::StageTile>& out);
 
 // The jobs of a split stage over blocks of ghosted extents m (3 per block),

@@ -108,6 +108,10 @@ cudaError_t stage_one(const StageBlock<R>* b, const StageTile* t, int nt,
         b, t, nt, info, phys, grid, st);
   else
     e = stage_fused<R, SOLVER, RECON, DE, EXTRA_NONE>(b, t, nt, info, phys, grid, st);
+  if (e == cudaSuccess && SOLVER != SOLVER_HLLC && info.final_stage && nt > 0) {
+    ring_bfield_kernel<R><<<nt, 128, 0, st>>>(b, t, info);
+    e = cudaGetLastError();
+  }
   // the passive scalars, on the same tiles, with the density fluxes the
   // stage kernel wrote
   if (e == cudaSuccess && info.npass > 0 && nt > 0) {

@@ -292,7 +292,7 @@ stage_kernel(const StageBlock<R>* __restrict__ blocks,
       T.HQ = tl.yb - tl.ya + 2;
       T.za = tl.za;
       T.zb = tl.zb;
-      T.olo = final_stage ? S : S + 1;
+      T.olo = S + 1;
       T.rowb = T.m0 * (int)sizeof(R);
       T.szb = (size_t)T.rowb * T.m1;
       T.fxzb = (size_t)(T.m0 + 1) * sizeof(R) * T.m1;
@@ -538,7 +538,7 @@ stage_kernel(const StageBlock<R>* __restrict__ blocks,
       // boundary fluxes for flux correction (EnzoMethodMHDVlct.cpp:250-330):
       // on the final stage, dt/dx times the flux through the block's active
       // boundary faces, each by the tile (and z-chunk) that owns the cell on
-      // its high side
+      // its high side, or the last cell along the axis
       auto store_face = [&](int d, int side, size_t at) {
         const FluxOut<R>* fo = reinterpret_cast<const FluxOut<R>*>(s_fo_raw);
         const R sc = T.dtdx[d];
@@ -586,7 +586,7 @@ stage_kernel(const StageBlock<R>* __restrict__ blocks,
           int x, y, i, j;
           place(x, y, i, j);
           const int side = x == gg - 1 ? 0 : (x == T.m0 - gg - 1 ? 1 : -1);
-          if (side >= 0 && i < T.HP - 2 && j >= 1 && j <= tl.yb - tl.ya && inr(y, gg, T.m1 - gg) &&
+          if (side >= 0 && (i < T.HP - 2 || on(XHI)) && j >= 1 && j <= tl.yb - tl.ya && inr(y, gg, T.m1 - gg) &&
               pl >= T.za && pl < zb && inr(pl, gg, T.m2 - gg))
             store_face(0, side, (size_t)(pl - gg) * (T.m1 - 2 * gg) + (y - gg));
         }
@@ -602,7 +602,7 @@ stage_kernel(const StageBlock<R>* __restrict__ blocks,
           int x, y, i, j;
           place(x, y, i, j);
           const int side = y == gg - 1 ? 0 : (y == T.m1 - gg - 1 ? 1 : -1);
-          if (side >= 0 && j < tl.yb - tl.ya && i >= 1 && i <= T.HP - 2 && inr(x, gg, T.m0 - gg) &&
+          if (side >= 0 && (j < tl.yb - tl.ya || on(YHI)) && i >= 1 && i <= T.HP - 2 && inr(x, gg, T.m0 - gg) &&
               pl >= T.za && pl < zb && inr(pl, gg, T.m2 - gg))
             store_face(1, side, (size_t)(pl - gg) * (T.m0 - 2 * gg) + (x - gg));
         }
@@ -628,7 +628,7 @@ stage_kernel(const StageBlock<R>* __restrict__ blocks,
         }
         if (EXTRA != EXTRA_NONE && store_fc && on(OUT)) {
           const int side = t == gg - 1 ? 0 : (t == T.m2 - gg - 1 ? 1 : -1);
-          if (side >= 0 && t >= T.za - 1 && t < zb - 1) {
+          if (side >= 0 && t >= T.za - 1 && (t < zb - 1 || t + 1 == T.m2 - T.olo)) {
             int x, y, i, j;
             place(x, y, i, j);
             if (inr(x, gg, T.m0 - gg) && inr(y, gg, T.m1 - gg))
@@ -901,6 +901,70 @@ stage_kernel(const StageBlock<R>* __restrict__ blocks,
     } else {
       it += gridDim.x;
     }
+  }
+}
+
+// On the final stage the reference also recomputes the cell-centred B of the one
+// layer of cells around the updated region, from faces of which the stage has
+// updated some (EnzoBfieldMethodCT.cpp:702-728).  The stage kernel's tiles cover
+// the updated region alone: as columns and planes of its march that layer made
+// a 32^3 block 34^3 zones, and 16^3 18^3.  This kernel, on the same tiles after
+// it, gives each tile the layer's cells next to it.  It moves nine values a cell
+// of the layer.
+template <class R>
+__global__ void __launch_bounds__(128)
+ring_bfield_kernel(const StageBlock<R>* __restrict__ blocks, const StageTile* __restrict__ tiles,
+                   StageInfo info) {
+  const StageTile tl = tiles[blockIdx.x];
+  const StageBlock<R>& B = blocks[tl.block];
+  const int S = info.S, m0 = B.m[0], m1 = B.m[1], m2 = B.m[2];
+  // how far the tile's box reaches into the layer on each side (0 or 1)
+  const int xl = tl.xa == S + 1, xh = tl.xb == m0 - S - 1;
+  const int yl = tl.ya == S + 1, yh = tl.yb == m1 - S - 1;
+  const int zl = tl.za == S + 1, zh = tl.zb == m2 - S - 1;
+  const int nx = tl.xb - tl.xa, ny = tl.yb - tl.ya, nz = tl.zb - tl.za;
+  const int ex = nx + xl + xh, ey = ny + yl + yh;
+  const int cz = (zl + zh) * ex * ey, cy = nz * (yl + yh) * ex, cx = nz * ny * (xl + xh);
+  const R *ox = B.out.f[0], *oy = B.out.f[1], *oz = B.out.f[2];
+  const R *bx = B.base.f[0], *by = B.base.f[1], *bz = B.base.f[2];
+  R *cbx = B.out.c[F_BX], *cby = B.out.c[F_BY], *cbz = B.out.c[F_BZ];
+  for (int q = threadIdx.x; q < cz + cy + cx; q += blockDim.x) {
+    int x, y, t;
+    if (q < cz) {
+      const int r = q / ex;
+      x = tl.xa - xl + (q - r * ex);
+      const int k = r / ey;
+      y = tl.ya - yl + (r - k * ey);
+      t = zl && k == 0 ? tl.za - 1 : tl.zb;
+    } else if (q < cz + cy) {
+      const int p = q - cz, r = p / ex;
+      x = tl.xa - xl + (p - r * ex);
+      const int k = r / nz;
+      t = tl.za + (r - k * nz);
+      y = yl && k == 0 ? tl.ya - 1 : tl.yb;
+    } else {
+      const int p = q - cz - cy, r = p / ny;
+      y = tl.ya + (p - r * ny);
+      const int k = r / nz;
+      t = tl.za + (r - k * nz);
+      x = xl && k == 0 ? tl.xa - 1 : tl.xb;
+    }
+    const bool ux = inr(x, S + 1, m0 - S - 1), uy = inr(y, S + 1, m1 - S - 1),
+               uz = inr(t, S + 1, m2 - S - 1);
+    const size_t c = ((size_t)t * m1 + y) * m0 + x;
+    const size_t fx = ((size_t)t * m1 + y) * (m0 + 1) + x;
+    const size_t fy = ((size_t)t * (m1 + 1) + y) * m0 + x;
+    const size_t szz = (size_t)m0 * m1;
+    R v[6];
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      v[k] = (uy && uz && inr(x + k, S + 1, m0 - S) ? ox : bx)[fx + k];
+      v[2 + k] = (ux && uz && inr(y + k, S + 1, m1 - S) ? oy : by)[fy + (size_t)k * m0];
+      v[4 + k] = (ux && uy && inr(t + k, S + 1, m2 - S) ? oz : bz)[c + (size_t)k * szz];
+    }
+    cbx[c] = R(0.5) * (v[0] + v[1]);
+    cby[c] = R(0.5) * (v[2] + v[3]);
+    cbz[c] = R(0.5) * (v[4] + v[5]);
   }
 }
 
