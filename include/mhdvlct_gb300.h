@@ -375,8 +375,9 @@ int mhdvlct_batch_run(mhdvlct_batch* b, int ncycles, int dt_mode,
 /* Work decomposition: tile extent used per block size class (0 = auto). */
 int mhdvlct_batch_set_tile(mhdvlct_batch* b, int tile_x, int tile_y);
 /* One stage's work decomposition for every block (stage 0: half dt, 1: full
- * dt): tile extents, z-chunk length (0 = whole block) and CTA size (256, or
- * 512 where the stage allows it; 0 = 256), e.g. to pin a tuned choice. */
+ * dt): tile extents, z-chunk length (0 = whole block), e.g. to pin a tuned
+ * choice.  A tile is cut down to what the stage's CTA holds; that CTA's size
+ * follows from the stage, and threads (0, 256 or 512) changes nothing. */
 int mhdvlct_batch_set_stage_tile(mhdvlct_batch* b, int stage, int tile_x,
                                  int tile_y, int zchunk, int threads);
 /* The autotuner: for every block-size class, time candidate (tile, z-chunk)
