@@ -219,8 +219,16 @@ int build_descriptors(mhdvlct_batch* b, cudaStream_t st) {
   std::vector<AuxBlock<R>> aux[2];
   std::vector<StageTile> tiles[2];
   std::vector<std::pair<double, StageTile>> order[2];
-  const std::map<std::vector<int>, TileChoice> choice = choices(b);
-  const StageKind kind[2] = {stage_kind(b->h, b->dtype, 0), stage_kind(b->h, b->dtype, 1)};
+  // the tiles that the kernels hold, found once for each block size
+  std::map<std::vector<int>, TileChoice> choice = choices(b);
+  for (auto& k : choice)
+    for (int s = 0; s < 2; s++) {
+      const int m[3] = {k.first[0] + 2 * b->g, k.first[1] + 2 * b->g, k.first[2] + 2 * b->g};
+      const Window w = stage_window(m, sp.S[s]);
+      if (w.len[0] > 0 && w.len[1] > 0)
+        fit_tile(stage_kind(b->h, b->dtype, s), w.len[0], w.len[1], k.second.tile_x[s],
+                 k.second.tile_y[s]);
+    }
   for (int i = 0; i < b->nblocks; i++) {
     const auto& O = b->off[i];
     FieldSet<R> ext, tmp;
@@ -279,7 +287,7 @@ int build_descriptors(mhdvlct_batch* b, cudaStream_t st) {
     const TileChoice& c = choice.at(class_of(b, i));
     for (int s = 0; s < 2; s++) {
       std::vector<StageTile> t;
-      make_tiles(kind[s], i, O.m, sp.S[s], c.tile_x[s], c.tile_y[s], c.zchunk[s], t);
+      make_tiles(i, O.m, sp.S[s], c.tile_x[s], c.tile_y[s], c.zchunk[s], t);
       for (auto& x : t) {
         const double cost = (double)(x.xb - x.xa + 2) * (x.yb - x.ya + 2) *
                             (x.zb - x.za + 2);

@@ -177,11 +177,10 @@ Decomp decompose(const StageKind& k, const Window& w, long nblocks) {
   return d;
 }
 
-void make_tiles(const StageKind& k, int block, const int m[3], int S, int tile_x,
-                int tile_y, int zchunk, std::vector<StageTile>& out) {
+void make_tiles(int block, const int m[3], int S, int tile_x, int tile_y, int zchunk,
+                std::vector<StageTile>& out) {
   const Window w = stage_window(m, S);
   if (w.len[0] <= 0 || w.len[1] <= 0 || w.len[2] <= 0) return;
-  fit_tile(k, w.len[0], w.len[1], tile_x, tile_y);
   std::vector<std::pair<int, int>> xs, ys, zs;
   split(w.lo, w.lo + w.len[0], tile_x, xs);
   split(w.lo, w.lo + w.len[1], tile_y, ys);

@@ -89,10 +89,10 @@ long tile_columns(const vlct::StageKind& k, int lx, int ly, int tx, int ty);
 // Tile and z-chunk for `nblocks` windows alone on the GPU.
 Decomp decompose(const vlct::StageKind& k, const Window& w, long nblocks);
 
-// Split the output window of a stage into tiles of at most tile_x x tile_y
-// columns (0: any) that the fused kernel holds.
-void make_tiles(const vlct::StageKind& k, int block, const int m[3], int S, int tile_x,
-                int tile_y, int zchunk, std::vector<vlct::StageTile>& out);
+// Split a stage's window into tiles of at most tile_x x tile_y columns (as
+// fit_tile gives them).
+void make_tiles(int block, const int m[3], int S, int tile_x, int tile_y, int zchunk,
+                std::vector<vlct::StageTile>& out);
 
 // The jobs of a split stage over blocks of ghosted extents m (3 per block),
 // blocks `ids` of them (all when empty), in groups whose workspace is bounded
