@@ -328,7 +328,7 @@ int build_descriptors(mhdvlct_batch* b, cudaStream_t st) {
       return rc;
   // the split stages depend on the blocks' extents alone: planned once
   std::vector<SplitJob> jobs[2];
-  if (sizeof(R) == 8 && !b->d_jobs[0]) {
+  if (sizeof(R) == 8 && b->h->use_split && !b->d_jobs[0]) {
     std::vector<int> m;
     for (const auto& o : b->off) m.insert(m.end(), o.m, o.m + 3);
     b->ws_elems = 0;

@@ -479,6 +479,13 @@ extern "C" int mhdvlct_create(const MhdVlctParams* p, mhdvlct_handle** out) {
   return MHD_OK;
 }
 
+extern "C" int mhdvlct_internal_use_split(mhdvlct_handle* h, int on) {
+  if (!h) return MHD_ERR_INVALID;
+  h->use_split = on != 0;
+  h->cache_dtype = -1;  // the next step lays its scratch out anew
+  return MHD_OK;
+}
+
 extern "C" int mhdvlct_destroy(mhdvlct_handle* h) {
   if (!h) return MHD_ERR_INVALID;
   if (h->scratch) cudaFree(h->scratch);
@@ -718,7 +725,7 @@ int ensure_scratch(mhdvlct_handle* h, const int m[3], int dtype,
     for (int i = 0; i < 2; i++) {
       h->sp_jobs[i].clear();
       h->sp_groups[i].clear();
-      if (sizeof(R) == 8 && i < sp.nstages)
+      if (sizeof(R) == 8 && h->use_split && i < sp.nstages)
         split_plan({m[0], m[1], m[2]}, {}, sp.S[i], i + 1 == sp.nstages, h->mhd != 0, h->de != 0,
                    h->sp_jobs[i], h->sp_groups[i], h->sp_ws);
     }

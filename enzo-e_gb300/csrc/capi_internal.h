@@ -42,12 +42,18 @@ struct mhdvlct_handle {
   std::vector<vlct::SplitGroup> sp_groups[2];
   size_t sp_ws = 0;
   bool split = false;
+  bool use_split = true;       // false: the fused kernels, as without room (tests)
   // mesh-refresh tables (pointer table, regions, chunks), reused across calls
   void* rf_dev = nullptr;
   size_t rf_bytes = 0;
   cudaEvent_t rf_done = nullptr;  // recorded after the last refresh launch
   std::vector<char> rf_host;
 };
+
+// Whether FP64 steps on this handle, and batches created on it from now on, run
+// the split stages where their workspace can be had (the default) or the fused
+// kernels, which otherwise run only where it cannot.  For tests.
+extern "C" int mhdvlct_internal_use_split(mhdvlct_handle* h, int on);
 
 namespace mhdint {
 
