@@ -180,7 +180,7 @@ TileChoice choice_for(const mhdvlct_batch* b, const std::vector<int>& cls, const
   for (int s = 0; s < 2; s++) {
     const StageKind k = stage_kind(b->h, b->dtype, s);
     if (columns[s] >= 2L * k.ctas() * sm_count()) continue;
-    const Decomp d = decompose(k, stage_window(m, sp.S[s]), b->nblocks);
+    const Decomp d = decompose(k, stage_window(m, sp.S[s]), b->nblocks, sm_count());
     c.tile_x[s] = d.tx;
     c.tile_y[s] = d.ty;
     c.zchunk[s] = d.zchunk;

@@ -94,12 +94,15 @@ int sm_count() {
 }
 
 static int parts_of(int len, int t) { return (len + t - 1) / t; }
+static int tile_warps(int tx, int ty) { return ((tx + 2) * (ty + 2) + 31) / 32; }
 // What a plane of a tile of tx x ty columns costs on a full GPU, in warps: those
-// of its halo grid, and about six for the barriers and latencies that two CTAs
-// on an SM do not hide.  Measured a plane and tile (us): MHD PLM, 64^3 blocks 13
-// x 10 (6 warps) 97, 16 x 10 (7) 99, 16 x 11 (8) 107; hydro PLM 14 x 14 (8) 50, 22 x
-// 10 (9) 53, 22 x 11 (10) 60.
-static double tile_cost(int tx, int ty) { return ((tx + 2) * (ty + 2) + 31) / 32 + 6.0; }
+// of its halo grid, and a fixed part.  FP32: about six, for the barriers and
+// latencies that two CTAs on an SM do not hide.  Measured a plane and tile (us):
+// MHD PLM, 64^3 blocks 13 x 10 (6 warps) 97, 16 x 10 (7) 99, 16 x 11 (8) 107; hydro
+// PLM 14 x 14 (8) 50, 22 x 10 (9) 53, 22 x 11 (10) 60.  FP64: see decompose.
+static double tile_cost(const StageKind& k, int tx, int ty) {
+  return tile_warps(tx, ty) + (k.f64 ? (k.nn ? 1.2 : 2.6) : 6.0);
+}
 
 void fit_tile(const StageKind& k, int lx, int ly, int& tx, int& ty) {
   const int top = k.f64 ? TileLimits<double>::TMAX : TileLimits<float>::TMAX;
@@ -111,7 +114,7 @@ void fit_tile(const StageKind& k, int lx, int ly, int& tx, int& ty) {
     for (int y = 1; y <= my; y++) {
       const int ax = parts_of(lx, parts_of(lx, x)), ay = parts_of(ly, parts_of(ly, y));
       if (!k.fits(ax, ay)) continue;
-      const double c = (double)parts_of(lx, ax) * parts_of(ly, ay) * tile_cost(ax, ay);
+      const double c = (double)parts_of(lx, ax) * parts_of(ly, ay) * tile_cost(k, ax, ay);
       // on ties the wider tile, with longer rows to load: 512 hydro blocks of
       // 32^3 16 x 11 1169 us, 11 x 16 1204; MHD 1309, 1431
       if (c <= best) {
@@ -130,24 +133,31 @@ long tile_columns(const StageKind& k, int lx, int ly, int tx, int ty) {
   return (long)parts_of(lx, tx) * parts_of(ly, ty);
 }
 
-// The tile and z-chunk that minimise a simple cost model, measured on 1 - 30
-// FP32 blocks of 8^3 - 96^3 at tiles of 3 x 3 - 20 x 8 and chunks of 1 - 24
-// planes: a chunk of L planes takes the time of L planes and two and a half more
-// (its prologue); a plane's time is a latency (3.5 us with NN, 4.8 with PLM
-// MHD), or, where the warps of an SM's CTAs fill its issue slots, grows with
-// them.  There a CTA counts as the next multiple of four warps, one for each
-// scheduler: 6 warps take 6.6 us a plane, 8 take 7.0 (PLM, two CTAs).  CTAs run
-// in waves of those the GPU holds at once.
-// Measured stage times (us), the first model (a fixed part and one that grows
-// with the tile) / this one: one 16^3 block, HLLD, half dt 31.7 / 17.4; one 96^3,
-// HLLD, full dt 238 / 154; not everywhere better: one 48^3, HLLD, full dt 61.6 /
-// 64.2.
-Decomp decompose(const StageKind& k, const Window& w, long nblocks) {
+// The tile and z-chunk that minimise a simple cost model: a chunk of L planes
+// takes the time of L planes and a few more (its prologue), and CTAs run in waves
+// of those the GPU holds at once.
+//
+// FP32, measured on 1 - 30 blocks of 8^3 - 96^3 at tiles of 3 x 3 - 20 x 8 and
+// chunks of 1 - 24 planes: two and a half planes more; a plane's time is a latency
+// (3.5 us with NN, 4.8 with PLM MHD), or, where the warps of an SM's CTAs fill its
+// issue slots, grows with them.  There a CTA counts as the next multiple of four
+// warps, one for each scheduler: 6 warps take 6.6 us a plane, 8 take 7.0 (PLM, two
+// CTAs).
+//
+// FP64 (the fused kernel; one CTA on an SM), measured on 1 - 12 blocks of 8^3 - 64^3
+// at tiles of 2 x 2 - 16 x 14 and chunks of 1 - 36 planes: 1.6 planes more; the FP64
+// pipe takes 9.1 - 9.9 us a warp and plane (MHD; hydro 5.3), beside a fixed part of
+// 1.2 (NN) or 2.6 (PLM) warps, and at least 4.8 or 6.4 warps' time.  That fits
+// 10 thousand times to 2 - 4%.  The FP32 model, which knows no such slope, took
+// tiles and chunks that execute up to 1.3 times the warps and planes: through the
+// no-allocation step, HLLD with PLM, 24^3 475 us, 28^3 588; with this one 418 and
+// 531; HLLE with NN, 24^3 504 and 407.
+Decomp decompose(const StageKind& k, const Window& w, long nblocks, int nsm) {
   Decomp d;
   if (w.len[0] <= 0 || w.len[1] <= 0 || w.len[2] <= 0) return d;
-  const int nsm = sm_count();
   const long resident = (long)k.ctas() * nsm;
   const int top = k.f64 ? TileLimits<double>::TMAX : TileLimits<float>::TMAX;
+  const double prologue = k.f64 ? 1.6 : 2.5;
   double best = 1e300;
   for (int y = 1; y <= std::min(top, w.len[1]); y++)
     for (int x = 1; x <= std::min(top, w.len[0]); x++) {
@@ -155,17 +165,18 @@ Decomp decompose(const StageKind& k, const Window& w, long nblocks) {
       const int ay = parts_of(w.len[1], parts_of(w.len[1], y));
       if (ax != x || ay != y || !k.fits(ax, ay)) continue;
       const long cols = (long)parts_of(w.len[0], ax) * parts_of(w.len[1], ay) * nblocks;
-      const int warps = ((ax + 2) * (ay + 2) + 31) / 32, even = (warps + 3) / 4 * 4;
+      const int warps = tile_warps(ax, ay), even = (warps + 3) / 4 * 4;
       // the time of a plane with n CTAs on an SM
       auto plane = [&](long n) {
-        return std::max(1.0 + 0.02 * warps, 0.35 + 0.065 * (double)n * even);
+        return k.f64 ? std::max(k.nn ? 4.8 : 6.4, tile_cost(k, ax, ay))
+                     : std::max(1.0 + 0.02 * warps, 0.35 + 0.065 * (double)n * even);
       };
       for (int L : {0, 32, 24, 16, 12, 10, 8, 7, 6, 5, 4, 3, 2, 1}) {
         if (L >= w.len[2]) continue;
         const int nz = L > 0 ? parts_of(w.len[2], L) : 1, tz = parts_of(w.len[2], nz);
         const long n = cols * nz, rest = n % resident;
         const double cost = ((double)(n / resident) * plane(k.ctas()) +
-                             (rest ? plane((rest + nsm - 1) / nsm) : 0.0)) * (tz + 2.5);
+                             (rest ? plane((rest + nsm - 1) / nsm) : 0.0)) * (tz + prologue);
         if (cost < best * 0.999) {  // on ties fewer chunks
           best = cost;
           d.tx = ax;
@@ -654,7 +665,7 @@ const PlainDecomp& plain_decomp(mhdvlct_handle* h, const int m[3], int dtype) {
   const StagePlan sp = stage_plan(h);
   h->dc = PlainDecomp();
   for (int i = 0; i < sp.nstages; i++) {
-    const Decomp c = decompose(stage_kind(h, dtype, i), stage_window(m, sp.S[i]), 1);
+    const Decomp c = decompose(stage_kind(h, dtype, i), stage_window(m, sp.S[i]), 1, sm_count());
     if (c.tx <= 0) continue;
     h->dc.tx[i] = c.tx;
     h->dc.ty[i] = c.ty;

@@ -92,8 +92,8 @@ struct Decomp {
 void fit_tile(const vlct::StageKind& k, int lx, int ly, int& tx, int& ty);
 // Columns that fit_tile cuts an lx x ly window into.
 long tile_columns(const vlct::StageKind& k, int lx, int ly, int tx, int ty);
-// Tile and z-chunk for `nblocks` windows alone on the GPU.
-Decomp decompose(const vlct::StageKind& k, const Window& w, long nblocks);
+// Tile and z-chunk for `nblocks` windows alone on a GPU of nsm SMs.
+Decomp decompose(const vlct::StageKind& k, const Window& w, long nblocks, int nsm);
 
 // Split a stage's window into tiles of at most tile_x x tile_y columns (as
 // fit_tile gives them).
