@@ -101,7 +101,7 @@ static int tile_warps(int tx, int ty) { return ((tx + 2) * (ty + 2) + 31) / 32; 
 // MHD PLM, 64^3 blocks 13 x 10 (6 warps) 97, 16 x 10 (7) 99, 16 x 11 (8) 107; hydro
 // PLM 14 x 14 (8) 50, 22 x 10 (9) 53, 22 x 11 (10) 60.  FP64: see decompose.
 static double tile_cost(const StageKind& k, int tx, int ty) {
-  return tile_warps(tx, ty) + (k.f64 ? (k.nn ? 1.2 : 2.6) : 6.0);
+  return tile_warps(tx, ty) + (k.f64 ? (k.nn ? 1.6 : 2.6) : 6.0);
 }
 
 void fit_tile(const StageKind& k, int lx, int ly, int& tx, int& ty) {
@@ -146,9 +146,9 @@ long tile_columns(const StageKind& k, int lx, int ly, int tx, int ty) {
 //
 // FP64 (the fused kernel; one CTA on an SM), measured on 1 - 12 blocks of 8^3 - 64^3
 // at tiles of 2 x 2 - 16 x 14 and chunks of 1 - 36 planes: 1.6 planes more; the FP64
-// pipe takes 9.1 - 9.9 us a warp and plane (MHD; hydro 5.3), beside a fixed part of
-// 1.2 (NN) or 2.6 (PLM) warps, and at least 4.8 or 6.4 warps' time.  That fits
-// 10 thousand times to 2 - 4%.  The FP32 model, which knows no such slope, took
+// pipe takes 8.0 - 8.6 us a warp and plane with NN, 9.7 with PLM (hydro 3.4, 5.4),
+// beside a fixed part of 1.6 or 2.6 warps, and at least 5.2 or 6.4 warps' time.
+// That fits 8 thousand times to 2 - 5%.  The FP32 model, which knows no such slope, took
 // tiles and chunks that execute up to 1.3 times the warps and planes: through the
 // no-allocation step, HLLD with PLM, 24^3 475 us, 28^3 588; with this one 418 and
 // 531; HLLE with NN, 24^3 504 and 407.
@@ -168,7 +168,7 @@ Decomp decompose(const StageKind& k, const Window& w, long nblocks, int nsm) {
       const int warps = tile_warps(ax, ay), even = (warps + 3) / 4 * 4;
       // the time of a plane with n CTAs on an SM
       auto plane = [&](long n) {
-        return k.f64 ? std::max(k.nn ? 4.8 : 6.4, tile_cost(k, ax, ay))
+        return k.f64 ? std::max(k.nn ? 5.2 : 6.4, tile_cost(k, ax, ay))
                      : std::max(1.0 + 0.02 * warps, 0.35 + 0.065 * (double)n * even);
       };
       for (int L : {0, 32, 24, 16, 12, 10, 8, 7, 6, 5, 4, 3, 2, 1}) {

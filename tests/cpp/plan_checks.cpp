@@ -21,7 +21,7 @@ static double f64_time(const vlct::StageKind& k, const Window& w, int tx, int ty
   const int ax = up(w.len[0], up(w.len[0], tx)), ay = up(w.len[1], up(w.len[1], ty));
   const double n = (double)up(w.len[0], ax) * up(w.len[1], ay) * nz;
   const double warps = up((ax + 2) * (ay + 2), 32);
-  const double plane = std::max(k.nn ? 4.8 : 6.4, warps + (k.nn ? 1.2 : 2.6));
+  const double plane = std::max(k.nn ? 5.2 : 6.4, warps + (k.nn ? 1.6 : 2.6));
   return std::ceil(n / kSms) * (up(w.len[2], nz) + 1.6) * plane;
 }
 
