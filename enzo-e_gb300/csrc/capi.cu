@@ -95,6 +95,13 @@ int sm_count() {
 
 static int parts_of(int len, int t) { return (len + t - 1) / t; }
 static int tile_warps(int tx, int ty) { return ((tx + 2) * (ty + 2) + 31) / 32; }
+// The lengths of at most `top` into which near-equal splits cut len, ascending.
+static std::vector<int> part_lengths(int len, int top) {
+  std::vector<int> v;
+  for (int t = 1; t <= std::min(len, top); t++)
+    if (parts_of(len, parts_of(len, t)) == t) v.push_back(t);
+  return v;
+}
 // What a plane of a tile of tx x ty columns costs on a full GPU, in warps: those
 // of its halo grid, and a fixed part.  FP32: about six, for the barriers and
 // latencies that two CTAs on an SM do not hide.  Measured a plane and tile (us):
@@ -106,21 +113,20 @@ static double tile_cost(const StageKind& k, int tx, int ty) {
 
 void fit_tile(const StageKind& k, int lx, int ly, int& tx, int& ty) {
   const int top = k.f64 ? TileLimits<double>::TMAX : TileLimits<float>::TMAX;
-  const int mx = std::min(lx, tx > 0 ? std::min(tx, top) : top);
-  const int my = std::min(ly, ty > 0 ? std::min(ty, top) : top);
+  const std::vector<int> xs = part_lengths(lx, tx > 0 ? std::min(tx, top) : top);
+  const std::vector<int> ys = part_lengths(ly, ty > 0 ? std::min(ty, top) : top);
   double best = 1e300;
   int bx = 1, by = 1;
-  for (int x = 1; x <= mx; x++)
-    for (int y = 1; y <= my; y++) {
-      const int ax = parts_of(lx, parts_of(lx, x)), ay = parts_of(ly, parts_of(ly, y));
-      if (!k.fits(ax, ay)) continue;
-      const double c = (double)parts_of(lx, ax) * parts_of(ly, ay) * tile_cost(k, ax, ay);
+  for (int x : xs)
+    for (int y : ys) {
+      if (!k.fits(x, y)) continue;
+      const double c = (double)parts_of(lx, x) * parts_of(ly, y) * tile_cost(k, x, y);
       // on ties the wider tile, with longer rows to load: 512 hydro blocks of
       // 32^3 16 x 11 1169 us, 11 x 16 1204; MHD 1309, 1431
       if (c <= best) {
         best = c;
-        bx = ax;
-        by = ay;
+        bx = x;
+        by = y;
       }
     }
   tx = bx;
@@ -152,36 +158,54 @@ long tile_columns(const StageKind& k, int lx, int ly, int tx, int ty) {
 // tiles and chunks that execute up to 1.3 times the warps and planes: through the
 // no-allocation step, HLLD with PLM, 24^3 475 us, 28^3 588; with this one 418 and
 // 531; HLLE with NN, 24^3 504 and 407.
+//
+// What cannot beat the best so far is passed over: the two searches of a block take
+// 4.6 us of an x86 core at 32^3 and 7.5 at 96^3 (FP32 HLLD), without that 44 and 89.
 Decomp decompose(const StageKind& k, const Window& w, long nblocks, int nsm) {
   Decomp d;
   if (w.len[0] <= 0 || w.len[1] <= 0 || w.len[2] <= 0) return d;
-  const long resident = (long)k.ctas() * nsm;
+  const int ctas = k.ctas();
+  const long resident = (long)ctas * nsm;
   const int top = k.f64 ? TileLimits<double>::TMAX : TileLimits<float>::TMAX;
   const double prologue = k.f64 ? 1.6 : 2.5;
+  // the distinct cuts of the planes: chunk length asked for, chunks, planes of one
+  struct Cut {
+    int L, n, planes;
+  };
+  Cut cuts[14];
+  int ncuts = 0;
+  for (int L : {0, 32, 24, 16, 12, 10, 8, 7, 6, 5, 4, 3, 2, 1}) {
+    if (L >= w.len[2]) continue;
+    const int n = L > 0 ? parts_of(w.len[2], L) : 1;
+    if (ncuts > 0 && cuts[ncuts - 1].n == n) continue;
+    cuts[ncuts++] = Cut{L, n, parts_of(w.len[2], n)};
+  }
+  const std::vector<int> xs = part_lengths(w.len[0], top), ys = part_lengths(w.len[1], top);
   double best = 1e300;
-  for (int y = 1; y <= std::min(top, w.len[1]); y++)
-    for (int x = 1; x <= std::min(top, w.len[0]); x++) {
-      const int ax = parts_of(w.len[0], parts_of(w.len[0], x));
-      const int ay = parts_of(w.len[1], parts_of(w.len[1], y));
-      if (ax != x || ay != y || !k.fits(ax, ay)) continue;
-      const long cols = (long)parts_of(w.len[0], ax) * parts_of(w.len[1], ay) * nblocks;
-      const int warps = tile_warps(ax, ay), even = (warps + 3) / 4 * 4;
+  for (int y : ys)
+    for (int x : xs) {
+      if (!k.fits(x, y)) continue;
+      const long cols = (long)parts_of(w.len[0], x) * parts_of(w.len[1], y) * nblocks;
+      const int warps = tile_warps(x, y), even = (warps + 3) / 4 * 4;
       // the time of a plane with n CTAs on an SM
       auto plane = [&](long n) {
-        return k.f64 ? std::max(k.nn ? 5.2 : 6.4, tile_cost(k, ax, ay))
+        return k.f64 ? std::max(k.nn ? 5.2 : 6.4, tile_cost(k, x, y))
                      : std::max(1.0 + 0.02 * warps, 0.35 + 0.065 * (double)n * even);
       };
-      for (int L : {0, 32, 24, 16, 12, 10, 8, 7, 6, 5, 4, 3, 2, 1}) {
-        if (L >= w.len[2]) continue;
-        const int nz = L > 0 ? parts_of(w.len[2], L) : 1, tz = parts_of(w.len[2], nz);
-        const long n = cols * nz, rest = n % resident;
-        const double cost = ((double)(n / resident) * plane(k.ctas()) +
-                             (rest ? plane((rest + nsm - 1) / nsm) : 0.0)) * (tz + prologue);
+      // no cut takes less than one CTA's planes, nor than the GPU's throughput
+      const double one = plane(1), full = plane(ctas), each = full * (double)cols / (double)resident;
+      if (each * w.len[2] >= best * 0.999) continue;
+      for (int i = 0; i < ncuts; i++) {
+        const double len = cuts[i].planes + prologue;
+        if (one * len >= best * 0.999 || each * cuts[i].n * len >= best * 0.999) continue;
+        const long n = cols * cuts[i].n, waves = n / resident, rest = n - waves * resident;
+        const double cost =
+            ((double)waves * full + (rest ? plane((rest + nsm - 1) / nsm) : 0.0)) * len;
         if (cost < best * 0.999) {  // on ties fewer chunks
           best = cost;
-          d.tx = ax;
-          d.ty = ay;
-          d.zchunk = L;
+          d.tx = x;
+          d.ty = y;
+          d.zchunk = cuts[i].L;
         }
       }
     }

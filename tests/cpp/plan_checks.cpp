@@ -1,7 +1,9 @@
 // Checks of the host-side work plans (capi_internal.h), no GPU needed: the FP64
 // fused kernel's tiles and chunks against the best that an exhaustive search
-// finds.  Usage: plan_checks <check>; prints "ok" or what is wrong.
+// finds, and the search for tiles and chunks against plain loops over all of them.
+// Usage: plan_checks <check>; prints "ok" or what is wrong.
 #include <algorithm>
+#include <chrono>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -49,9 +51,116 @@ static int check_f64_tiles() {
   return bad;
 }
 
+// decompose and fit_tile as plain loops over every extent and chunk length: what the
+// library's search must find.
+static double cost_of(const vlct::StageKind& k, int tx, int ty) {
+  return up((tx + 2) * (ty + 2), 32) + (k.f64 ? (k.nn ? 1.6 : 2.6) : 6.0);
+}
+static Decomp all_choices(const vlct::StageKind& k, const Window& w, long nblocks) {
+  Decomp d;
+  const int top = k.f64 ? 16 : 40;
+  double best = 1e300;
+  for (int y = 1; y <= std::min(top, w.len[1]); y++)
+    for (int x = 1; x <= std::min(top, w.len[0]); x++) {
+      if (up(w.len[0], up(w.len[0], x)) != x || up(w.len[1], up(w.len[1], y)) != y ||
+          !k.fits(x, y))
+        continue;
+      const int warps = up((x + 2) * (y + 2), 32);
+      auto plane = [&](long n) {
+        return k.f64 ? std::max(k.nn ? 5.2 : 6.4, cost_of(k, x, y))
+                     : std::max(1.0 + 0.02 * warps, 0.35 + 0.065 * (double)n * (up(warps, 4) * 4));
+      };
+      for (int L : {0, 32, 24, 16, 12, 10, 8, 7, 6, 5, 4, 3, 2, 1}) {
+        if (L >= w.len[2]) continue;
+        const int nz = L > 0 ? up(w.len[2], L) : 1;
+        const long res = (long)k.ctas() * kSms;
+        const long n = (long)up(w.len[0], x) * up(w.len[1], y) * nblocks * nz, rest = n % res;
+        const double cost = ((double)(n / res) * plane(k.ctas()) +
+                             (rest ? plane((rest + kSms - 1) / kSms) : 0.0)) *
+                            (up(w.len[2], nz) + (k.f64 ? 1.6 : 2.5));
+        if (cost < best * 0.999) {
+          best = cost;
+          d.tx = x;
+          d.ty = y;
+          d.zchunk = L;
+        }
+      }
+    }
+  return d;
+}
+static void all_tiles(const vlct::StageKind& k, int lx, int ly, int& tx, int& ty) {
+  const int top = k.f64 ? 16 : 40;
+  const int mx = std::min(lx, tx > 0 ? std::min(tx, top) : top);
+  const int my = std::min(ly, ty > 0 ? std::min(ty, top) : top);
+  double best = 1e300;
+  for (int x = 1; x <= mx; x++)
+    for (int y = 1; y <= my; y++) {
+      const int ax = up(lx, up(lx, x)), ay = up(ly, up(ly, y));
+      if (!k.fits(ax, ay)) continue;
+      const double c = (double)up(lx, ax) * up(ly, ay) * cost_of(k, ax, ay);
+      if (c <= best) {
+        best = c;
+        tx = ax;
+        ty = ay;
+      }
+    }
+}
+static int check_search() {
+  int bad = 0;
+  for (int kind = 0; kind < 8; kind++) {
+    const vlct::StageKind k = {(kind & 1) != 0, (kind & 2) != 0, (kind & 4) != 0};
+    for (int i = 0; i < 400; i++) {
+      const unsigned r = 2654435761u * (unsigned)(i + 1);
+      const int big = i % 10 == 0 ? 300 : 70;
+      const Window w = {1, {1 + (int)(r % big), 1 + (int)(r / 97 % big), 1 + (int)(r / 9409 % big)}};
+      const long nb = 1 + (long)(r >> 27);
+      const Decomp a = decompose(k, w, nb, kSms), b = all_choices(k, w, nb);
+      int tx = i % 3 * 7, ty = i % 5 * 4, ux = tx, uy = ty;
+      fit_tile(k, w.len[0], w.len[1], tx, ty);
+      all_tiles(k, w.len[0], w.len[1], ux, uy);
+      if (a.tx != b.tx || a.ty != b.ty || a.zchunk != b.zchunk || tx != ux || ty != uy) {
+        std::printf("kind %d %d x %d x %d, %ld blocks: %d x %d x %d, not %d x %d x %d; %d x %d, not %d x %d\n",
+                    kind, w.len[0], w.len[1], w.len[2], nb, a.tx, a.ty, a.zchunk, b.tx, b.ty,
+                    b.zchunk, tx, ty, ux, uy);
+        bad = 1;
+      }
+    }
+  }
+  return bad;
+}
+
+// The search of a block's two stages, which a handle's first step at an extent and
+// every small batch wait for: at most a tenth of the plain loops' time.
+static int check_search_time() {
+  int bad = 0;
+  for (int f64 = 0; f64 < 2; f64++)
+    for (int n : {32, 64, 96}) {
+      const vlct::StageKind nn = {f64 != 0, true, true}, plm = {f64 != 0, false, true};
+      const Window w0 = {1, {n + 4, n + 4, n + 4}}, w1 = {3, {n, n, n}};
+      double t[2] = {1e9, 1e9};
+      for (int rep = 0; rep < 200; rep++)
+        for (int which = 0; which < 2; which++) {
+          const auto t0 = std::chrono::steady_clock::now();
+          const Decomp a = which ? all_choices(nn, w0, 1) : decompose(nn, w0, 1, kSms);
+          const Decomp b = which ? all_choices(plm, w1, 1) : decompose(plm, w1, 1, kSms);
+          const std::chrono::duration<double, std::micro> us = std::chrono::steady_clock::now() - t0;
+          if (a.tx + b.tx <= 0) return 1;
+          t[which] = std::min(t[which], us.count());
+        }
+      std::fprintf(stderr, "f64 %d, %d^3: %.1f us, plain loops %.1f us\n", f64, n, t[0], t[1]);
+      if (t[0] > 0.25 * t[1]) {
+        std::printf("f64 %d, %d^3: %.1f us, plain loops %.1f us\n", f64, n, t[0], t[1]);
+        bad = 1;
+      }
+    }
+  return bad;
+}
+
 int main(int argc, char** argv) {
   int bad = 2;
   if (argc > 1 && !std::strcmp(argv[1], "f64_tiles")) bad = check_f64_tiles();
+  if (argc > 1 && !std::strcmp(argv[1], "search")) bad = check_search();
+  if (argc > 1 && !std::strcmp(argv[1], "search_time")) bad = check_search_time();
   if (!bad) std::printf("ok\n");
   return bad;
 }
