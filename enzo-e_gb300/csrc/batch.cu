@@ -269,8 +269,8 @@ int build_descriptors(mhdvlct_batch* b, cudaStream_t st) {
     for (int s = 0; s < 2; s++)
       split_plan(m, {}, sp.S[s], s == 1, b->h->mhd != 0, b->h->de != 0, jobs[s], b->sp_groups[s],
                  b->ws_elems);
-    if (!b->ws_asked &&
-        bmalloc(b, &b->d_ws, std::max<size_t>(b->ws_elems, 1) * sizeof(R)) != cudaSuccess) {
+    if (!b->ws_asked && b->ws_elems > 0 &&
+        bmalloc(b, &b->d_ws, b->ws_elems * sizeof(R)) != cudaSuccess) {
       cudaGetLastError();
       b->d_ws = nullptr;
     }
@@ -1312,14 +1312,15 @@ int autotune_t(mhdvlct_batch* b, int reps, std::string& json, cudaStream_t st) {
       std::vector<TileChoice> cands;
       // the split FP64 stages have no tiles: the choice in force is the only
       // candidate
-      if (b->d_ws) cands.push_back(bestc);
+      const bool split = b->d_ws && !b->sp_groups[s].empty();
+      if (split) cands.push_back(bestc);
       // the least-work tile, then each shape, as the fused kernel takes them
       const int m[3] = {cls[0] + 2 * b->g, cls[1] + 2 * b->g, cls[2] + 2 * b->g};
       const Window w = stage_window(m, sp.S[s]);
       std::vector<std::pair<int, int>> seen;
       shapes.insert(shapes.begin(), {0, 0});
       for (auto sh : shapes) {
-        if (b->d_ws || w.len[0] <= 0 || w.len[1] <= 0) break;
+        if (split || w.len[0] <= 0 || w.len[1] <= 0) break;
         fit_tile(stage_kind(b->h, b->dtype, s), w.len[0], w.len[1], sh.first, sh.second);
         if (std::find(seen.begin(), seen.end(), sh) != seen.end()) continue;
         seen.push_back(sh);

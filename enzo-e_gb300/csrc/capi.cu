@@ -233,6 +233,12 @@ void split_plan(const std::vector<int>& m, const std::vector<int>& ids, int S, b
   // (a group ends in a partly filled wave), 0.3 GB of workspace with CT
   constexpr size_t kGroupCells = 1300000;
   constexpr int kGroupJobs = 16384;  // below the grid's y limit
+  // Planes of a slab, at least.  A slab of n planes solves the x and y faces of n + 2
+  // planes with CT, so below five the fused kernel is as fast (HLLD with PLM, split /
+  // fused: 340 x 340 x 32 cells, six planes, 27.3 / 31.7 ms; 400 x 400 x 64, three,
+  // 88.8 / 82.7; 512 x 512 x 64, one, 242 / 132; HLLE with NN the same ratios).  Hydro
+  // solves no such faces: one plane, 512 x 512 x 16, 19.8 / 20.3 ms.
+  const int least = mhd ? 5 : 1;
   const size_t arrays = split_arrays(mhd, de);
   const size_t limit = max_elems ? max_elems / arrays : kGroupCells;
   struct Piece {
@@ -250,6 +256,11 @@ void split_plan(const std::vector<int>& m, const std::vector<int>& ids, int S, b
     const size_t plane = (size_t)e[0] * e[1];
     const int most = (int)std::max<long long>(1, (long long)(kGroupCells / plane) - 4);
     const int len = e[2] - 2 * lo, parts = (len + most - 1) / most;
+    if (most < std::min(least, len)) {
+      jobs.clear();
+      groups.clear();
+      return;
+    }
     for (int p = 0, z = lo; p < parts; p++) {
       const int n = len / parts + (p < len % parts ? 1 : 0);
       pieces.push_back({SplitJob{i, z, z + n, 0}, plane * (size_t)(n + 4)});

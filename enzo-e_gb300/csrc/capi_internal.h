@@ -103,7 +103,8 @@ void make_tiles(int block, const int m[3], int S, int tile_x, int tile_y, int zc
 // The jobs of a split stage over blocks of ghosted extents m (3 per block),
 // blocks `ids` of them (all when empty), in groups whose workspace is bounded
 // (by max_elems too, when given); ws_elems is raised to the elements the
-// largest group needs.
+// largest group needs.  No jobs when a block's planes are so wide that the fused
+// kernel is the faster form.
 void split_plan(const std::vector<int>& m, const std::vector<int>& ids, int S, bool final,
                 bool mhd, bool de, std::vector<vlct::SplitJob>& jobs,
                 std::vector<vlct::SplitGroup>& groups, size_t& ws_elems, size_t max_elems = 0);

@@ -156,11 +156,45 @@ static int check_search_time() {
   return bad;
 }
 
+// A z-slab of a split MHD stage solves the x and y faces of two planes more than it
+// updates: over all slabs of a block, at most half again as many (or the stage runs
+// as the fused kernel), and every plane is updated once, within the workspace.
+static int check_slabs() {
+  int bad = 0;
+  for (int mhd = 0; mhd < 2; mhd++)
+    for (int nx : {8, 118, 256, 340, 390, 400, 512, 800, 2000})
+      for (int nz : {4, 8, 16, 64, 300}) {
+        const int S = 2, lo = S + 1;
+        const std::vector<int> m = {nx + 6, nx + 6, nz + 6};
+        std::vector<vlct::SplitJob> jobs;
+        std::vector<vlct::SplitGroup> groups;
+        size_t ws = 0;
+        split_plan(m, {}, S, false, mhd != 0, false, jobs, groups, ws);
+        int next = lo, planes = 0;
+        for (const auto& j : jobs) {
+          if (j.za != next) bad = 1;
+          next = j.zb;
+          planes += j.zb - j.za + 2;
+        }
+        const int len = m[2] - 2 * lo;
+        if ((!jobs.empty() && next != m[2] - lo) || (jobs.empty() && ws != 0)) bad = 1;
+        if (mhd && jobs.size() > 1 && planes > 1.5 * len) bad = 1;
+        if (mhd && jobs.empty() && nx < 380) bad = 1;  // narrow planes are never refused
+        if (bad) {
+          std::printf("mhd %d, %d x %d x %d: %zu slabs, %d planes of faces for %d\n", mhd, nx, nx,
+                      nz, jobs.size(), planes, len);
+          return 1;
+        }
+      }
+  return 0;
+}
+
 int main(int argc, char** argv) {
   int bad = 2;
   if (argc > 1 && !std::strcmp(argv[1], "f64_tiles")) bad = check_f64_tiles();
   if (argc > 1 && !std::strcmp(argv[1], "search")) bad = check_search();
   if (argc > 1 && !std::strcmp(argv[1], "search_time")) bad = check_search_time();
+  if (argc > 1 && !std::strcmp(argv[1], "slabs")) bad = check_slabs();
   if (!bad) std::printf("ok\n");
   return bad;
 }

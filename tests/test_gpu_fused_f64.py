@@ -174,3 +174,24 @@ def test_block_step_with_stored_fluxes():
     for a, b in zip(*out):
         for k in a:
             assert np.array_equal(a[k], b[k]), k
+
+
+@pytest.mark.parametrize("n", [(380, 350, 14), (410, 400, 9)])
+def test_wide_planes(n):
+    # the widest planes that the split stages take, in slabs of five planes, and
+    # wider ones
+    out = []
+    for form in FORMS:
+        meth = _method(form)
+        blk = B.Block(n, 3, (1.0 / 64,) * 3)
+        g = torch.Generator(device="cuda")
+        g.manual_seed(2)
+        for k, t in blk.fields.items():
+            r = torch.rand(t.shape, generator=g, dtype=t.dtype, device="cuda")
+            t.copy_({"density": 1.0, "total_energy": 4.0}.get(k, 0.0) + 0.3 * r)
+        meth.compute(blk, 1e-3)
+        torch.cuda.synchronize()
+        out.append(blk.fields)
+    for k in out[0]:
+        assert torch.isfinite(out[0][k]).all(), k
+        assert torch.equal(out[0][k], out[1][k]), k

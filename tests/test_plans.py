@@ -25,7 +25,7 @@ def checks(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("check", ["f64_tiles", "search", "search_time"])
+@pytest.mark.parametrize("check", ["f64_tiles", "search", "search_time", "slabs"])
 def test_plan(checks, check):
     r = subprocess.run([checks, check], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout + r.stderr
