@@ -1153,13 +1153,17 @@ constexpr int kNoAllocMaxTiles = 1024;                    // per stage
 constexpr int kNoAllocMaxDevices = 64;
 
 __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
+// the tile lists of both stages: beside the scratch, so that how finely a block
+// is cut does not decide whether it fits
+__device__ StageTile g_noalloc_tiles[2 * kNoAllocMaxTiles];
 
 std::mutex g_noalloc_mu;
 char* g_noalloc_base[kNoAllocMaxDevices] = {};
+StageTile* g_noalloc_tile_base[kNoAllocMaxDevices] = {};
 
-// Device address of the scratch array on the current device (first call per
-// device resolves it; later calls read the cache).
-int noalloc_base(mhdvlct_handle* h, char** out) {
+// Device addresses of the two arrays on the current device (first call per
+// device resolves them; later calls read the cache).
+int noalloc_base(mhdvlct_handle* h, char** out, StageTile** tiles) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return cuda_fail(h, e, "cudaGetDevice");
@@ -1170,9 +1174,14 @@ int noalloc_base(mhdvlct_handle* h, char** out) {
     void* p = nullptr;
     e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
     if (e != cudaSuccess) return cuda_fail(h, e, "cudaGetSymbolAddress(no-alloc scratch)");
+    void* q = nullptr;
+    e = cudaGetSymbolAddress(&q, g_noalloc_tiles);
+    if (e != cudaSuccess) return cuda_fail(h, e, "cudaGetSymbolAddress(no-alloc tiles)");
     g_noalloc_base[dev] = (char*)p;
+    g_noalloc_tile_base[dev] = (StageTile*)q;
   }
   *out = g_noalloc_base[dev];
+  *tiles = g_noalloc_tile_base[dev];
   return MHD_OK;
 }
 
@@ -1205,8 +1214,7 @@ int block_step_noalloc_t(mhdvlct_handle* h, const MhdBlockView* b, double dt,
   }
 
   // carve the static array: cells, half-step scalars, stage-0 faces, final
-  // faces, dt, stage descriptors, flux-output record, tiles (each region
-  // 256-byte aligned)
+  // faces, dt, stage descriptors (each region 256-byte aligned)
   const size_t M = (size_t)m[0] * m[1] * m[2];
   const size_t F[3] = {(size_t)(m[0] + 1) * m[1] * m[2], (size_t)m[0] * (m[1] + 1) * m[2],
                        (size_t)m[0] * m[1] * (m[2] + 1)};
@@ -1224,7 +1232,6 @@ int block_step_noalloc_t(mhdvlct_handle* h, const MhdBlockView* b, double dt,
   for (int d = 0; d < 3; d++) o_ff[d] = take(F[d] * sizeof(R));
   const size_t o_dt = take(sizeof(double));
   const size_t o_sb = take(2 * sizeof(StageBlock<R>));
-  const size_t o_tl = take((size_t)(nt[0] + nt[1]) * sizeof(StageTile));
   if (off > kNoAllocScratchBytes)
     return fail(h, MHD_ERR_INVALID,
                 "block needs " + std::to_string(off) +
@@ -1233,7 +1240,8 @@ int block_step_noalloc_t(mhdvlct_handle* h, const MhdBlockView* b, double dt,
                     " bytes (use mhdvlct_block_step)");
 
   char* base = nullptr;
-  int rc = noalloc_base(h, &base);
+  StageTile* tiles = nullptr;
+  int rc = noalloc_base(h, &base, &tiles);
   if (rc) return rc;
   PlainScratch<R> S{};
   for (int k = 0; k < NCELL; k++) S.tmp[k] = (R*)(base + o_tmp[k]);
@@ -1245,11 +1253,11 @@ int block_step_noalloc_t(mhdvlct_handle* h, const MhdBlockView* b, double dt,
   }
   S.d_dt = (double*)(base + o_dt);
   S.d_sblocks = (StageBlock<R>*)(base + o_sb);
-  S.d_tiles = (StageTile*)(base + o_tl);
+  S.d_tiles = tiles;
   S.ntiles[0] = (int)nt[0];
   S.ntiles[1] = (int)nt[1];
   // every call rewrites the dt slot, the descriptors and the tile lists (the
-  // array keeps whatever the previous call left)
+  // arrays keep whatever the previous call left)
   cudaError_t e = launch_set_scalar(S.d_dt, dt, st);
   if (e == cudaSuccess) e = launch_make_tiles(S.d_tiles, ts[0], st);
   if (e == cudaSuccess) e = launch_make_tiles(S.d_tiles + nt[0], ts[1], st);

@@ -185,18 +185,18 @@ int mhdvlct_block_step_device_dt(mhdvlct_handle* h, const MhdBlockView* b,
  * a call that may synchronise the whole device while other streams run.
  * Same operation and results as mhdvlct_block_step, but allocates no device
  * memory: its scratch
- * is one file-scope __device__ array of 8 MiB (8388608 bytes) per device,
- * whose address is taken with cudaGetSymbolAddress on the first call on each
- * device and cached.  Make that first call on a device outside stream
+ * is one file-scope __device__ array of 8 MiB (8388608 bytes) per device, and
+ * one of 56 KiB for its tile lists, whose addresses are taken with
+ * cudaGetSymbolAddress on the first call on each device and cached.  Make that first call on a device outside stream
  * capture.  A block whose scratch (all cell fields, the passive scalars'
  * half step and two sets of face fields at the ghosted extents, plus
  * descriptors) exceeds 8 MiB, or whose
  * stage needs more than 1024 tiles, is rejected with MHD_ERR_INVALID and a
  * message naming the bytes needed (an FP64 block of 32^3 cells with 3 ghost
- * zones needs about 6.7 MB).  Nothing in the array has to start at zero:
+ * zones needs about 6.7 MB).  Nothing in the arrays has to start at zero:
  * every call rewrites the dt slot, the stage descriptors and the tile list,
  * and each intermediate value a stage reads was written earlier in the same
- * call.  All calls on one device share the array: two calls that overlap in
+ * call.  All calls on one device share the arrays: two calls that overlap in
  * time (different streams, threads or handles) race on it; order them on one
  * stream or synchronise between them. */
 int mhdvlct_block_step_noalloc(mhdvlct_handle* h, const MhdBlockView* b,
