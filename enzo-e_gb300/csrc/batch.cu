@@ -145,6 +145,15 @@ int bfail(mhdvlct_batch* b, int code, const std::string& m) {
   return code;
 }
 
+void drop_graphs(mhdvlct_batch* b) {
+  for (int p = 0; p < 2; p++)
+    for (int d = 0; d < 2; d++)
+      if (b->graph[p][d]) {
+        cudaGraphExecDestroy(b->graph[p][d]);
+        b->graph[p][d] = nullptr;
+      }
+}
+
 // Device memory of a batch: stream-ordered on the batch's stream for an
 // ordered batch, plain cudaMalloc / cudaFree otherwise.
 cudaError_t bmalloc(mhdvlct_batch* b, void** p, size_t n) {
@@ -157,19 +166,28 @@ void bfree(mhdvlct_batch* b, void* p) {
   if (b->ordered) cudaFreeAsync(p, b->ost);
   else cudaFree(p);
 }
+// The same for what a batch is set up with (descriptors, refresh and correction
+// tables, the autotuner's copy).  Without room the split stages' workspace is given
+// back first, and the fused kernels run from then on: what a call needs comes
+// before what makes the stages faster.  Set-up calls only: the workspace's address
+// may be in a graph that the caller captured from a step.
+cudaError_t setup_malloc(mhdvlct_batch* b, void** p, size_t n) {
+  cudaError_t e = bmalloc(b, p, n);
+  if (e != cudaSuccess && b->d_ws) {
+    cudaGetLastError();
+    if (b->ordered) cudaStreamSynchronize(b->ost);
+    else cudaDeviceSynchronize();
+    drop_graphs(b);
+    bfree(b, b->d_ws);
+    b->d_ws = nullptr;
+    e = bmalloc(b, p, n);
+  }
+  return e;
+}
 // The stream of a batch's own set-up work (its ordered stream, else the
 // caller's).
 cudaStream_t setup_stream(const mhdvlct_batch* b, cudaStream_t st) {
   return b->ordered ? b->ost : st;
-}
-
-void drop_graphs(mhdvlct_batch* b) {
-  for (int p = 0; p < 2; p++)
-    for (int d = 0; d < 2; d++)
-      if (b->graph[p][d]) {
-        cudaGraphExecDestroy(b->graph[p][d]);
-        b->graph[p][d] = nullptr;
-      }
 }
 
 // The work decomposition of blocks of ghosted extents m: the one tuned or set
@@ -356,7 +374,7 @@ int build_descriptors(mhdvlct_batch* b, cudaStream_t st) {
     }
   }
   void* fresh = nullptr;
-  if (bmalloc(b, &fresh, bytes) != cudaSuccess)
+  if (setup_malloc(b, &fresh, bytes) != cudaSuccess)
     return bfail(b, MHD_ERR_NOMEM, "descriptor allocation");
   if (cudaMemcpyAsync(fresh, image.get(), bytes, cudaMemcpyHostToDevice, st) != cudaSuccess) {
     bfree(b, fresh);
@@ -712,7 +730,7 @@ int set_flux_correction_t(mhdvlct_batch* b, unsigned quantities, const MhdRefres
   int nq = 0;
   for (int q = 0; q < MHD_FC_NQ; q++) nq += (quantities >> q) & 1u;
   const size_t per_block = 2 * (face_elems[0] + face_elems[1] + face_elems[2]) * nq;
-  if (bmalloc(b, &b->d_flux, per_block * b->nblocks * sizeof(R)) != cudaSuccess) {
+  if (setup_malloc(b, &b->d_flux, per_block * b->nblocks * sizeof(R)) != cudaSuccess) {
     b->d_flux = nullptr;
     return bfail(b, MHD_ERR_NOMEM, "flux buffers");
   }
@@ -737,8 +755,8 @@ int set_flux_correction_t(mhdvlct_batch* b, unsigned quantities, const MhdRefres
   int rc = plan_flux_correct(b->h, views.data(), b->nblocks, fcs.data(), faces, nfaces,
                              conservative, b->fcplan);
   if (rc != MHD_OK) return bfail(b, rc, b->h->err);
-  if (bmalloc(b, &b->d_fluxout, outs.size() * sizeof(FluxOut<R>)) != cudaSuccess ||
-      bmalloc(b, (void**)&b->d_fcplan, std::max<size_t>(b->fcplan.blob.size(), 16)) !=
+  if (setup_malloc(b, &b->d_fluxout, outs.size() * sizeof(FluxOut<R>)) != cudaSuccess ||
+      setup_malloc(b, (void**)&b->d_fcplan, std::max<size_t>(b->fcplan.blob.size(), 16)) !=
           cudaSuccess)
     return bfail(b, MHD_ERR_NOMEM, "flux-correction tables");
   cudaError_t e = cudaMemcpy(b->d_fluxout, outs.data(), outs.size() * sizeof(FluxOut<R>),
@@ -813,7 +831,7 @@ extern "C" int mhdvlct_batch_set_refresh_faces(mhdvlct_batch* b, const MhdRefres
   memcpy(host.data() + b->rf_ptr[1], plan[1].ptrs.data(), bp);
   memcpy(host.data() + b->rf_items, plan[0].items.data(), plan[0].items.size());
   memcpy(host.data() + b->rf_chunks, plan[0].chunks.data(), plan[0].chunks.size());
-  if (bmalloc(b, (void**)&b->d_rf, total) != cudaSuccess) {
+  if (setup_malloc(b, (void**)&b->d_rf, total) != cudaSuccess) {
     b->d_rf = nullptr;
     return bfail(b, MHD_ERR_NOMEM, "refresh tables");
   }
@@ -1265,7 +1283,7 @@ int autotune_t(mhdvlct_batch* b, int reps, std::string& json, cudaStream_t st) {
   // save the state so the trial steps leave no trace
   const size_t bytes = b->state_elems * sizeof(R);
   void* save = nullptr;
-  if (bmalloc(b, &save, bytes) != cudaSuccess)
+  if (setup_malloc(b, &save, bytes) != cudaSuccess)
     return bfail(b, MHD_ERR_NOMEM, "autotune state copy");
   const int parity0 = b->parity;
   cudaMemcpyAsync(save, b->pool, bytes, cudaMemcpyDeviceToDevice, st);
