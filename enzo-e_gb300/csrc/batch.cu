@@ -1385,26 +1385,34 @@ int autotune_t(mhdvlct_batch* b, int reps, std::string& json, cudaStream_t st) {
       best_stage[s] = best / std::max(1, reps);
       if (e != cudaSuccess) break;
     }
-    // the tiles in force: what the fused kernel makes of the choices
+    // what is in force: of a fused stage the tile that the kernel makes of the
+    // choice and its CTA's size; a split stage has no tile
     const int m[3] = {cls[0] + 2 * b->g, cls[1] + 2 * b->g, cls[2] + 2 * b->g};
-    int shape[2][2];
+    std::string stage[2];
     for (int k = 0; k < 2; k++) {
+      const bool split = b->d_ws && !b->sp_groups[k].empty();
+      const StageKind kind = stage_kind(b->h, b->dtype, k);
       const Window w = stage_window(m, sp.S[k]);
-      shape[k][0] = bestc.tile_x[k];
-      shape[k][1] = bestc.tile_y[k];
-      fit_tile(stage_kind(b->h, b->dtype, k), w.len[0], w.len[1], shape[k][0], shape[k][1]);
+      int tx = 0, ty = 0;
+      if (!split) {
+        tx = bestc.tile_x[k];
+        ty = bestc.tile_y[k];
+        fit_tile(kind, w.len[0], w.len[1], tx, ty);
+      }
+      char part[160];
+      std::snprintf(part, sizeof(part),
+                    "{\"form\": \"%s\", \"tile_x\": %d, \"tile_y\": %d, \"zchunk\": %d, "
+                    "\"threads\": %d}",
+                    split ? "split" : "fused", tx, ty, split ? 0 : bestc.zchunk[k],
+                    split ? kSplitThreads : kind.threads());
+      stage[k] = part;
     }
-    const int threads[2] = {stage_kind(b->h, b->dtype, 0).threads(),
-                            stage_kind(b->h, b->dtype, 1).threads()};
     char buf[512];
     std::snprintf(buf, sizeof(buf),
-                  "%s\"%dx%dx%d\": {\"stage1\": {\"tile_x\": %d, \"tile_y\": %d, "
-                  "\"zchunk\": %d, \"threads\": %d}, \"stage2\": {\"tile_x\": %d, "
-                  "\"tile_y\": %d, \"zchunk\": %d, \"threads\": %d}, "
+                  "%s\"%dx%dx%d\": {\"stage1\": %s, \"stage2\": %s, "
                   "\"ms_per_step\": %.4f, \"candidates\": %zu}",
-                  first_cls ? "" : ", ", cls[0], cls[1], cls[2], shape[0][0],
-                  shape[0][1], bestc.zchunk[0], threads[0], shape[1][0],
-                  shape[1][1], bestc.zchunk[1], threads[1], best_stage[1], ncand);
+                  first_cls ? "" : ", ", cls[0], cls[1], cls[2], stage[0].c_str(),
+                  stage[1].c_str(), best_stage[1], ncand);
     json += buf;
     first_cls = false;
     if (e != cudaSuccess) break;

@@ -33,7 +33,7 @@ cudaError_t stage_split(const StageBlock<R>* b, const SplitLaunch& sp, const Sta
   for (int k = 0; k < sp.ngroups; k++) {
     const SplitGroup& G = sp.groups[k];
     const SplitJob* jobs = sp.jobs + G.first;
-    const unsigned gx = (unsigned)((G.cells + 127) / 128);
+    const unsigned gx = (unsigned)((G.cells + kSplitThreads - 1) / kSplitThreads);
     const dim3 cells(gx, G.count);
     // faces a thread takes: as many as leave 256 threads to every SM
     int kmax = 1;
@@ -41,10 +41,10 @@ cudaError_t stage_split(const StageBlock<R>* b, const SplitLaunch& sp, const Sta
       kmax = (int)std::max<size_t>(1, std::min<size_t>(12, 3 * G.total / ((size_t)nsm * 256)));
     const int kmin = (kmax + 1) / 2;
     const dim3 faces((gx + kmin - 1) / kmin, G.count, 3);
-    split_prim_kernel<R, SOLVER, RECON == RECON_NN, DE><<<cells, 128, 0, st>>>(b, jobs, ws, info, phys);
-    split_flux_kernel<R, SOLVER, RECON, DE><<<faces, 128, 0, st>>>(b, jobs, ws, info, phys, kmax);
-    if constexpr (MHD) split_emf_kernel<R, DE><<<cells, 128, 0, st>>>(b, jobs, ws, info);
-    split_update_kernel<R, MHD, DE><<<cells, 128, 0, st>>>(b, jobs, ws, info, phys);
+    split_prim_kernel<R, SOLVER, RECON == RECON_NN, DE><<<cells, kSplitThreads, 0, st>>>(b, jobs, ws, info, phys);
+    split_flux_kernel<R, SOLVER, RECON, DE><<<faces, kSplitThreads, 0, st>>>(b, jobs, ws, info, phys, kmax);
+    if constexpr (MHD) split_emf_kernel<R, DE><<<cells, kSplitThreads, 0, st>>>(b, jobs, ws, info);
+    split_update_kernel<R, MHD, DE><<<cells, kSplitThreads, 0, st>>>(b, jobs, ws, info, phys);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }

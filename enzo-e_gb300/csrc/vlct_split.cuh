@@ -69,7 +69,7 @@ __device__ __forceinline__ SplitCtx<R> split_ctx(const StageBlock<R>& B, const S
 // quantities that the faces of a cell share in an NN stage, and the cell-centred
 // E = -v x B (EnzoComputePressure.cpp:127-190, EnzoBfieldMethodCT.cpp:267-292)
 template <class R, int SOLVER, bool NN, bool DE>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(kSplitThreads)
 split_prim_kernel(const StageBlock<R>* __restrict__ blocks, const SplitJob* __restrict__ jobs,
                   R* __restrict__ ws, StageInfo info, PhysParams phys) {
   constexpr bool MHD = SOLVER != SOLVER_HLLC;
@@ -123,7 +123,7 @@ split_prim_kernel(const StageBlock<R>* __restrict__ blocks, const SplitJob* __re
 // more where a line of faces is cut).  K: as many faces as leave the GPU's
 // pipes filled (host), with the cut of the line that wastes least (below).
 template <class R, int SOLVER, int RECON, bool DE>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(kSplitThreads)
 split_flux_kernel(const StageBlock<R>* __restrict__ blocks, const SplitJob* __restrict__ jobs,
                   R* __restrict__ ws, StageInfo info, PhysParams phys, int kmax) {
   constexpr bool MHD = SOLVER != SOLVER_HLLC;
@@ -294,7 +294,7 @@ split_flux_kernel(const StageBlock<R>* __restrict__ blocks, const SplitJob* __re
 // ---- edge EMFs (EnzoBfieldMethodCT.cpp:480-590): the three edges on the high
 // side of each cell
 template <class R, bool DE>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(kSplitThreads)
 split_emf_kernel(const StageBlock<R>* __restrict__ blocks, const SplitJob* __restrict__ jobs,
                  R* __restrict__ ws, StageInfo info) {
   using L = SplitLayout<true, DE>;
@@ -340,7 +340,7 @@ split_emf_kernel(const StageBlock<R>* __restrict__ blocks, const SplitJob* __res
 // conserved update, floors and energy sync, the stored boundary fluxes and the
 // density fluxes of the passive scalars (phase D of the fused kernel)
 template <class R, bool MHD, bool DE>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(kSplitThreads)
 split_update_kernel(const StageBlock<R>* __restrict__ blocks, const SplitJob* __restrict__ jobs,
                     R* __restrict__ ws, StageInfo info, PhysParams phys) {
   using L = SplitLayout<MHD, DE>;

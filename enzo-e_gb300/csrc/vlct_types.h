@@ -48,6 +48,8 @@ struct StageTile {
   int xa, xb, ya, yb, za, zb;
 };
 
+constexpr int kSplitThreads = 128;  // of a CTA of the split stages
+
 // One unit of work of the split stages (vlct_split.cuh): the output planes
 // [za, zb) of one block over its whole x-y extent, and where its workspace
 // arrays start (in elements).

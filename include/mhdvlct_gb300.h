@@ -372,7 +372,14 @@ int mhdvlct_batch_timestep(mhdvlct_batch* b, double* dt_out, void* stream);
  * replayed.  elapsed_time_out (may be NULL) receives the sum of dt. */
 int mhdvlct_batch_run(mhdvlct_batch* b, int ncycles, int dt_mode,
                       double* elapsed_time_out, void* stream);
-/* Work decomposition: tile extent used per block size class (0 = auto). */
+/* Work decomposition: tile extent used per block size class (0 = auto).  Tiles
+ * are the fused stage kernel's, which FP32 batches run.  FP64 batches run their
+ * stages as split kernels over whole blocks, where tiles, chunks and the autotuner
+ * change nothing (but the cutting of the passive scalars' kernel); they run the
+ * fused kernel when the GPU has no room for the split kernels' workspace (0.4 GB
+ * at most a batch, or a handle for mhdvlct_block_step; for hydro blocks of planes
+ * wider than 500 x 500 cells 1.3 KB a cell of five planes), and for MHD blocks of planes
+ * wider than about 380 x 380 cells. */
 int mhdvlct_batch_set_tile(mhdvlct_batch* b, int tile_x, int tile_y);
 /* One stage's work decomposition for every block (stage 0: half dt, 1: full
  * dt): tile extents, z-chunk length (0 = whole block), e.g. to pin a tuned
@@ -383,7 +390,8 @@ int mhdvlct_batch_set_stage_tile(mhdvlct_batch* b, int stage, int tile_x,
 /* The autotuner: for every block-size class, time candidate (tile, z-chunk)
  * work decompositions on the batch's own data and keep the fastest.  The
  * state is restored afterwards.  json_out (may be NULL) receives a JSON
- * description of the choices. */
+ * description of the choices: per class and stage its form ("fused" or "split"),
+ * tile_x, tile_y, zchunk (0 for a split stage, which has none) and threads. */
 int mhdvlct_batch_autotune(mhdvlct_batch* b, int reps, char* json_out,
                            size_t json_len, void* stream);
 /* Device address and size of the contiguous region holding every block's

@@ -4,6 +4,7 @@ launch's queue, gravity and passive scalars, stored boundary fluxes with flux
 correction, and the host-state run by groups of blocks.  The results are the
 split kernels' bit for bit, and where a cheap oracle run exists the oracle's."""
 import ctypes
+import json
 
 import numpy as np
 import pytest
@@ -195,3 +196,24 @@ def test_wide_planes(n):
     for k in out[0]:
         assert torch.isfinite(out[0][k]).all(), k
         assert torch.equal(out[0][k], out[1][k]), k
+
+
+@pytest.mark.parametrize("dtype,form,says", [
+    (capi.MHD_DTYPE_F64, "split", "split"), (capi.MHD_DTYPE_F64, "fused", "fused"),
+    (capi.MHD_DTYPE_F32, "split", "fused")])
+def test_autotuner_reports_what_runs(dtype, form, says):
+    meth = _method(form)
+    n = (12, 10, 9)
+    s, w = ic.smooth_block(n, 3, seed=2)
+    bt = Batch(meth, [n], [w], dtype=dtype)
+    bt.upload(0, s)
+    buf = ctypes.create_string_buffer(4096)
+    capi.check(capi.lib().mhdvlct_batch_autotune(bt.h, 1, buf, 4096, None), meth.handle, "autotune")
+    got = json.loads(buf.value.decode())["12x10x9"]
+    for k in ("stage1", "stage2"):
+        assert got[k]["form"] == says, got
+        tile = got[k]["tile_x"], got[k]["tile_y"]
+        if says == "split":
+            assert tile == (0, 0) and got[k]["zchunk"] == 0 and got[k]["threads"] == 128, got
+        else:
+            assert min(tile) >= 1 and (tile[0] + 2) * (tile[1] + 2) <= got[k]["threads"], got
