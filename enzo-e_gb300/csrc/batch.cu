@@ -458,32 +458,40 @@ cudaError_t launch_stages(mhdvlct_batch* b, cudaStream_t st) {
   return cudaSuccess;
 }
 
-// 256-thread CTAs that fill the GPU about four times over (SM count of the
-// current device, thread-safe one-time initialisation)
-size_t fill_ctas() {
-  static const size_t n = [] {
-    int dev = 0, nsm = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        nsm <= 0)
-      nsm = 1;
-    return (size_t)nsm * 8 * 4;
-  }();
-  return n;
+// The blocks' mean cells and ghost cells, and whether the largest has half as many
+// again; fill: CTAs of 256 threads that fill the GPU about four times over.
+struct Sizes {
+  size_t cells = 0, shell = 0, fill = 0;
+  bool uneven = false;
+};
+Sizes sizes_of(const mhdvlct_batch* b) {
+  Sizes z;
+  size_t largest = 0, act = 0;
+  for (int i = 0; i < b->nblocks; i++) {
+    const int *m = b->off[i].m, *n = &b->dims[3 * i];
+    const size_t c = (size_t)m[0] * m[1] * m[2];
+    z.cells += c;
+    act += (size_t)n[0] * n[1] * n[2];
+    largest = std::max(largest, c);
+  }
+  z.shell = (z.cells - act) / b->nblocks;
+  z.cells /= b->nblocks;
+  z.uneven = 2 * largest > 3 * z.cells;
+  z.fill = (size_t)sm_count() * 32;
+  return z;
 }
 
 template <class R>
 cudaError_t launch_timestep_b(mhdvlct_batch* b, int global_min, cudaStream_t st) {
-  // Chunks per block: a few thousand cells each, fewer (down to two passes of
-  // a CTA) while the grid does not cover the GPU a few times over: one block of
-  // 16^3 in 10 CTAs instead of one, 25 -> 14 us (FP64: 162 -> 30 us).
-  size_t cells = 0;
-  for (auto& o : b->off) cells += (size_t)o.m[0] * o.m[1] * o.m[2];
-  const size_t per = std::max<size_t>(1, cells / b->nblocks);
-  const int cpb = (int)std::max<size_t>(
-      1, std::min<size_t>(per / 1024, std::max<size_t>(per / 8192, fill_ctas() / b->nblocks)));
+  const Sizes z = sizes_of(b);
+  // blocks of different sizes take the same number of chunks: a few thousand cells
+  // each, so that the largest ones' do not outlast the rest
+  int cpb = 0;
+  if (z.uneven)
+    cpb = (int)std::max<size_t>(
+        1, std::min(z.cells / 1024, std::max(z.cells / 8192, z.fill / b->nblocks)));
   return launch_timestep<R>(b->h->mhd != 0, b->h->de != 0,
-                            (const AuxBlock<R>*)b->d_aux[b->parity], b->nblocks, cpb,
+                            (const AuxBlock<R>*)b->d_aux[b->parity], b->nblocks, cpb, z.cells,
                             b->h->phys, b->d_smax, b->h->params.courant, global_min,
                             b->d_dt, b->d_dtmin, st);
 }
@@ -494,25 +502,17 @@ cudaError_t launch_refresh_b(mhdvlct_batch* b, cudaStream_t st) {
     return launch_refresh_faces(b->dtype, b->d_rf + b->rf_items, b->d_rf + b->rf_chunks,
                                 b->rf_nchunks, (void* const*)(b->d_rf + b->rf_ptr[b->parity]),
                                 st);
-  size_t cells = 0;
-  for (auto& o : b->off) cells += (size_t)o.m[0] * o.m[1] * o.m[2];
-  // Chunks of at most 1700 shell positions (500 in large blocks), shorter ones,
-  // down to one pass of a CTA, only while the grid is less than the three CTAs
-  // an SM holds: a CTA's pointer tables cost it two memory round trips.  One
-  // block of 16^3 18 -> 10 us; 30 of 24^3 with four such waves 24 us, with one
-  // 18 us.
-  size_t act = 0;
-  for (int i = 0; i < 3 * b->nblocks; i += 3)
-    act += (size_t)b->dims[i] * b->dims[i + 1] * b->dims[i + 2];
-  const size_t per = cells / b->nblocks, shell = (cells - act) / b->nblocks;
-  const size_t large = std::min(per / 4096, std::max<size_t>(32, fill_ctas() / b->nblocks));
-  const size_t wave = fill_ctas() * 3 / 32 / b->nblocks;
-  const int cpb = (int)std::max<size_t>(
-      1, std::min(shell / 256, std::max({large, shell / 1700, wave})));
+  const Sizes z = sizes_of(b);
+  int cpb = 0;
+  if (z.uneven)
+    cpb = (int)std::max<size_t>(
+        1, std::min(z.shell / 256,
+                    std::max({std::min(z.cells / 4096, std::max<size_t>(32, z.fill / b->nblocks)),
+                              z.shell / 1700, z.fill * 3 / 32 / b->nblocks})));
   int max_m = 0;
   for (auto& o : b->off) max_m = std::max(max_m, std::max(o.m[0], std::max(o.m[1], o.m[2])));
   return launch_refresh<R>((const AuxBlock<R>*)b->d_aux[b->parity], b->d_nbr,
-                           b->nblocks, b->g, cpb, max_m, st);
+                           b->nblocks, b->g, cpb, z.shell, b->h->mhd != 0, max_m, st);
 }
 
 template <class R>

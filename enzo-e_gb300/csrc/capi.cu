@@ -1008,7 +1008,7 @@ int block_timestep_t(mhdvlct_handle* h, const MhdBlockView* b, double* dt_out,
   const int g = b->ghost[0];
   const size_t M = (size_t)(b->n[0] + 2 * g) * (b->n[1] + 2 * g) * (b->n[2] + 2 * g);
   const int chunks = (int)std::min<size_t>(std::max<size_t>(1, M / 1024), 1024);
-  cudaError_t e = launch_timestep<R>(h->mhd != 0, h->de != 0, S.d_aux, 1, chunks, h->phys,
+  cudaError_t e = launch_timestep<R>(h->mhd != 0, h->de != 0, S.d_aux, 1, chunks, M, h->phys,
                                      S.d_smax, h->params.courant, 0,
                                      d_dt_out ? d_dt_out : S.d_dtout, nullptr, st);
   if (e != cudaSuccess) return cuda_fail(h, e, "timestep launch");
@@ -1027,7 +1027,7 @@ int fill_ghosts_t(mhdvlct_handle* h, const MhdBlockView* b, cudaStream_t st) {
   if (rc) return rc;
   const int g = b->ghost[0];
   const int max_m = std::max(b->n[0], std::max(b->n[1], b->n[2])) + 2 * g;
-  cudaError_t e = launch_refresh<R>(S.d_aux, S.d_nbr, 1, g, 64, max_m, st);
+  cudaError_t e = launch_refresh<R>(S.d_aux, S.d_nbr, 1, g, 64, 0, h->mhd != 0, max_m, st);
   if (e != cudaSuccess) return cuda_fail(h, e, "refresh launch");
   return MHD_OK;
 }

@@ -53,14 +53,19 @@ __device__ __forceinline__ double speed_max(double a, double b) { return fmax_i(
 // FP32 is bound by the bytes in flight: with 4 cells a thread (120 registers, 2
 // CTAs on an SM) DRAM was 59% busy, as an SM's loads came in two bursts with
 // arithmetic between; with 2 cells and 64 registers 4 CTAs overlap (512 blocks of
-// 32^3, MHD 223 -> 194 us; 5 CTAs, which spill, 252; 3 CTAs 214).  With dual
-// energy, which also stores, 4 cells are faster (64 blocks of 64^3 223 us, with 2
-// cells 301).  FP64 is bound by its pipe and keeps 4 cells.
-template <class R, bool DE> struct TimestepTune { static constexpr int U = 4, ctas = 1; };
-template <> struct TimestepTune<float, false> { static constexpr int U = 2, ctas = 4; };
+// 32^3, MHD 223 -> 194 us; 5 CTAs, which spill, 252; 3 CTAs 214).  Hydro, with half
+// the arrays, has the registers for 3 cells (the same set 143 us; 2 cells 155, 4 in 3
+// CTAs 146, 4 in 2 147).  With dual energy, which also stores, 4 cells are faster
+// (64 blocks of 64^3 223 us, with 2 cells 301).  FP64 is bound by its pipe and keeps
+// 4 cells.
+template <class R, bool MHD, bool DE> struct TimestepTune {
+  static constexpr int U = 4, ctas = 1;
+};
+template <> struct TimestepTune<float, true, false> { static constexpr int U = 2, ctas = 4; };
+template <> struct TimestepTune<float, false, false> { static constexpr int U = 3, ctas = 4; };
 
 template <class R, bool MHD, bool DE>
-__global__ void __launch_bounds__(256, TimestepTune<R, DE>::ctas)
+__global__ void __launch_bounds__(256, TimestepTune<R, MHD, DE>::ctas)
 timestep_kernel(const AuxBlock<R>* __restrict__ blocks, int nblocks,
                 int chunks_per_block, PhysParams phys,
                 typename SpeedBits<R>::T* __restrict__ smax_out) {
@@ -91,7 +96,7 @@ timestep_kernel(const AuxBlock<R>* __restrict__ blocks, int nblocks,
   R* __restrict__ const f_p = B.pressure;
   // U cells per thread per pass, every load of the pass issued before the
   // arithmetic (the pass's stores would otherwise hold later loads back)
-  constexpr int U = TimestepTune<R, DE>::U;
+  constexpr int U = TimestepTune<R, MHD, DE>::U;
   const size_t stride = (size_t)chunks_per_block * blockDim.x;
   for (size_t c0 = (size_t)chunk * blockDim.x + threadIdx.x; c0 < ncell; c0 += U * stride) {
     R rho[U], vx[U], vy[U], vz[U], bx[U], by[U], bz[U], et[U], ei[U];

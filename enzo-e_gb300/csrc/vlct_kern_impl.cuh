@@ -17,6 +17,43 @@ namespace {
 // Device ordinals a per-device cache covers.
 constexpr int kMaxDevices = 64;
 
+// CTAs of a kernel that the current device holds at once, asked for once per
+// device (the query costs as much as a launch) and kept in `cache`.
+inline cudaError_t resident_ctas(const void* k, int threads, size_t smem,
+                                 std::atomic<int>* cache, int& out) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  out = dev < kMaxDevices ? cache[dev].load(std::memory_order_acquire) : 0;
+  if (out > 0) return cudaSuccess;
+  int nsm = 1, per_sm = 1;
+  e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  if (e == cudaSuccess)
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, smem);
+  if (e != cudaSuccess) return e;
+  out = std::max(1, per_sm) * std::max(1, nsm);
+  if (dev < kMaxDevices) cache[dev].store(out, std::memory_order_release);
+  return cudaSuccess;
+}
+
+template <class R, bool MHD, bool DE>
+cudaError_t timestep_one(const AuxBlock<R>* b, int nb, int cpb, size_t cells,
+                         const PhysParams& phys, typename SpeedBits<R>::T* smax,
+                         cudaStream_t st) {
+  auto* k = timestep_kernel<R, MHD, DE>;
+  if (cpb <= 0) {
+    static std::atomic<int> cache[kMaxDevices];
+    int resident = 1;
+    const cudaError_t e = resident_ctas((const void*)k, 256, 0, cache, resident);
+    if (e != cudaSuccess) return e;
+    // at least a pass of an FP64 CTA, two of an FP32 one: one FP64 block of 16^3 in
+    // 41 CTAs 19 us, in 10 33 us
+    cpb = wave_chunks(nb, resident, cells, sizeof(R) == 8 ? 256 : 512);
+  }
+  k<<<nb * cpb, 256, 0, st>>>(b, nb, cpb, phys, smax);
+  return cudaGetLastError();
+}
+
 // One stage as the kernels of vlct_split.cuh, group after group of jobs.
 template <class R, int SOLVER, int RECON, bool DE>
 cudaError_t stage_split(const StageBlock<R>* b, const SplitLaunch& sp, const StageInfo& info,
@@ -61,21 +98,17 @@ cudaError_t stage_fused(const StageBlock<R>* b, const StageTile* t, int nt,
   auto* k = stage_kernel<R, SOLVER, RECON, DE, EXTRA>;
   constexpr size_t smem = stage_smem_bytes<R, SOLVER, RECON, DE>();
   constexpr int threads = StageBounds<R, SOLVER, RECON>::threads;
-  static std::atomic<int> resident[kMaxDevices];
-  int dev = 0;
+  static std::atomic<int> resident[kMaxDevices], ready[kMaxDevices];
+  int dev = 0, fit = 1;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  int fit = dev < kMaxDevices ? resident[dev].load(std::memory_order_acquire) : 0;
-  if (fit == 0) {
+  if (dev >= kMaxDevices || !ready[dev].load(std::memory_order_acquire)) {
     e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    int nsm = 1, per_sm = 1;
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    if (e == cudaSuccess)
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, smem);
     if (e != cudaSuccess) return e;
-    fit = std::max(1, per_sm) * std::max(1, nsm);
-    if (dev < kMaxDevices) resident[dev].store(fit, std::memory_order_release);
+    if (dev < kMaxDevices) ready[dev].store(1, std::memory_order_release);
   }
+  e = resident_ctas((const void*)k, threads, smem, resident, fit);
+  if (e != cudaSuccess) return e;
   if (nt <= 0) return cudaSuccess;
   if (grid <= 0) grid = fit;
   k<<<std::min(grid, nt), threads, smem, st>>>(b, t, nt, info, phys);
@@ -163,7 +196,7 @@ cudaError_t launch_stage<VLCT_REAL>(int solver, int recon, bool de,
 template <>
 cudaError_t launch_timestep<VLCT_REAL>(bool mhd, bool de,
                                        const AuxBlock<VLCT_REAL>* b, int nb,
-                                       int cpb, const PhysParams& phys,
+                                       int cpb, size_t cells, const PhysParams& phys,
                                        void* d_smax, double courant,
                                        int global_min, double* d_dt,
                                        double* d_dt_min, cudaStream_t st) {
@@ -171,15 +204,12 @@ cudaError_t launch_timestep<VLCT_REAL>(bool mhd, bool de,
   T* smax = (T*)d_smax;
   cudaError_t e = cudaMemsetAsync(smax, 0, sizeof(T) * 3 * (size_t)nb, st);
   if (e != cudaSuccess) return e;
-  const int grid = nb * cpb;
-  if (mhd) {
-    if (de) timestep_kernel<VLCT_REAL, true, true><<<grid, 256, 0, st>>>(b, nb, cpb, phys, smax);
-    else timestep_kernel<VLCT_REAL, true, false><<<grid, 256, 0, st>>>(b, nb, cpb, phys, smax);
-  } else {
-    if (de) timestep_kernel<VLCT_REAL, false, true><<<grid, 256, 0, st>>>(b, nb, cpb, phys, smax);
-    else timestep_kernel<VLCT_REAL, false, false><<<grid, 256, 0, st>>>(b, nb, cpb, phys, smax);
-  }
-  e = cudaGetLastError();
+  if (mhd)
+    e = de ? timestep_one<VLCT_REAL, true, true>(b, nb, cpb, cells, phys, smax, st)
+           : timestep_one<VLCT_REAL, true, false>(b, nb, cpb, cells, phys, smax, st);
+  else
+    e = de ? timestep_one<VLCT_REAL, false, true>(b, nb, cpb, cells, phys, smax, st)
+           : timestep_one<VLCT_REAL, false, false>(b, nb, cpb, cells, phys, smax, st);
   if (e != cudaSuccess) return e;
   timestep_finish_kernel<VLCT_REAL><<<1, 256, 0, st>>>(b, nb, smax, courant, global_min,
                                                        d_dt, d_dt_min);
@@ -188,11 +218,33 @@ cudaError_t launch_timestep<VLCT_REAL>(bool mhd, bool de,
 
 template <>
 cudaError_t launch_refresh<VLCT_REAL>(const AuxBlock<VLCT_REAL>* b, const int* nbr,
-                                      int nb, int g, int cpb, int max_m, cudaStream_t st) {
+                                      int nb, int g, int cpb, size_t shell, bool mhd, int max_m,
+                                      cudaStream_t st) {
   // the decode of refresh_shell_kernel is exact while (shell elements of a
   // field) x (largest divisor) < 2^32; bound the shell by the whole field
   const unsigned long long mm = (unsigned long long)max_m + 1;
-  if (mm * mm * mm * mm < (1ull << 32))
+  const bool quick = mm * mm * mm * mm < (1ull << 32);
+  if (cpb <= 0) {
+    // One wave of CTAs, of a pass each at least, where that leaves none more than
+    // 6000 ghost cells, with B, twice the arrays, 2000 (4000 in small blocks: FP32, 200
+    // of 16^3, 400 CTAs 33 us, 1000 37; FP64 hydro, one block of 64^3:
+    // 304 CTAs 9.9 us, 456 12.1; FP32, eight of 128^3: 456 CTAs 55.5 us, 4864 61.7).  More
+    // work in chunks of 1700, with B 1100: a CTA's pointer tables cost it two memory
+    // round trips (FP32, 512 blocks of 32^3: 6656 CTAs 193 us, 2048 206, 9728 197; MHD, 30
+    // of 56^3: 1740 CTAs 74 us, 450 82).
+    static std::atomic<int> cache[2][kMaxDevices];
+    int resident = 1;
+    const cudaError_t e =
+        resident_ctas(quick ? (const void*)refresh_shell_kernel<VLCT_REAL>
+                            : (const void*)refresh_kernel<VLCT_REAL>,
+                      256, 0, cache[quick], resident);
+    if (e != cudaSuccess) return e;
+    const size_t one = (size_t)resident / nb;
+    const size_t most = !mhd ? 6000 : one <= 2 ? 4000 : 2000;
+    const bool wave = 4 * one * nb >= 3 * (size_t)resident && shell <= most * one;
+    cpb = (int)std::max<size_t>(1, wave ? std::min(one, shell / 256) : shell / (mhd ? 1100 : 1700));
+  }
+  if (quick)
     refresh_shell_kernel<VLCT_REAL><<<nb * cpb, 256, 0, st>>>(b, nbr, nb, g, cpb);
   else
     refresh_kernel<VLCT_REAL><<<nb * cpb, 256, 0, st>>>(b, nbr, nb, g, NCELL + 11, cpb);

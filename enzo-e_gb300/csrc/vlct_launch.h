@@ -3,6 +3,8 @@
 // kern_f32.cu).
 #pragma once
 #include <cuda_runtime.h>
+
+#include <algorithm>
 #include <stddef.h>
 
 #include "vlct_types.h"
@@ -45,18 +47,42 @@ cudaError_t launch_stage(int solver, int recon, bool de,
                          const PhysParams& phys, int grid, cudaStream_t st,
                          const SplitLaunch& split = SplitLaunch());
 
+// Chunks a block is cut into by a kernel that takes nb x chunks CTAs of which the GPU
+// holds `resident` at once, for blocks of `work` items, at least `least` of them a
+// chunk.  A grid of exactly the CTAs held is best, as a few more make the whole GPU
+// wait for them (FP32 hydro timestep, 16 blocks of 64^3: 608 CTAs, four on each SM,
+// 44 us; 656 54 us; 304 56 us; 4864 47 us); where nb divides that badly, the fewest
+// waves that are nine tenths full.
+inline int wave_chunks(long nb, long resident, size_t work, size_t least) {
+  const long most = std::max<long>(1, (long)(work / least));
+  long best = 1;
+  double full = 0.0;
+  for (long w = 1; w <= 8 && full < 0.9; w++) {
+    const long c = w * resident / nb;
+    if (c >= most) return (int)most;
+    const double f = (double)(c * nb) / (double)(w * resident);
+    if (f > full + 1e-9) {
+      full = f;
+      best = c;
+    }
+  }
+  return (int)best;
+}
+
+// chunks_per_block 0: as fills the GPU best, blocks having `cells` cells on average
 template <class R>
 cudaError_t launch_timestep(bool mhd, bool de, const AuxBlock<R>* d_blocks,
-                            int nblocks, int chunks_per_block,
+                            int nblocks, int chunks_per_block, size_t cells,
                             const PhysParams& phys, void* d_smax,
                             double courant, int global_min, double* d_dt,
                             double* d_dt_min, cudaStream_t st);
 
 // max_m: the largest ghosted extent of any block (selects the multiply-high
-// shell decode when it is exact for every block)
+// shell decode when it is exact for every block); chunks_per_block 0: as fills the
+// GPU best, blocks having `shell` ghost cells on average
 template <class R>
 cudaError_t launch_refresh(const AuxBlock<R>* d_blocks, const int* d_nbr,
-                           int nblocks, int g, int chunks_per_block, int max_m,
+                           int nblocks, int g, int chunks_per_block, size_t shell, bool mhd, int max_m,
                            cudaStream_t st);
 
 template <class R>

@@ -189,12 +189,38 @@ static int check_slabs() {
   return 0;
 }
 
+// The chunks of the timestep's launch: within the work there is, and a grid that is a
+// whole number of waves but for a tenth, or as near as eight waves come.
+static int check_chunks() {
+  for (long nb : {1, 2, 3, 7, 30, 64, 128, 152, 200, 305, 512, 608, 1000, 2000, 100000})
+    for (long res : {1, 152, 304, 608})
+      for (size_t work : {(size_t)1, (size_t)2744, (size_t)10648, (size_t)343000, (size_t)20000000}) {
+        const int c = vlct::wave_chunks(nb, res, work, 512);
+        const long most = std::max<long>(1, (long)(work / 512));
+        bool ok = c >= 1 && c <= most;
+        if (c < most && nb <= 8 * res) {
+          double best = 0.0, got = 0.0;
+          for (long w = 1; w <= 8; w++) {
+            best = std::max(best, (double)(w * res / nb * nb) / (double)(w * res));
+            if (w * res >= c * nb) got = std::max(got, (double)(c * nb) / (double)(w * res));
+          }
+          ok = ok && (got >= 0.9 || got >= best - 1e-9);
+        }
+        if (!ok) {
+          std::printf("%ld blocks, %ld CTAs at once, %zu items: %d chunks\n", nb, res, work, c);
+          return 1;
+        }
+      }
+  return 0;
+}
+
 int main(int argc, char** argv) {
   int bad = 2;
   if (argc > 1 && !std::strcmp(argv[1], "f64_tiles")) bad = check_f64_tiles();
   if (argc > 1 && !std::strcmp(argv[1], "search")) bad = check_search();
   if (argc > 1 && !std::strcmp(argv[1], "search_time")) bad = check_search_time();
   if (argc > 1 && !std::strcmp(argv[1], "slabs")) bad = check_slabs();
+  if (argc > 1 && !std::strcmp(argv[1], "chunks")) bad = check_chunks();
   if (!bad) std::printf("ok\n");
   return bad;
 }

@@ -30,7 +30,7 @@ def checks(tmp_path_factory):
     return _build("plan_checks", tmp_path_factory.mktemp("plans"))
 
 
-@pytest.mark.parametrize("check", ["f64_tiles", "search", "search_time", "slabs"])
+@pytest.mark.parametrize("check", ["f64_tiles", "search", "search_time", "slabs", "chunks"])
 def test_plan(checks, check):
     r = subprocess.run([checks, check], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout + r.stderr
