@@ -5,11 +5,10 @@
 // is kinetically or magnetically dominated.  FP64 path: the reference's
 // expressions in double, operation for operation.  FP32 path: the products
 // and differences are carried in float-float (an unevaluated sum hi + lo of
-// two floats, ~48-bit significand) with error-free transformations (Knuth's
-// TwoSum, the FMA-based TwoProduct), so the recovery is as accurate as an
-// FP64 evaluation of the same float inputs while running on the FP32 pipes
-// (GB300's FP64 rate is 1/64 of its FP32 rate).  The result is rounded to
-// float once.
+// two floats, 46 bits and more) with error-free transformations (Knuth's
+// TwoSum, the FMA-based TwoProduct), so that the recovery, rounded to float
+// once, keeps a float's accuracy through a cancellation of 20 bits, while
+// running on the FP32 pipes (GB300's FP64 rate is 1/64 of its FP32 rate).
 // Reference: src/Enzo/fluid-props/EnzoComputePressure.cpp:127-190,
 // EnzoPhysicsFluidProps.cpp:162-290.
 #pragma once

@@ -25,10 +25,11 @@ template <> struct TileLimits<float> { static constexpr int TMAX = 40; };
 //
 // Threads and CTAs per SM: FP32 MHD stages want up to 166 registers a thread
 // and run at 128 (two CTAs of 256); more, smaller-register CTAs spill (256^3
-// HLLD + PLM box, cycle: 256 x 2 6.34 ms, NN at 224 x 3 and PLM at 224 x 2 6.71,
-// both at 288 x 2 7.54).  Hydro stages are lighter: NN four CTAs of 256, PLM two
-// of 320 (960-leaf HLLC mesh with flux correction, cycle: 6.23 ms; 3 x 256 and
-// 2 x 288 6.40; 3 x 256 both 6.45; 2 x 288 and 2 x 384 6.95).
+// HLLD + PLM box, cycle: 256 x 2 5.65 ms; NN at 224 x 3 and PLM at 224 x 2 6.05;
+// both at 288 x 2 7.07).  Hydro stages are lighter: NN four CTAs of 256, PLM two
+// of 320 (960-leaf HLLC mesh with flux correction, cycle: 6.00 ms; 3 x 256 and
+// 2 x 288 5.98; 2 x 288 and 2 x 384 6.11; 3 x 256 both, slower while the tiles
+// covered the layer around the updated cells too, 5.80: not taken up yet).
 struct StageKind {
   bool f64, nn, mhd;
   constexpr int threads() const { return !f64 && !mhd && !nn ? 320 : 256; }

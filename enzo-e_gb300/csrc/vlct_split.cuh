@@ -15,14 +15,15 @@
 // reference's), so the FP64 results are the same bit for bit.
 //
 // Measured (HLLD + PLM): a 128^3 box of 64 blocks of 32^3, one cycle, 37.9 ms
-// with the fused kernel and the reference's own HLLD branches, 17.6 ms here;
-// one 32^3 block through the Method (dt, ghosts, step) 981 -> 427 us.  The FP64
-// pipe is 84-86% busy in the flux kernels, which take 81% of a cycle at 408
-// (NN) and 488 (PLM) pipe operations a face.
+// with a fused kernel and the reference's own HLLD branches, 14.9 ms here; one
+// 32^3 block through the Method (dt, ghosts, step) 981 -> 386 us.  The FP64 pipe
+// is 84-86% busy in the flux kernels, which take 85% of the stages' time at 333
+// (NN) and 413 (PLM) pipe operations a face, idle lanes included.
 //
 // Work is cut into jobs: one block, or a z-slab of one, with its slice of the
 // workspace.  A launch covers a group of jobs (blockIdx.y), so the workspace
-// stays bounded whatever the size of the batch.
+// stays bounded whatever the size of the batch.  MHD blocks of planes too wide
+// for slabs of five run the fused kernel (split_plan).
 #pragma once
 #include "vlct_stage.cuh"
 

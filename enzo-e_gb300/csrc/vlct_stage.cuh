@@ -27,14 +27,15 @@
 //   A  (PLM) the x and y slopes of the plane published in C, each formed once
 //      and read by both faces of its cell; | barrier
 //
-// What bounds it: issue slots (51-55% used; FMA, ALU and LSU pipes 24-33%, DRAM
+// What bounds it: issue slots (53-57% used; FMA, ALU and LSU pipes 24-33%, DRAM
 // 10%), with 16 warps an SM, as the Riemann solvers want 128 registers.  Against
 // the form it replaced, whose threads took each phase's items in rounds (every
-// item's place worked out anew, launch shapes of one block size compiled in):
-// HLLD + PLM warp instructions per zone 129 -> 94 (half dt), 135 -> 121 (full).
-// One cycle, before -> after: 256^3 in blocks of 32^3 6.60 -> 6.29 ms; in blocks
-// of 64^3 with dual energy 11.7 -> 5.35 ms; 1000 blocks of 16^3 - 64^3
-// 29.2 -> 12.6 ms; 960 hydro leaves with flux correction 7.45 -> 6.21 ms.
+// item's place worked out anew, launch shapes of one block size compiled in, the
+// layer around the updated cells in the tiles): HLLD + PLM warp instructions per
+// zone 129 -> 98 (half dt), 135 -> 98 (full).  One cycle, before -> after: 256^3
+// in blocks of 32^3 6.60 -> 5.65 ms; in blocks of 64^3 with dual energy 11.7 ->
+// 5.39 ms; 1000 blocks of 16^3 - 64^3 29.2 -> 12.2 ms; 960 hydro leaves with flux
+// correction 7.45 -> 6.00 ms.
 //
 // The index windows of every quantity are those of the reference's array
 // passes (EnzoMHDIntegratorStageCommands::compute_update_stage,
@@ -51,9 +52,10 @@
 // advected by passive_kernel, vlct_passive.cuh); the default one compiles
 // all of these out.
 //
-// FP64 runs this kernel only where the split kernels' workspace cannot be had
-// (vlct_split.cuh: the no-allocation step, or a GPU that is full); FP32, whose
-// arithmetic is 64 times cheaper, always does.
+// FP64 runs this kernel only where the split kernels (vlct_split.cuh) cannot or
+// should not: the no-allocation step, a GPU too full for their workspace, MHD
+// blocks of very wide planes.  FP32, whose arithmetic is 64 times cheaper, always
+// does.
 #pragma once
 #include <type_traits>
 
@@ -945,7 +947,7 @@ stage_kernel(const StageBlock<R>* __restrict__ blocks,
 // the updated region alone: as columns and planes of its march that layer made
 // a 32^3 block 34^3 zones, and 16^3 18^3.  This kernel, on the same tiles after
 // it, gives each tile the layer's cells next to it.  It moves nine values a cell
-// of the layer: 56 us for 216 blocks of 32^3 (DRAM 36 B a zone).  With it and the
+// of the layer: 57 us for 216 blocks of 32^3 (DRAM 36 B a zone).  With it and the
 // tiles that fit_tile then takes, the full-dt stage of 512 blocks of 32^3 with
 // dual energy takes 2.94 instead of 3.71 ms, and the cycle of the 256^3 box
 // without it 5.65 instead of 6.28 ms.
