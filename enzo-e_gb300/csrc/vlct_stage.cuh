@@ -32,7 +32,7 @@
 // the form it replaced, whose threads took each phase's items in rounds (every
 // item's place worked out anew, launch shapes of one block size compiled in, the
 // layer around the updated cells in the tiles): HLLD + PLM warp instructions per
-// zone 129 -> 98 (half dt), 135 -> 98 (full).  One cycle, before -> after: 256^3
+// zone 129 -> 98 (half dt), 135 -> 97 (full).  One cycle, before -> after: 256^3
 // in blocks of 32^3 6.60 -> 5.65 ms; in blocks of 64^3 with dual energy 11.7 ->
 // 5.39 ms; 1000 blocks of 16^3 - 64^3 29.2 -> 12.2 ms; 960 hydro leaves with flux
 // correction 7.45 -> 6.00 ms.
@@ -949,7 +949,7 @@ stage_kernel(const StageBlock<R>* __restrict__ blocks,
 // the updated region alone: as columns and planes of its march that layer made
 // a 32^3 block 34^3 zones, and 16^3 18^3.  This kernel, on the same tiles after
 // it, gives each tile the layer's cells next to it.  It moves nine values a cell
-// of the layer: 57 us for 216 blocks of 32^3 (DRAM 36 B a zone).  With it and the
+// of the layer: 56 us for 216 blocks of 32^3 (DRAM 36 B a zone).  With it and the
 // tiles that fit_tile then takes, the full-dt stage of 512 blocks of 32^3 with
 // dual energy takes 2.94 instead of 3.71 ms, and the cycle of the 256^3 box
 // without it 5.65 instead of 6.28 ms.
